@@ -345,14 +345,9 @@ cudaError_t adjoint_vjp_muscl(const DevMesh& m, const DevState& s, const SpatOpt
   if (m.ng > 0) k_ghost_prim<<<nblk(m.ng), kBlock, 0, st>>>(m, s.prim, o);
   if (o.postlim != TY_POSTLIM_NONE) {  // gradient and the Barth ratios of the forward residual
     const double klim = o.postlim == TY_POSTLIM_SUPERBARTH ? 1.0 : 0.5;
-    if (kFast) {
-      if (m.nslot <= 4) k_cell_fast<4, 128><<<(unsigned)((m.nci + 127) / 128), 128, 0, st>>>(m, s, o, klim, true);
-      else k_cell_fast<8, 64><<<(unsigned)((m.nci + 63) / 64), 64, 0, st>>>(m, s, o, klim, true);
-    } else {
-      k_grad<<<nblk(m.nci), kBlock, 0, st>>>(m, s);
-      k_face_states<<<nblk(m.nf), kBlock, 0, st>>>(m, s, o);
-      k_barth<<<nblk(m.nci), kBlock, 0, st>>>(m, s, klim);
-    }
+    k_grad<<<nblk(m.nci), kBlock, 0, st>>>(m, s);
+    k_face_states<<<nblk(m.nf), kBlock, 0, st>>>(m, s, o);
+    k_barth<<<nblk(m.nci), kBlock, 0, st>>>(m, s, klim);
   } else {
     k_grad<<<nblk(m.nci), kBlock, 0, st>>>(m, s);
   }
@@ -741,11 +736,7 @@ cudaError_t adjoint_vjp_muscl_fast(const DevMesh& m, const DevState& s, const Sp
   k_prim<<<nblk(m.nci), kBlock, 0, st>>>(m, u, s.prim, o.gamma);
   if (m.ng > 0) k_ghost_prim<<<nblk(m.ng), kBlock, 0, st>>>(m, s.prim, o);
   const bool post = o.postlim != TY_POSTLIM_NONE;
-  if (post) {  // gradient and the Barth ratios of the forward residual
-    const double klim = o.postlim == TY_POSTLIM_SUPERBARTH ? 1.0 : 0.5;
-    if (m.nslot <= 4) k_cell_fast<4, 128><<<(unsigned)((m.nci + 127) / 128), 128, 0, st>>>(m, s, o, klim, true);
-    else k_cell_fast<8, 64><<<(unsigned)((m.nci + 63) / 64), 64, 0, st>>>(m, s, o, klim, true);
-  }
+  if (post) cell_fast(m, s, o, true, false, st);  // gradient and the Barth ratios of the forward residual
   k_adj_pack<<<nblk(m.nci), kBlock, 0, st>>>(m, s, post, lamR, ldR, dt, wtab, crec);
   const unsigned gf = (unsigned)((m.nf + 127) / 128);
   if (o.scheme == TY_SCH_HLLC) k_adj_face2f<TY_SCH_HLLC><<<gf, 128, 0, st>>>(m, o, crec, frec);

@@ -309,12 +309,27 @@ int ready(ty_mesh* h) {
 int stage_faces(ty_mesh* h) {
   // every table a kernel of this configuration reads must exist before any launch
   if ((h->o.viscous != TY_VISC_NONE && !h->m.vgeo) || (h->o.gradmeth != TY_GRAD_NONE && !h->m.lsq) ||
-      (h->o.highres != TY_HRES_NONE && !h->m.dLR)) {
+      (h->o.highres != TY_HRES_NONE && !h->m.dLR) ||
+      (h->o.mode == TY_MODE_FAST && h->o.highres != TY_HRES_NONE && !h->m.stab &&
+       (!h->m.mtab || h->o.viscous != TY_VISC_NONE))) {
     tyi::set_error("internal: a geometry table of the selected scheme is missing");
     return TY_ERR_STATE;
   }
   cudaError_t e = MODE_CALL(h, residual_faces, h->m, h->s, h->o, h->stream, &h->prof);
   if (e != cudaSuccess) return cuda_fail(e, "residual faces");
+  return TY_OK;
+}
+
+// the slot tables of the fast cell kernel for the selected gradient method and MUSCL variant
+int ensure_stab(ty_mesh* h) {
+  const int key = h->geo_highres * 16 + h->lsq_gradmeth;
+  if (h->m.stab && h->stab_key == key) return TY_OK;
+  int rc;
+  if (!h->stab_buf && (rc = h->alloc(h->stab_buf, (size_t)tyk::kSlotTab * h->m.nslot * (size_t)h->m.nci))) return rc;
+  cudaError_t e = tyk::kfast::build_stab(h->m, h->geo_highres, h->stab_buf, h->stream);
+  if (e != cudaSuccess) return cuda_fail(e, "slot tables");
+  h->m.stab = h->stab_buf;
+  h->stab_key = key;
   return TY_OK;
 }
 
@@ -537,6 +552,7 @@ int ty_mesh_create(const ty_mesh_desc* d, int device, ty_mesh** out) {
   TY_CU(cudaMemset(s.ratio, 0, 3 * lc * sizeof(double)));
   if (cudaMallocHost((void**)&h->dtbits_host, 4 * sizeof(double)) != cudaSuccess) return bail(TY_ERR_NOMEM);
   h->nslot = nslot;
+  m.ghost_copy = ng > 0 && !h->nonperiodic_bc;
   *out = h;
   return TY_OK;
 }
@@ -592,6 +608,7 @@ int ty_mesh_set_face_rotation(ty_mesh* h, const double* rot) {
       any = any || v != ((q % 4 == 0) ? 1.0 : 0.0);
     }
   if (!any) return TY_OK;  // translations only: nothing to rotate
+  h->m.ghost_copy = false;
   if (!h->m.frot) {
     if (int rc = h->upload(h->m.frot, d)) return rc;
   } else {
@@ -645,6 +662,8 @@ int ty_set_params(ty_mesh* h, const ty_spat_params* p) {
     if (e != cudaSuccess) return cuda_fail(e, "increment matrices");
     h->m.mtab = h->mtab_buf;
   }
+  if (p->mode == TY_MODE_FAST && p->highres != TY_HRES_NONE && (!h->m.mtab || p->viscous != TY_VISC_NONE))
+    if ((rc = ensure_stab(h))) return rc;
   h->o.scheme = p->scheme; h->o.highres = p->highres; h->o.limiter = p->limiter; h->o.postlim = p->postlim;
   h->o.gradmeth = p->gradmeth; h->o.mode = p->mode; h->o.gamma = p->gamma; h->o.entropy_fix = p->entropy_fix;
   h->o.inv_entropy_fix = p->entropy_fix > 0.0 ? 1.0 / p->entropy_fix : 0.0;

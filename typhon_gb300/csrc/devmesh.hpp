@@ -16,6 +16,7 @@ namespace tyk {
 
 constexpr int kMaxSlot = 8;    // faces per cell held in the gather list (hexahedra need 6)
 constexpr int kMaxStage = 6;   // Runge-Kutta stages
+constexpr int kSlotTab = 11;   // columns of DevMesh::stab
 
 struct DevMesh {
   int dim = 0, nci = 0, nc = 0, nfi = 0, nf = 0, ng = 0, nslot = 0;
@@ -53,6 +54,9 @@ struct DevMesh {
                                   // increments of a cell are linear in its neighbour differences,
                                   // D_i = sum_j M_ij dq_j (gradient and reconstruction folded);
                                   // null when not built
+  const double* stab = nullptr;   // [nslot][kSlotTab][nci] fast MUSCL schemes: per slot the vectors and
+                                  // factors of the gradient and the limited increment (k_build_stab)
+  bool ghost_copy = false;        // every boundary face is periodic by translation: ghost = source cell
   const int* cfn = nullptr;       // [nslot][nci] neighbour cell across each gather-list face
   const double* invV = nullptr;   // [nci] 1 / V (fast mode)
   const double* geo2 = nullptr;   // [nci] 2 V / sum S (fast mode time step)
@@ -187,6 +191,8 @@ TY_DECLARE_MODE(kfast)
 namespace kfast {
 // the per-cell increment matrices of DevMesh::mtab, from lsqw, recw and the gather lists
 cudaError_t build_mtab(const DevMesh& m, double* mtab, cudaStream_t st);
+// DevMesh::stab for a MUSCL variant, from lsqw, uLR, dLR, kLF, kRF and recw
+cudaError_t build_stab(const DevMesh& m, int highres, double* stab, cudaStream_t st);
 }
 
 }  // namespace tyk

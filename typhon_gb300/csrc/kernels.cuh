@@ -1042,256 +1042,224 @@ __global__ void __launch_bounds__(kBlock) k_face_flux_lim(DevMesh m, DevState s,
 }
 
 
-// Increment q_face - q_c of the 5 primitive variables on one side of face f, from the
-// cell's gradient gr (15), its value qc and dq = q_nb - q_c.
-__device__ __forceinline__ void delta_fast(const DevMesh& m, const SpatOpts& o, int f, int side, const double* gr,
-                                           const double* dq, double* D) {
-  const size_t lf = m.ldf;
-  if ((o.highres == TY_HRES_MUSCL || o.highres == TY_HRES_MUSCLUNS) && o.limiter == TY_LIM_NONE) {
-    const double wx = m.recw[(4 * side) * lf + f], wy = m.recw[(4 * side + 1) * lf + f];
-    const double wz = m.recw[(4 * side + 2) * lf + f], k = m.recw[(4 * side + 3) * lf + f];
-#pragma unroll
-    for (int v = 0; v < 5; ++v) D[v] = fma(gr[3 * v], wx, fma(gr[3 * v + 1], wy, fma(gr[3 * v + 2], wz, dq[v] * k)));
-    return;
-  }
-  const double ux = d3(m.uLR, m.ldf, f, 0), uy = d3(m.uLR, m.ldf, f, 1), uz = d3(m.uLR, m.ldf, f, 2);
-  const double idLR = m.invdLR[f];
-  const double sgn = side ? -1.0 : 1.0;  // (q(fc2) - q(fc1)) = sgn * dq
-  if (o.highres == TY_HRES_MUSCLFAST) {
-    const double k = side ? m.kRF[f] : m.kLF[f];
-#pragma unroll
-    for (int v = 0; v < 5; ++v) {
-      const double LR = sgn * dq[v] * idLR;
-      double sg = LR;
-      if (o.limiter != TY_LIM_NONE) {
-        const double g = gr[3 * v] * ux + gr[3 * v + 1] * uy + gr[3 * v + 2] * uz;
-        sg = apply_lim(o.limiter, false, v < 2, g, LR);
-      }
-      D[v] = sg * k;
-    }
-    return;
-  }
-  const bool uns = o.highres == TY_HRES_MUSCLUNS;
-  const double* CF = side ? m.RF : m.LF;
-  const double cx = d3(CF, m.ldf, f, 0), cy = d3(CF, m.ldf, f, 1), cz = d3(CF, m.ldf, f, 2);
-  const double uc = ux * cx + uy * cy + uz * cz;
-#pragma unroll
-  for (int v = 0; v < 5; ++v) {
-    const double LR = sgn * dq[v] * idLR;
-    const double g = gr[3 * v] * ux + gr[3 * v + 1] * uy + gr[3 * v + 2] * uz;
-    const double sg = (o.limiter == TY_LIM_NONE ? LR : apply_lim(o.limiter, uns, v < 2, g, LR)) - g;
-    D[v] = gr[3 * v] * cx + gr[3 * v + 1] * cy + gr[3 * v + 2] * cz + sg * uc;
-  }
-}
-
-// Fused per-cell kernel: least-squares gradient (A^-1 d weights), face increments on every
-// face of the cell, Barth-type ratio without per-face divisions, and the limited face
-// states written once per face side (cl for the fc1 side, cr for the fc2 side).
-// The neighbour differences dq of the gradient pass and the increments are staged in shared
-// memory ([slot*5+var][thread], conflict-free), so each is computed once and the kernel keeps
-// few registers live (four blocks of 128 threads per SM).
-// The ratio min_f max(klim (q_nb - q_c)/increment, 0) is tracked as a fraction n/d; the
-// comparisons run on the integer pipe (positive finite doubles order like their bit
-// patterns), leaving the FP64 pipe to the arithmetic, and the one division per variable
-// group is a Newton-Raphson reciprocal.  The increment is the reconstruction's value (the
-// exact mode, like Typhon, rounds it through the face value first); an increment of exactly
-// zero imposes no constraint in both modes.
+#if TY_FAST
 __device__ __forceinline__ long long dbits(double x) { return __double_as_longlong(x); }
 
+// x == 0 on the integer pipe (on the 32-bit halves: the compiler turns a test of the 64-bit
+// pattern back into an FP64 comparison)
+__device__ __forceinline__ bool is_zero(double x) {
+  return (((unsigned)__double2hiint(x) << 1) | (unsigned)__double2loint(x)) == 0u;
+}
+
+// |x| without the FP64 instruction of fabs
+__device__ __forceinline__ double abs_bits(double x) {
+  return __hiloint2double(__double2hiint(x) & 0x7fffffff, __double2loint(x));
+}
+
+// |x| as an FP32 number, truncated (relative error below 2^-23) on the integer pipe, when x lies
+// in [2^-60, 2^60); ok is cleared otherwise.
+__device__ __forceinline__ float trunc32(double x, bool& ok) {
+  const int hi = __double2hiint(x) & 0x7fffffff;
+  ok = ok && (unsigned)(hi - ((1023 - 60) << 20)) < (unsigned)(120 << 20);
+  return __uint_as_float(__funnelshift_l((unsigned)__double2loint(x), (unsigned)hi, 3) - ((1023u - 127u) << 23));
+}
+
+// |a| b < |c| d of positive products, as bit patterns.  A call, so that the multiplications are
+// not if-converted into the callers: a predicated-off FP64 instruction occupies the pipe as well.
+__device__ __noinline__ bool product_less(double a, double b, double c, double d) {
+  return __double_as_longlong(fabs(a) * b) < __double_as_longlong(d * fabs(c));
+}
+
+// van Albada's phi(a, b) = a b (a + b) / (a^2 + b^2) where a b > 0, else 0, sum = a + b given.
+// Products below 2^-1000 count as 0 (the reciprocal's seed flushes subnormal numbers).
+__device__ __forceinline__ double albada_fast(double a, double b, double sum) {
+  const double ab = a * b;
+  if (__double2hiint(ab) < (23 << 20)) return 0.0;
+  return ab * sum * rcp_nr(fma(a, a, b * b));
+}
+
+// Fused cell kernel: neighbour differences, face increments, Barth-type ratio and the limited
+// face states, written once per face side (cl for the fc1 side, cr for the fc2 side).
 //
-// With DevMesh::mtab (MUSCL / MUSCL-UNS without limiter) the increments come from the cell's
-// matrix, D_i = sum_j M_ij dq_j: the gradient G = sum_j (+-A^-1 d_j) dq_j and the increment
-// D_i = G . w_i + dq_i k_i folded into one product of nslot^2 multiply-adds per variable (16
-// for a tetrahedron, against 12 for the gradient and 16 for the increments), read coalesced
-// per cell instead of per face; the gradient itself is then computed only when asked
-// (want_grad: a viscous flux or the adjoint reads it).
-template <int NS, int BLK>
-__global__ void __launch_bounds__(BLK, 512 / BLK) k_cell_fast(DevMesh m, DevState s, SpatOpts o, double klim,
-                                                              bool want_grad) {
-  __shared__ double sD[NS * 5][BLK];
-  __shared__ double sQ[NS * 5][BLK];
-  const int c = blockIdx.x * BLK + threadIdx.x;
-  if (c >= m.nci) return;
-  const int t = threadIdx.x;
-  const size_t ld = m.ldc, lf = m.ldf, ni = m.nci;
-  const double* __restrict__ prim = s.prim;
-  double qc[5];
-#pragma unroll
-  for (int v = 0; v < 5; ++v) qc[v] = prim[v * ld + c];
-  const bool mt = m.mtab != nullptr;
-  const bool grad = !mt || want_grad;
-  double gr[15];
-#pragma unroll
-  for (int k = 0; k < 15; ++k) gr[k] = 0.0;
-  // the gather-list entries and neighbours of every slot first, so that the neighbour loads
-  // below are independent of each other and issue together
+// One thread per cell and variable: a warp holds 32 cells of one variable, a block the five
+// variables of its cells.  GB300 issues one FP64 warp instruction per 64 clocks and SM quarter
+// and everything here but the velocities' common ratio is per variable, so five short chains
+// replace one long one: small meshes occupy five times as many SM quarters, and the differences
+// and increments of the (at most NS) faces fit in registers at full occupancy.  The lists and
+// tables are read by five warps of one block, from L1 after the first.
+//
+// FORM 0 (MUSCL / MUSCL-UNS without limiter): D_i = sum_j M_ij dq_j from the cell's matrix
+//   (DevMesh::mtab).
+// FORM 1 (van Albada) and FORM 2 (the other limiters, none included): the least-squares
+//   gradient G, then per face, with the slot table of DevMesh::stab (outward vectors),
+//     D = G . w + phi(a, dq) k,  a = 2 G . d - dq (MUSCL, MUSCL-FAST) or G . d (MUSCL-UNS),
+//   the slopes scaled by the distance |d| (the limiters are homogeneous of degree one; LIM03,
+//   which is not, gets them unscaled).
+//
+// The ratio min_f max(klim dq/D, 0) is kept as a fraction n/d.  A candidate is compared with it
+// in FP32 on truncated operands, which decides all but comparisons closer than 2^-20, and those
+// are redone with the FP64 products: the same winner as an FP64 comparison without its two
+// multiplications per face.  An increment of exactly zero imposes no constraint.
+//
+// copy_ghosts: every boundary face is a translational periodic one; the ghosts' states are
+// copies of their source cells', written here by the one cell that reads them, and
+// k_ghost_prim is not launched.
+//
+// Bound by the FP64 pipe (82 % busy at 30 operations per thread in FORM 0 with the ratio).
+// Comparisons of doubles, |x| and predicated-off arithmetic run on that pipe too, so tests are
+// made on bit patterns and rare FP64 work sits behind a call.  Microseconds per launch on GB300,
+// one thread per cell (differences staged in shared memory) -> one thread per cell and variable:
+// 1,310,720 tetrahedra FORM 0 + ratio 628 -> 350; 370,440 tetrahedra FORM 1 460 -> 283; 87,500
+// prisms and tetrahedra FORM 1 133 -> 78; 163,840 tetrahedra FORM 1 213 -> 127.
+constexpr int kCellVars = 5;
+
+template <int NS, int FORM>
+__global__ void __launch_bounds__(32 * kCellVars) k_cell_fast(DevMesh m, DevState s, SpatOpts o, double klim,
+                                                              bool copy_ghosts) {
+  __shared__ double sr[3][32];
+  const int c0 = blockIdx.x * 32 + threadIdx.x, v = threadIdx.y;
+  const bool on = c0 < m.nci;
+  const int c = on ? c0 : m.nci - 1;
+  const size_t ld = m.ldc, lf = m.ldf, n = m.nci;
   int es[NS], nbs[NS];
-  int ns = 0;
+#pragma unroll
+  for (int sl = 0; sl < NS; ++sl) es[sl] = sl < m.nslot ? m.cf[sl * n + c] : -1;
+#pragma unroll
+  for (int sl = 0; sl < NS; ++sl) nbs[sl] = es[sl] >= 0 ? m.cfn[sl * n + c] : c;
+  double* __restrict__ prim = s.prim + v * ld;
+  const double qc = prim[c];
+  double dq[NS];
 #pragma unroll
   for (int sl = 0; sl < NS; ++sl) {
-    es[sl] = sl < m.nslot ? m.cf[sl * ni + c] : -1;
-    nbs[sl] = es[sl] >= 0 ? m.cfn[sl * ni + c] : c;
-    ns += es[sl] >= 0 ? 1 : 0;
+    const bool ghost = copy_ghosts && nbs[sl] >= m.nci;
+    const double q = prim[ghost ? m.gsrc[nbs[sl] - m.nci] : nbs[sl]];
+    if (ghost && on) prim[nbs[sl]] = q;
+    dq[sl] = q - qc;  // 0 on an unused slot
   }
+  double D[NS];
+  if constexpr (FORM == 0) {
+    const double* M = m.mtab + c;
+#pragma unroll
+    for (int i = 0; i < NS; ++i) {
+      double d = 0.0;
+      if (es[i] >= 0) {
+#pragma unroll
+        for (int j = 0; j < NS; ++j)
+          if (j < m.nslot) d = fma(__ldg(M + ((size_t)i * m.nslot + j) * n), dq[j], d);
+      }
+      D[i] = d;
+    }
+  } else {
+    const double* T = m.stab + c;
+    const bool uns = o.highres == TY_HRES_MUSCLUNS, fst = o.highres == TY_HRES_MUSCLFAST;
+    double gx = 0.0, gy = 0.0, gz = 0.0;
+#pragma unroll
+    for (int i = 0; i < NS; ++i) {
+      if (es[i] < 0) continue;
+      const double* t = T + (size_t)(kSlotTab * i) * n;
+      gx = fma(dq[i], __ldg(t), gx);
+      gy = fma(dq[i], __ldg(t + n), gy);
+      gz = fma(dq[i], __ldg(t + 2 * n), gz);
+    }
+    if (on) {
+      double* g = s.grad + 3 * v * ld + c;
+      g[0] = gx; g[ld] = gy; g[2 * ld] = gz;
+    }
+#pragma unroll
+    for (int i = 0; i < NS; ++i) {
+      D[i] = 0.0;
+      if (es[i] < 0) continue;
+      const double* t = T + (size_t)(kSlotTab * i + 3) * n;
+      const double k = __ldg(t + 6 * n), b = dq[i];
+      double phi = b;
+      if (FORM == 1 || o.limiter != TY_LIM_NONE) {
+        const double g = fma(gx, __ldg(t), fma(gy, __ldg(t + n), gz * __ldg(t + 2 * n)));  // G . d, twice it unless UNS
+        if constexpr (FORM == 1) {
+          phi = uns ? albada_fast(g, b, g + b) : albada_fast(g - b, b, g);
+        } else if (o.limiter == TY_LIM_LIM03) {
+          const double id = __ldg(t + 7 * n);
+          phi = apply_lim(o.limiter, uns, v < 2, (uns ? g : 0.5 * g) * id, b * id);
+          D[i] = fst ? 0.0 : fma(gx, __ldg(t + 3 * n), fma(gy, __ldg(t + 4 * n), gz * __ldg(t + 5 * n)));
+          D[i] = fma(phi, k / id, D[i]);
+          continue;
+        } else {
+          phi = apply_lim(o.limiter, uns, v < 2, uns ? g : 0.5 * g, b);
+        }
+      }
+      D[i] = fst ? phi * k : fma(gx, __ldg(t + 3 * n), fma(gy, __ldg(t + 4 * n), fma(gz, __ldg(t + 5 * n), phi * k)));
+    }
+  }
+  double r = 1.0;
+  if (o.postlim != TY_POSTLIM_NONE) {
+    double bn = 1.0, bd = klim;
+    float fn = 1.0f, fd = o.postlim == TY_POSTLIM_SUPERBARTH ? 1.0f : 0.5f;
+    bool zero = false, far = false;  // far: the fraction is outside the FP32 comparison's range
+#pragma unroll
+    for (int i = 0; i < NS; ++i) {
+      if (es[i] < 0 || is_zero(D[i])) continue;
+      if (is_zero(dq[i]) || (__double2hiint(dq[i]) ^ __double2hiint(D[i])) < 0) {  // dq/D <= 0
+        zero = true;
+        continue;
+      }
+      bool ok = !far;
+      const float fq = trunc32(dq[i], ok), fD = trunc32(D[i], ok);
+      const float x = fq * fd, y = fn * fD;
+      bool less = x < y;
+      if (!ok || fabsf(x - y) <= 9.6e-7f * y) less = product_less(dq[i], bd, D[i], bn);
+      if (less) {
+        bn = abs_bits(dq[i]);
+        bd = abs_bits(D[i]);
+        bool in = true;
+        fn = trunc32(dq[i], in); fd = trunc32(D[i], in);
+        far = !in;
+      }
+    }
+    // the fraction starts at 1: min(1, klim n/d), as bit patterns (positive doubles order alike)
+    r = klim * bn * rcp_nr(bd);
+    if (dbits(r) > dbits(1.0)) r = 1.0;
+    if (zero) r = 0.0;
+    if (v >= 2) sr[v - 2][threadIdx.x] = r;
+    __syncthreads();
+    if (v >= 2) {  // the three velocity components share the smallest ratio (compared as bit patterns)
+      const double a = sr[0][threadIdx.x], b = sr[1][threadIdx.x], d = sr[2][threadIdx.x];
+      r = dbits(a) < dbits(b) ? a : b;
+      r = dbits(d) < dbits(r) ? d : r;
+    }
+    if (on && v < 3) s.ratio[v * ld + c] = r;
+  }
+  if (!on) return;
 #pragma unroll
   for (int sl = 0; sl < NS; ++sl) {
-    const int e = es[sl];
-    if (e < 0) continue;
-    const int f = e >> 1, side = e & 1, nb = nbs[sl];
-    if (grad) {
-      // q(fc2) - q(fc1) = +-dq: the weight's sign flipped on the integer pipe for side 1
-      const long long sb = (long long)side << 63;
-      const double wx = __longlong_as_double(__double_as_longlong(m.lsqw[(3 * side) * lf + f]) ^ sb);
-      const double wy = __longlong_as_double(__double_as_longlong(m.lsqw[(3 * side + 1) * lf + f]) ^ sb);
-      const double wz = __longlong_as_double(__double_as_longlong(m.lsqw[(3 * side + 2) * lf + f]) ^ sb);
-#pragma unroll
-      for (int v = 0; v < 5; ++v) {
-        const double dq = prim[v * ld + nb] - qc[v];
-        sQ[sl * 5 + v][t] = dq;
-        gr[3 * v] = fma(dq, wx, gr[3 * v]);
-        gr[3 * v + 1] = fma(dq, wy, gr[3 * v + 1]);
-        gr[3 * v + 2] = fma(dq, wz, gr[3 * v + 2]);
-      }
-    } else {
-#pragma unroll
-      for (int v = 0; v < 5; ++v) sQ[sl * 5 + v][t] = prim[v * ld + nb] - qc[v];
-    }
-  }
-  if (grad) {
-#pragma unroll
-    for (int k = 0; k < 15; ++k) s.grad[k * ld + c] = gr[k];
-  }
-  const bool barth = o.postlim != TY_POSTLIM_NONE;
-  double bn[3] = {1.0, 1.0, 1.0}, bd[3] = {klim, klim, klim};
-  bool zero[3] = {false, false, false};
-  for (int sl = 0; sl < ns; ++sl) {
-    const int e = m.cf[sl * ni + c], f = e >> 1, side = e & 1;
-    double dq[5], D[5];
-#pragma unroll
-    for (int v = 0; v < 5; ++v) dq[v] = sQ[sl * 5 + v][t];
-    if (mt) {
-      // the row's NS coefficients loaded together (one memory latency per row, not per term)
-      const double* M = m.mtab + (size_t)sl * m.nslot * ni + c;
-      double mr[NS];
-#pragma unroll
-      for (int j = 0; j < NS; ++j) mr[j] = j < ns ? __ldg(M + (size_t)j * ni) : 0.0;
-#pragma unroll
-      for (int v = 0; v < 5; ++v) D[v] = 0.0;
-#pragma unroll
-      for (int j = 0; j < NS; ++j) {
-        if (j < ns) {
-#pragma unroll
-          for (int v = 0; v < 5; ++v) D[v] = fma(mr[j], sQ[j * 5 + v][t], D[v]);
-        }
-      }
-    } else {
-      delta_fast(m, o, f, side, gr, dq, D);
-    }
-#pragma unroll
-    for (int v = 0; v < 5; ++v) {
-      const double den = D[v];
-      sD[sl * 5 + v][t] = den;
-      if (barth) {
-        const int k = v < 2 ? v : 2;
-        const long long bden = dbits(den), bdq = dbits(dq[v]);
-        if ((bden << 1) != 0) {                                   // den != 0
-          if ((bdq << 1) == 0 || ((bdq ^ bden) < 0)) {             // dq/den <= 0
-            zero[k] = true;
-          } else {
-            const double x = fabs(dq[v]) * bd[k], y = bn[k] * fabs(den);
-            if (dbits(x) < dbits(y)) { bn[k] = fabs(dq[v]); bd[k] = fabs(den); }
-          }
-        }
-      }
-    }
-  }
-  double r[3] = {1.0, 1.0, 1.0};
-  if (barth) {
-#pragma unroll
-    for (int k = 0; k < 3; ++k) r[k] = zero[k] ? 0.0 : fmin(1.0, klim * bn[k] * rcp_nr(bd[k]));
-#pragma unroll
-    for (int k = 0; k < 3; ++k) s.ratio[k * ld + c] = r[k];
-  }
-  for (int sl = 0; sl < ns; ++sl) {
-    const int e = m.cf[sl * ni + c], f = e >> 1, side = e & 1;
-    double* out = side ? s.cr : s.cl;
-#pragma unroll
-    for (int v = 0; v < 5; ++v) out[v * lf + f] = fma(r[v < 2 ? v : 2], sD[sl * 5 + v][t], qc[v]);
+    if (es[sl] < 0) continue;
+    double* out = (es[sl] & 1) ? s.cr : s.cl;
+    out[v * lf + (es[sl] >> 1)] = fma(r, D[sl], qc);
   }
 }
 
-// k_cell_fast for the case of DevMesh::mtab without a gradient output (MUSCL / MUSCL-UNS
-// without limiter, inviscid): the neighbour differences and the increments of the (at most
-// NS) faces stay in registers instead of shared memory, which the FP64 pipe no longer waits
-// for.  Same arithmetic as k_cell_fast.
-template <int NS, int BLK>
-__global__ void __launch_bounds__(BLK, 512 / BLK) k_cell_fast_mt(DevMesh m, DevState s, SpatOpts o, double klim) {
-  const int c = blockIdx.x * BLK + threadIdx.x;
-  if (c >= m.nci) return;
-  const size_t ld = m.ldc, lf = m.ldf, ni = m.nci;
-  const double* __restrict__ prim = s.prim;
-  int es[NS], nbs[NS];
-  int ns = 0;
-#pragma unroll
-  for (int sl = 0; sl < NS; ++sl) {
-    es[sl] = sl < m.nslot ? m.cf[sl * ni + c] : -1;
-    nbs[sl] = es[sl] >= 0 ? m.cfn[sl * ni + c] : c;
-    ns += es[sl] >= 0 ? 1 : 0;
-  }
-  double qc[5];
-#pragma unroll
-  for (int v = 0; v < 5; ++v) qc[v] = prim[v * ld + c];
-  double dq[NS][5];
-#pragma unroll
-  for (int sl = 0; sl < NS; ++sl)
-#pragma unroll
-    for (int v = 0; v < 5; ++v) dq[sl][v] = prim[v * ld + nbs[sl]] - qc[v];  // 0 on an unused slot
-  const bool barth = o.postlim != TY_POSTLIM_NONE;
-  double bn[3] = {1.0, 1.0, 1.0}, bd[3] = {klim, klim, klim};
-  bool zero[3] = {false, false, false};
-  double D[NS][5];
-#pragma unroll
-  for (int sl = 0; sl < NS; ++sl) {
-    const double* M = m.mtab + (size_t)sl * m.nslot * ni + c;
-    double mr[NS];
-#pragma unroll
-    for (int j = 0; j < NS; ++j) mr[j] = (sl < ns && j < ns) ? __ldg(M + (size_t)j * ni) : 0.0;
-#pragma unroll
-    for (int v = 0; v < 5; ++v) {
-      double d = 0.0;
-#pragma unroll
-      for (int j = 0; j < NS; ++j) d = fma(mr[j], dq[j][v], d);
-      D[sl][v] = d;
-      if (barth && sl < ns) {
-        const int k = v < 2 ? v : 2;
-        const long long bden = dbits(d), bdq = dbits(dq[sl][v]);
-        if ((bden << 1) != 0) {                                   // d != 0
-          if ((bdq << 1) == 0 || ((bdq ^ bden) < 0)) {             // dq/d <= 0
-            zero[k] = true;
-          } else {
-            const double x = fabs(dq[sl][v]) * bd[k], y = bn[k] * fabs(d);
-            if (dbits(x) < dbits(y)) { bn[k] = fabs(dq[sl][v]); bd[k] = fabs(d); }
-          }
-        }
-      }
-    }
-  }
-  double r[3] = {1.0, 1.0, 1.0};
-  if (barth) {
-#pragma unroll
-    for (int k = 0; k < 3; ++k) r[k] = zero[k] ? 0.0 : fmin(1.0, klim * bn[k] * rcp_nr(bd[k]));
-#pragma unroll
-    for (int k = 0; k < 3; ++k) s.ratio[k * ld + c] = r[k];
-  }
-#pragma unroll
-  for (int sl = 0; sl < NS; ++sl) {
-    if (sl >= ns) continue;
-    const int e = es[sl], f = e >> 1, side = e & 1;
-    double* out = side ? s.cr : s.cl;
-#pragma unroll
-    for (int v = 0; v < 5; ++v) out[v * lf + f] = fma(r[v < 2 ? v : 2], D[sl][v], qc[v]);
-  }
+template <int NS>
+void cell_fast_ns(const DevMesh& m, const DevState& s, const SpatOpts& o, double klim, bool copy_ghosts, bool matrix,
+                  cudaStream_t st) {
+  const dim3 b(32, kCellVars);
+  const unsigned g = (unsigned)((m.nci + 31) / 32);
+  if (matrix) k_cell_fast<NS, 0><<<g, b, 0, st>>>(m, s, o, klim, copy_ghosts);
+  else if (o.limiter == TY_LIM_ALBADA) k_cell_fast<NS, 1><<<g, b, 0, st>>>(m, s, o, klim, copy_ghosts);
+  else k_cell_fast<NS, 2><<<g, b, 0, st>>>(m, s, o, klim, copy_ghosts);
 }
+
+// want_grad: the caller reads s.grad (a viscous flux, the adjoint); the matrix form has none.
+// NS is the mesh's largest number of faces per cell (3 triangles, 4 quadrangles and tetrahedra,
+// 5 pyramids and prisms, 6 hexahedra), so that no unrolled slot is idle on a uniform mesh.
+void cell_fast(const DevMesh& m, const DevState& s, const SpatOpts& o, bool want_grad, bool copy_ghosts,
+               cudaStream_t st) {
+  const double klim = o.postlim == TY_POSTLIM_SUPERBARTH ? 1.0 : 0.5;
+  const bool matrix = m.mtab && !want_grad;
+  if (m.nslot <= 3) cell_fast_ns<3>(m, s, o, klim, copy_ghosts, matrix, st);
+  else if (m.nslot == 4) cell_fast_ns<4>(m, s, o, klim, copy_ghosts, matrix, st);
+  else if (m.nslot == 5) cell_fast_ns<5>(m, s, o, klim, copy_ghosts, matrix, st);
+  else if (m.nslot == 6) cell_fast_ns<6>(m, s, o, klim, copy_ghosts, matrix, st);
+  else cell_fast_ns<kMaxSlot>(m, s, o, klim, copy_ghosts, matrix, st);
+}
+#endif
 
 #if TY_FAST
 // DevMesh::mtab of every interior cell: M_ij = (+-A^-1 d_j) . w_i + k_i [i == j] over the
@@ -1317,6 +1285,38 @@ __global__ void k_build_mtab(DevMesh m, double* __restrict__ mt) {
       mt[((size_t)i * ns + j) * n + c] = v;
     }
   }
+}
+
+// DevMesh::stab of every interior cell and slot: the least-squares weight +-A^-1 d (3), the
+// vector to the neighbour (3; doubled unless MUSCL-UNS, whose limiter takes G . d itself), the
+// reconstruction weight CF - (u . CF) u (3; 0 for MUSCL-FAST), the slope's factor (u . CF)/|d|
+// or, MUSCL-FAST, |F - C|/dLR, and 1/dLR, all seen from the cell outwards
+__global__ void k_build_stab(DevMesh m, int highres, double* __restrict__ T) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= m.nci) return;
+  const size_t n = m.nci, lf = m.ldf;
+  for (int i = 0; i < m.nslot; ++i) {
+    double* t = T + (size_t)(kSlotTab * i) * n + c;
+    const int e = m.cf[i * n + c];
+    if (e < 0) {
+      for (int k = 0; k < kSlotTab; ++k) t[k * n] = 0.0;
+      continue;
+    }
+    const int f = e >> 1, side = e & 1;
+    const double sg = side ? -1.0 : 1.0, two = highres == TY_HRES_MUSCLUNS ? 1.0 : 2.0;
+    for (int k = 0; k < 3; ++k) {
+      t[k * n] = sg * m.lsqw[(3 * side + k) * lf + f];
+      t[(3 + k) * n] = two * sg * (m.uLR[k * lf + f] * m.dLR[f]);
+      t[(6 + k) * n] = m.recw[(4 * side + k) * lf + f];
+    }
+    t[9 * n] = highres == TY_HRES_MUSCLFAST ? (side ? -m.kRF[f] : m.kLF[f]) * m.invdLR[f] : m.recw[(4 * side + 3) * lf + f];
+    t[10 * n] = m.invdLR[f];
+  }
+}
+
+cudaError_t build_stab(const DevMesh& m, int highres, double* stab, cudaStream_t st) {
+  k_build_stab<<<(unsigned)((m.nci + kBlock - 1) / kBlock), kBlock, 0, st>>>(m, highres, stab);
+  return cudaGetLastError();
 }
 
 cudaError_t build_mtab(const DevMesh& m, double* mtab, cudaStream_t st) {
@@ -1546,29 +1546,18 @@ cudaError_t prim_from(const DevMesh& m, const DevState& s, const SpatOpts& o, co
 
 // everything between the primitive variables of a stage state and the face fluxes
 cudaError_t residual_faces(const DevMesh& m, const DevState& s, const SpatOpts& o, cudaStream_t st, Prof* pr) {
-  if (m.ng > 0)
+  const bool cell_kernel = kFast && o.highres != TY_HRES_NONE;
+  if (m.ng > 0 && !(cell_kernel && m.ghost_copy))
     pr->launch(K_GHOST_PRIM, st, [&] { k_ghost_prim<<<nblk(m.ng), kBlock, 0, st>>>(m, s.prim, o); });
-  if (kFast && o.highres != TY_HRES_NONE) {
-    const double klim = o.postlim == TY_POSTLIM_SUPERBARTH ? 1.0 : 0.5;
-    if (m.nslot <= 4 && m.mtab && o.viscous == TY_VISC_NONE)
-      pr->launch(K_CELL_FAST, st, [&] {
-        k_cell_fast_mt<4, 128><<<(unsigned)((m.nci + 127) / 128), 128, 0, st>>>(m, s, o, klim);
-      });
-    else if (m.nslot <= 4)
-      pr->launch(K_CELL_FAST, st, [&] {
-        k_cell_fast<4, 128><<<(unsigned)((m.nci + 127) / 128), 128, 0, st>>>(m, s, o, klim,
-                                                                              o.viscous != TY_VISC_NONE);
-      });
-    else
-      pr->launch(K_CELL_FAST, st, [&] {
-        k_cell_fast<8, 64><<<(unsigned)((m.nci + 63) / 64), 64, 0, st>>>(m, s, o, klim,
-                                                                           o.viscous != TY_VISC_NONE);
-      });
+#if TY_FAST
+  if (cell_kernel) {
+    pr->launch(K_CELL_FAST, st, [&] { cell_fast(m, s, o, o.viscous != TY_VISC_NONE, m.ghost_copy, st); });
     if (o.viscous != TY_VISC_NONE && m.ng > 0)
       pr->launch(K_GHOST_GRAD, st, [&] { k_ghost_grad<<<nblk(m.ng), kBlock, 0, st>>>(m, s.grad); });
     pr->launch(K_FACE_FLUX_FAST, st, [&] { k_face_flux_fast<<<nblk(m.nf), kBlock, 0, st>>>(m, s, o); });
     return cudaGetLastError();
   }
+#endif
   if (o.gradmeth != TY_GRAD_NONE) {
     pr->launch(K_GRAD, st, [&] { k_grad<<<nblk(m.nci), kBlock, 0, st>>>(m, s); });
     if (m.ng > 0)
