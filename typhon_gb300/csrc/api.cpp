@@ -669,6 +669,9 @@ int ty_set_params(ty_mesh* h, const ty_spat_params* p) {
   h->o.inv_entropy_fix = p->entropy_fix > 0.0 ? 1.0 / p->entropy_fix : 0.0;
   h->o.ig1 = 1.0 / (p->gamma - 1.0);
   h->o.gig1 = p->gamma * h->o.ig1;
+  h->o.roe_sub = 1.0 - p->entropy_fix;
+  h->o.irgas = p->rgas != 0.0 ? 1.0 / p->rgas : 0.0;
+  h->o.iprandtl = p->prandtl != 0.0 ? 1.0 / p->prandtl : 0.0;
   {  // the HLL family's wave-speed variant (def_spat.f90:68-76, calc_flux_hllc.f90:64-72)
     const int sc = p->scheme;
     h->o.hll_family = (sc == TY_SCH_HLLC || (sc >= TY_SCH_HLLCB && sc <= TY_SCH_HLLCKB)) ? 1

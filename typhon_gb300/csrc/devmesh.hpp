@@ -89,6 +89,8 @@ struct SpatOpts {
   double gamma, entropy_fix;
   double inv_entropy_fix;  // 1 / entropy_fix (fast-mode Roe flux)
   double ig1, gig1;        // 1 / (gamma - 1), gamma / (gamma - 1) (fast-mode fluxes)
+  double roe_sub;          // 1 - entropy_fix: |u.n| up to this times a is outside the entropy fix
+  double irgas, iprandtl;  // 1 / rgas, 1 / prandtl (0 when not set)
   // HLL family (TY_SCH_HLLC / HLLE and their B, K, KB variants): 1 HLLC, 2 HLLE, 0 other;
   // kinetic wave speeds; beta; f1 = sqrt(gamma/2), f2 = 1/(2 sqrt(pi)) of the kinetic estimates
   int hll_family, hll_kin;

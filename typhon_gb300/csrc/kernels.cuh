@@ -252,6 +252,14 @@ __global__ void k_ghost_prim(DevMesh m, double* __restrict__ prim, SpatOpts o) {
   if (kind == TY_BC_WALL || kind == TY_BC_NOSLIP) {
     const double r = o.rgas, lflux = 0.0;
     const double rho = prim[src], p = prim[ld + src];
+    if constexpr (kFast) {  // lflux = 0: the wall's temperature is the cell's, its density too
+      prim[ld + g] = p;
+      prim[g] = rho;
+      prim[2 * ld + g] = fma(2.0, d3(m.fwall, m.ldf, f, 0), -vx);
+      prim[3 * ld + g] = fma(2.0, d3(m.fwall, m.ldf, f, 1), -vy);
+      prim[4 * ld + g] = fma(2.0, d3(m.fwall, m.ldf, f, 2), -vz);
+      return;
+    }
     const double mu = viscosity(o, rho, p / (r * rho));
     const double cp = o.gamma / (o.gamma - 1.0) * r;
     const double conduct = mu * cp / o.prandtl;
@@ -693,114 +701,177 @@ __device__ void flux_roe(double g, double eps, const double* L, const double* R,
 // so reciprocals, reconstruction weights and geometric factors are precomputed once
 // (HBM-resident) and the per-stage work avoids divisions.
 
-// Roe flux with shared reciprocals: no division, 1 reciprocal and 3 reciprocal square roots
-// by Newton-Raphson steps (fastmath.cuh) per face.  The same flux as flux_roe, regrouped so
-// that the central and dissipative parts share their products:
-//   2 F_mass = m_L + m_R - d_mass                       (m = rho u.n)
-//   2 F_ener = m_L H_L + m_R H_R - d_ener               (rho u.n (rho E + p) = m H)
-//   2 F_mom  = A u_L + B u_R + c_n n, with the Roe velocity u~ = k_L u_L + k_R u_R and the
-//              shear jump written through u_R - u_L:
-//              A = m_L + ws - d_mass k_L, B = m_R - ws - d_mass k_R,
-//              c_n = p_L + p_R - (w5 - w1) a + ws (u_R - u_L).n
-__device__ void flux_roe_fast(const SpatOpts& o, const double* L, const double* R, double nx, double ny, double nz,
-                              double S, double* F) {
-  const double g1 = o.gamma - 1.0, eps = o.entropy_fix, ieps = o.inv_entropy_fix, gig1 = o.gig1;
-  // Roe weights from one reciprocal square root: with y = 1/sqrt(rho_L rho_R),
-  // rroe = sqrt(rho_L rho_R) = rho_L rho_R y, kl = sqrt(rho_L) / (sqrt(rho_L) + sqrt(rho_R)) =
-  // rho_L / (rho_L + rroe), kr = rroe / (rho_L + rroe), 1/rho_L = y^2 rho_R, 1/rho_R = y^2 rho_L
-  const double P = L[0] * R[0], y = rsqrt_nr(P), y2 = y * y;
-  const double rroe = P * y;
-  const double inv = rcp_nr(L[0] + rroe);
-  const double kl = L[0] * inv, kr = rroe * inv;
-  const double iL = y2 * R[0], iR = y2 * L[0];
-  const double ux = kl * L[2] + kr * R[2], uy = kl * L[3] + kr * R[3], uz = kl * L[4] + kr * R[4];
-  const double sqL = L[2] * L[2] + L[3] * L[3] + L[4] * L[4];
-  const double sqR = R[2] * R[2] + R[3] * R[3] + R[4] * R[4];
-  const double hl = (gig1 * L[1]) * iL + 0.5 * sqL, hr = (gig1 * R[1]) * iR + 0.5 * sqR;
-  const double hroe = kl * hl + kr * hr;
-  const double q2 = ux * ux + uy * uy + uz * uz;
-  const double a2 = g1 * (hroe - 0.5 * q2);
-  const double ra = rsqrt_nr(a2), a = a2 * ra, ia2 = ra * ra;
-  const double vn = ux * nx + uy * ny + uz * nz;
-  const double vnl = L[2] * nx + L[3] * ny + L[4] * nz, vnr = R[2] * nx + R[3] * ny + R[4] * nz;
-  const double drho = R[0] - L[0], dp = R[1] - L[1], dvn = vnr - vnl;
-  const double h = 0.5 * ia2, rad = rroe * a * dvn;
-  const double al1 = (dp - rad) * h, al5 = (dp + rad) * h, al2 = drho - dp * ia2;
-  double l1 = fabs(vn - a), l5 = fabs(vn + a);
-  const double l2 = fabs(vn);
-  const double delta = eps * a;
-  // non-negative doubles compare like their bit patterns: test on the integer pipe
-  if (__double_as_longlong(l1) < __double_as_longlong(delta) || __double_as_longlong(l5) < __double_as_longlong(delta)) {
-    const double hd = 0.5 * ra * ieps;  // 1 / (2 delta)
-    if (l1 < delta) l1 = (l1 * l1 + delta * delta) * hd;
-    if (l5 < delta) l5 = (l5 * l5 + delta * delta) * hd;
-  }
-  const double w1 = l1 * al1, w2 = l2 * al2, w5 = l5 * al5, ws = l2 * rroe;
-  const double d_mass = w1 + w2 + w5;
-  const double wa = (w5 - w1) * a;
-  const double ml = vnl * L[0], mr = vnr * R[0];
-  const double hs = 0.5 * S;  // flux times surface: the 1/2 of the Roe average folded in
-  // momentum
-  const double A = ml + ws - d_mass * kl, B = mr - ws - d_mass * kr;
-  const double cn = (L[1] + R[1]) - wa + ws * dvn;
-  F[2] = hs * (A * L[2] + B * R[2] + cn * nx);
-  F[3] = hs * (A * L[3] + B * R[3] + cn * ny);
-  F[4] = hs * (A * L[4] + B * R[4] + cn * nz);
-  // energy
-  const double udu = ux * (R[2] - L[2]) + uy * (R[3] - L[3]) + uz * (R[4] - L[4]);
-  const double d_ener = (w1 + w5) * hroe + wa * vn + w2 * (0.5 * q2) + ws * (udu - vn * dvn);
-  F[1] = hs * (ml * hl + mr * hr - d_ener);
-  F[0] = hs * (ml + mr - d_mass);
+#if TY_FAST
+// Comparisons of doubles run on the FP64 pipe (a minimum is a comparison and a select); on bit
+// patterns they run on the integer pipe.
+__device__ __forceinline__ long long order_key(double x) {  // orders like x
+  const long long b = __double_as_longlong(x);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+__device__ __forceinline__ double min_bits(double a, double b) { return order_key(a) < order_key(b) ? a : b; }
+__device__ __forceinline__ double max_bits(double a, double b) { return order_key(a) < order_key(b) ? b : a; }
+__device__ __forceinline__ bool is_neg(double x) { return __double2hiint(x) < 0; }  // sign bit
+// x without the sign (fabs of a stored value is an FP64 instruction)
+__device__ __forceinline__ double abs_bits(double x) {
+  return __hiloint2double(__double2hiint(x) & 0x7fffffff, __double2loint(x));
 }
 
-// HLLC (calc_flux_hllc.f90 with beta = 1) with shared reciprocals: no division; the
-// reciprocals, square roots and reciprocal square roots by Newton-Raphson iterations
-// (fastmath.cuh), the Roe weights and both 1/rho from one reciprocal square root.
-__device__ void flux_hllc_fast(const SpatOpts& o, const double* L, const double* R, double nx, double ny, double nz,
-                               double* F) {
-  const double g = o.gamma, ig1 = o.ig1, gig1 = o.gig1;
-  // Roe weights from one reciprocal square root (as flux_roe_fast)
-  const double P = L[0] * R[0], y = rsqrt_nr(P), y2 = y * y;
-  const double rroe = P * y;
-  const double inv = rcp_nr(L[0] + rroe);
-  const double kl = L[0] * inv, kr = rroe * inv;
-  const double iL = y2 * R[0], iR = y2 * L[0];
-  const double rux = kl * L[2] + kr * R[2], ruy = kl * L[3] + kr * R[3], ruz = kl * L[4] + kr * R[4];
-  const double sqL = L[2] * L[2] + L[3] * L[3] + L[4] * L[4];
-  const double sqR = R[2] * R[2] + R[3] * R[3] + R[4] * R[4];
-  const double hroe = kl * (gig1 * L[1] * iL + 0.5 * sqL) + kr * (gig1 * R[1] * iR + 0.5 * sqR);
-  const double vnl = L[2] * nx + L[3] * ny + L[4] * nz, vnr = R[2] * nx + R[3] * ny + R[4] * nz;
-  const double al = sqrt_nr(g * L[1] * iL), ar = sqrt_nr(g * R[1] * iR);
-  const double vm = rux * nx + ruy * ny + ruz * nz;
-  const double am = sqrt_nr((g - 1.0) * (hroe - 0.5 * (rux * rux + ruy * ruy + ruz * ruz)));
-  const double rel = ig1 * L[1] + 0.5 * L[0] * sqL, rer = ig1 * R[1] + 0.5 * R[0] * sqR;
-  double sl, sr;
-  hll_speeds(o, vnl, vnr, al, ar, vm, am, sl, sr);
-  if (sl >= 0.0) {
-    const double m0 = vnl * L[0];
-    F[0] = m0; F[1] = vnl * (rel + L[1]);
-    F[2] = m0 * L[2] + L[1] * nx; F[3] = m0 * L[3] + L[1] * ny; F[4] = m0 * L[4] + L[1] * nz;
-  } else if (sr <= 0.0) {
-    const double m0 = vnr * R[0];
-    F[0] = m0; F[1] = vnr * (rer + R[1]);
-    F[2] = m0 * R[2] + R[1] * nx; F[3] = m0 * R[3] + R[1] * ny; F[4] = m0 * R[4] + R[1] * nz;
-  } else {
-    const double rqL = L[0] * (sl - vnl), rqR = R[0] * (sr - vnr);
-    const double Sst = (rqR * vnr - rqL * vnl - R[1] + L[1]) * rcp_nr(rqR - rqL);
-    const bool left = Sst >= 0.0;
-    const double* Q = left ? L : R;
-    const double rq = left ? rqL : rqR, s = left ? sl : sr, vnq = left ? vnl : vnr, re = left ? rel : rer;
-    const double iks = rcp_nr(s - Sst);
-    const double pst = Q[1] - rq * (vnq - Sst);
-    const double dp = pst - Q[1];
-    const double m0 = Sst * iks;
-    F[0] = m0 * rq;
-    F[1] = Sst * (iks * (re * (s - vnq) - Q[1] * vnq + pst * Sst) + pst);
-    F[2] = m0 * (rq * Q[2] + dp * nx) + pst * nx;
-    F[3] = m0 * (rq * Q[3] + dp * ny) + pst * ny;
-    F[4] = m0 * (rq * Q[4] + dp * nz) + pst * nz;
-  }
+// Roe weights and reciprocal densities from one reciprocal square root: with y = 1/sqrt(rho_L
+// rho_R), rroe = sqrt(rho_L rho_R) = rho_L rho_R y, kl = rho_L / (rho_L + rroe), kr = rroe /
+// (rho_L + rroe), 1/rho_L = y^2 rho_R, 1/rho_R = y^2 rho_L.
+struct RoeAvg {
+  F64 rroe, kl, kr, TL, TR;  // TL = p_L / rho_L
+};
+__device__ __forceinline__ RoeAvg roe_avg(const F64* L, const F64* R) {
+  RoeAvg r;
+  const F64 P = L[0] * R[0], y = rsqrt_nr(P), y2 = y * y;
+  r.rroe = P * y;
+  const F64 inv = rcp_nr(L[0] + r.rroe);
+  r.kl = L[0] * inv;
+  r.kr = r.rroe * inv;
+  r.TL = L[1] * (y2 * R[0]);
+  r.TR = R[1] * (y2 * L[0]);
+  return r;
 }
+
+// The acoustic waves of the Roe flux with Harten's fix, any regime: sum = w1 + w5 and
+// wa = (w5 - w1) a.  A call, taken by supersonic faces and those inside the fix.
+__device__ __noinline__ double2 roe_acoustic(double vn, double a, double ra, double dp, double Q, double eps, double ieps) {
+  const double h = 0.5 * ra * ra, rad = Q * a;
+  const double al1 = (dp - rad) * h, al5 = (dp + rad) * h, delta = eps * a;
+  double l1 = fabs(vn - a), l5 = fabs(vn + a);
+  const double hd = 0.5 * ra * ieps;  // 1 / (2 delta)
+  if (l1 < delta) l1 = (l1 * l1 + delta * delta) * hd;
+  if (l5 < delta) l5 = (l5 * l5 + delta * delta) * hd;
+  const double w1 = l1 * al1, w5 = l5 * al5;
+  return make_double2(w1 + w5, (w5 - w1) * a);
+}
+
+// Roe flux times S: no division, one reciprocal and two reciprocal square roots by
+// Newton-Raphson steps (fastmath.cuh).  The same flux as flux_roe, regrouped so that the
+// central and dissipative parts share their products (u~ = u_L + k_r du, du = u_R - u_L):
+//   2 F_mass = M = m_L + m_R - d                       (m = rho u.n, d = w1 + w2 + w5)
+//   2 F_mom  = M u_L + (m_R - ws - d k_r) du + c_n n,  c_n = p_L + p_R - (w5 - w1) a + ws du.n
+//   2 F_ener = m_L H_L + m_R H_R - d_ener              (rho u.n (rho E + p) = m H)
+// Where |u~.n| <= (1 - eps) a (subsonic, outside the entropy fix) the acoustic waves add up to
+//   w1 + w5 = dp/a + vn Q/a,  (w5 - w1) a = a Q + vn dp/a,  Q = rroe du.n,
+// without their strengths: 105 FP64 operations a face instead of 127, all of them DFMA (F64,
+// fastmath.cuh).  The face kernel of TGV 64^3x5 on GB300: 585 -> 507 us regrouped -> 456 us as F64
+// (FP64 pipe 96 % busy).
+__device__ void flux_roe_fast(const SpatOpts& o, const F64* L, const F64* R, F64 nx, F64 ny, F64 nz,
+                              F64 S, F64* F) {
+  const F64 gig2 = 2.0 * o.gig1, hg1 = 0.5 * (o.gamma - 1.0);
+  const RoeAvg r = roe_avg(L, R);
+  const F64 dx = R[2] - L[2], dy = R[3] - L[3], dz = R[4] - L[4];
+  const F64 ux = fma(r.kr, dx, L[2]), uy = fma(r.kr, dy, L[3]), uz = fma(r.kr, dz, L[4]);
+  // twice the enthalpies, and |u|^2 of the average
+  const F64 hl = fma(gig2, r.TL, fma(L[2], L[2], fma(L[3], L[3], L[4] * L[4])));
+  const F64 hr = fma(gig2, r.TR, fma(R[2], R[2], fma(R[3], R[3], R[4] * R[4])));
+  const F64 h = fma(r.kl, hl, r.kr * hr);
+  const F64 q2 = fma(ux, ux, fma(uy, uy, uz * uz));
+  const F64 a2 = hg1 * (h - q2);
+  const F64 ra = rsqrt_nr(a2), a = a2 * ra;
+  const F64 vnl = fma(L[2], nx, fma(L[3], ny, L[4] * nz)), vnr = fma(R[2], nx, fma(R[3], ny, R[4] * nz));
+  const F64 dvn = vnr - vnl, vn = fma(r.kr, dvn, vnl), dp = R[1] - L[1], drho = R[0] - L[0];
+  const F64 p1 = dp * ra, Q = r.rroe * dvn, l2 = abs_bits(vn.v);
+  F64 sum, wa;
+  if (__double_as_longlong(l2.v) <= __double_as_longlong((F64(o.roe_sub) * a).v)) {
+    sum = fma(vn, Q * ra, p1);
+    wa = fma(a, Q, vn * p1);
+  } else {
+    const double2 w = roe_acoustic(vn.v, a.v, ra.v, dp.v, Q.v, o.entropy_fix, o.inv_entropy_fix);
+    sum = w.x;
+    wa = w.y;
+  }
+  const F64 w2 = l2 * fma(-p1, ra, drho), ws = l2 * r.rroe, d = sum + w2;
+  const F64 ml = vnl * L[0], mr = vnr * R[0];
+  const F64 M = ml + mr - d, hs = F64(0.5) * S;
+  const F64 B = hs * fma(-d, r.kr, mr - ws);
+  const F64 cn = hs * (fma(ws, dvn, L[1] + R[1]) - wa);
+  const F64 F0 = hs * M;
+  F[0] = F0;
+  F[2] = fma(F0, L[2], fma(B, dx, cn * nx));
+  F[3] = fma(F0, L[3], fma(B, dy, cn * ny));
+  F[4] = fma(F0, L[4], fma(B, dz, cn * nz));
+  const F64 X = fma(-vn, dvn, fma(ux, dx, fma(uy, dy, uz * dz)));
+  const F64 Y = fma(wa, vn, ws * X);
+  const F64 d2 = fma(sum, h, fma(w2, q2, Y + Y));  // twice d_ener
+  F[1] = (F64(0.5) * hs) * (fma(ml, hl, mr * hr) - d2);
+}
+
+// mass and energy flux and pressure term of a supersonic face, times S (a call: see product_less)
+__device__ __noinline__ double3 hllc_supersonic(double S, double vq, double q0, double re, double p) {
+  return make_double3(S * (vq * q0), (S * vq) * (re + p), S * p);
+}
+
+// HLLC times S (calc_flux_hllc.f90) without divisions: Roe weights and both 1/rho from one
+// reciprocal square root, the average sound speed from
+//   a~^2 = g (k_l p_l/rho_l + k_r p_r/rho_r) + (g - 1)/2 k_l k_r |u_R - u_L|^2
+// (the kinetic energies of the enthalpies cancel against |u~|^2, which is not formed), only the
+// upwind side's energy, comparisons on bit patterns.  The face kernel of 370,440 tetrahedra:
+// 208 -> 137 us.
+__device__ void flux_hllc_fast(const SpatOpts& o, const F64* L, const F64* R, F64 nx, F64 ny, F64 nz,
+                               F64 S, F64* F) {
+  const F64 g = o.gamma;
+  const RoeAvg r = roe_avg(L, R);
+  const F64 dx = R[2] - L[2], dy = R[3] - L[3], dz = R[4] - L[4];
+  const F64 dd = fma(dx, dx, fma(dy, dy, dz * dz));
+  const F64 vnl = fma(L[2], nx, fma(L[3], ny, L[4] * nz)), vnr = fma(R[2], nx, fma(R[3], ny, R[4] * nz));
+  const F64 vm = fma(r.kr, vnr - vnl, vnl);
+  const F64 al = sqrt_nr(g * r.TL), ar = sqrt_nr(g * r.TR);
+  const F64 am = sqrt_nr(fma(g, fma(r.kl, r.TL, r.kr * r.TR), F64(0.5 * (o.gamma - 1.0)) * (r.kl * r.kr * dd)));
+  F64 sl, sr;
+  if (o.hll_kin) {
+    hll_speeds(o, vnl.v, vnr.v, al.v, ar.v, vm.v, am.v, sl.v, sr.v);
+  } else {
+    sl = min_bits(fma(F64(-o.hll_beta), al, vnl).v, (vm - am).v);
+    sr = max_bits(fma(F64(o.hll_beta), ar, vnr).v, (vm + am).v);
+  }
+  const F64 dl = sl - vnl, dr = sr - vnr;
+  const F64 rql = L[0] * dl, rqr = R[0] * dr;
+  const F64 Sst = (fma(rqr, vnr, fma(-rql, vnl, L[1])) - R[1]) * rcp_nr(rqr - rql);
+  // the side whose state gives the flux, and its wave speed
+  const bool supl = !is_neg(sl.v), supr = !supl && (is_neg(sr.v) || __double2hiint(sr.v) == 0);
+  const bool left = supl || (!supr && !is_neg(Sst.v));
+  const F64 q0 = left ? L[0] : R[0], p = left ? L[1] : R[1];
+  const F64 qx = left ? L[2] : R[2], qy = left ? L[3] : R[3], qz = left ? L[4] : R[4];
+  const F64 vq = left ? vnl : vnr, ds = left ? dl : dr, rq = left ? rql : rqr, sq = left ? sl : sr;
+  const F64 re = fma(F64(o.ig1), p, (F64(0.5) * q0) * fma(qx, qx, fma(qy, qy, qz * qz)));
+  F64 m0, E, c;
+  if (supl || supr) {
+    const double3 w = hllc_supersonic(S.v, vq.v, q0.v, re.v, p.v);
+    m0 = w.x; E = w.y; c = w.z;
+  } else {
+    const F64 i = rcp_nr(sq - Sst), dp = rq * (Sst - vq), pst = p + dp;
+    const F64 w = S * Sst, wi = w * i;
+    m0 = wi * rq;
+    E = w * fma(i, fma(re, ds, fma(pst, Sst, -p * vq)), pst);
+    c = fma(wi, dp, S * pst);
+  }
+  F[0] = m0;
+  F[1] = E;
+  F[2] = fma(m0, qx, c * nx);
+  F[3] = fma(m0, qy, c * ny);
+  F[4] = fma(m0, qz, c * nz);
+}
+
+// Rusanov times S (calc_flux_rusanov.f90:57-83) without divisions
+__device__ void flux_rusanov_fast(const SpatOpts& o, const F64* L, const F64* R, F64 nx, F64 ny, F64 nz,
+                                  F64 S, F64* F) {
+  const F64 TL = L[1] * rcp_nr(L[0]), TR = R[1] * rcp_nr(R[0]);
+  const F64 vnl = fma(L[2], nx, fma(L[3], ny, L[4] * nz)), vnr = fma(R[2], nx, fma(R[3], ny, R[4] * nz));
+  const F64 cl = F64(abs_bits(vnl.v)) + sqrt_nr(F64(o.gamma) * TL), cr = F64(abs_bits(vnr.v)) + sqrt_nr(F64(o.gamma) * TR);
+  const F64 ray = max_bits(cl.v, cr.v), hs = F64(0.5) * S;
+  const F64 el = fma(F64(o.ig1), TL, F64(0.5) * fma(L[2], L[2], fma(L[3], L[3], L[4] * L[4])));
+  const F64 er = fma(F64(o.ig1), TR, F64(0.5) * fma(R[2], R[2], fma(R[3], R[3], R[4] * R[4])));
+  const F64 A = hs * ((vnl + ray) * L[0]), B = hs * ((vnr - ray) * R[0]), pp = hs * (L[1] + R[1]);
+  F[0] = A + B;
+  F[1] = fma(A, el, fma(B, er, hs * fma(vnl, L[1], vnr * R[1])));
+  F[2] = fma(A, L[2], fma(B, R[2], pp * nx));
+  F[3] = fma(A, L[3], fma(B, R[3], pp * ny));
+  F[4] = fma(A, L[4], fma(B, R[4], pp * nz));
+}
+#endif
 
 // Laminar viscous flux added to F (per unit area), calc_flux_viscous_cell.f90:71-144, on the
 // cell states and cell gradients of the face's two cells (integration_ns_ust.f90:139-159).
@@ -889,50 +960,120 @@ __device__ void add_viscous(const DevMesh& m, const DevState& s, const SpatOpts&
   if (f >= m.nfi && (m.fbc[f] == TY_BC_WALL || m.fbc[f] == TY_BC_NOSLIP)) F[1] = F[1] + conduct * gTH + 0.0;
 }
 
-__device__ __forceinline__ void face_flux_fast(const DevMesh& m, const DevState& s, const SpatOpts& o, int f,
-                                               const double* QL, const double* QR, double* __restrict__ flux) {
-  const double nx = d3(m.fn, m.ldf, f, 0), ny = d3(m.fn, m.ldf, f, 1), nz = d3(m.fn, m.ldf, f, 2);
-  double F[5];
-  const double S = m.fs[f];
-  if (o.scheme == TY_SCH_ROE && o.viscous == TY_VISC_NONE) {
-    flux_roe_fast(o, QL, QR, nx, ny, nz, S, F);
-  } else {
-    if (o.scheme == TY_SCH_ROE) flux_roe_fast(o, QL, QR, nx, ny, nz, 1.0, F);
-    else if (o.hll_family == 1) flux_hllc_fast(o, QL, QR, nx, ny, nz, F);
-    else if (o.hll_family == 2) flux_hlle(o, QL, QR, nx, ny, nz, F);
-    else if (o.scheme == TY_SCH_AUSMM) flux_ausmm(o.gamma, QL, QR, nx, ny, nz, F);
-    else flux_rusanov(o.gamma, QL, QR, nx, ny, nz, F);
-    if (o.viscous != TY_VISC_NONE) add_viscous(m, s, o, f, F);
-#pragma unroll
-    for (int v = 0; v < 5; ++v) F[v] = S * F[v];
+#if TY_FAST
+// add_viscous times S: the same flux with theta = p/rho = r T in place of T (the gas constant
+// cancels between the conductivity mu cp / Pr and grad T), the temperature gradient contracted
+// with its normal before it is formed, Sutherland's (T/T0)^1.5 as x^2 / sqrt(x), and the
+// reciprocals by Newton-Raphson.  550 -> 215 FP64 operations a face with HLLC (plate of 87,500
+// cells: the face kernel 175 -> 72 us on GB300).
+__device__ void add_viscous_fast(const DevMesh& m, const DevState& s, const SpatOpts& o, int f, F64 S, F64* F) {
+  const size_t ld = m.ldc, lf = m.ldf;
+  const int icl = m.fc1[f], icr = m.fc2[f];
+  const double* __restrict__ q = s.prim;
+  const double* __restrict__ gl = s.grad + icl;
+  const double* __restrict__ gr = s.grad + icr;
+  const F64 hl = m.vgeo[f], hr = m.vgeo[lf + f];
+  const F64 nx = d3(m.fn, m.ldf, f, 0), ny = d3(m.fn, m.ldf, f, 1), nz = d3(m.fn, m.ldf, f, 2);
+  const F64 rL = q[icl], rR = q[icr], pL = q[ld + icl], pR = q[ld + icr];
+  const F64 iL = rcp_nr(rL), iR = rcp_nr(rR), tL = pL * iL, tR = pR * iR;
+  const F64 tH = fma(hr, tL, hl * tR);
+  F64 mu;
+  if (o.visc_law == TY_VISC_KINEMATIC) {
+    mu = F64(o.visc_kin) * fma(hr, rL, hl * rR);
+  } else {  // mu0 (T/T0)^1.5 (T0 + S) / (T + S), T = tH / r
+    const double T0 = 273.00, S0 = 110.50;
+    const F64 T = tH * F64(o.irgas), x = T * F64(1.0 / T0);
+    mu = F64(0.0000168 * (T0 + S0)) * (x * x * rsqrt_nr(x)) * rcp_nr(T + F64(S0));
   }
+  // velocity gradient at the face (CELL-AVERAGE), G n and G^T n and the divergence
+  F64 vL[3], vR[3], G[3][3];
 #pragma unroll
-  for (int v = 0; v < 5; ++v) flux[v * (size_t)m.ldf + f] = F[v];
+  for (int i = 0; i < 3; ++i) {
+    vL[i] = q[(2 + i) * ld + icl];
+    vR[i] = q[(2 + i) * ld + icr];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) G[i][j] = fma(hl, F64(gr[(6 + 3 * i + j) * ld]), hr * F64(gl[(6 + 3 * i + j) * ld]));
+  }
+  F64 mx = nx, my = ny, mz = nz, comp = 0.0;  // direction of grad theta, and the compact part
+  if (o.viscous == TY_VISC_CELLFULL) {           // compact correction along C_L C_R
+    const F64 wx = m.vgeo[2 * lf + f], wy = m.vgeo[3 * lf + f], wz = m.vgeo[4 * lf + f];
+    const F64 it = rcp_nr(fma(wx, wx, fma(wy, wy, wz * wz)));
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const F64 c = it * (vR[i] - vL[i] - fma(G[i][0], wx, fma(G[i][1], wy, G[i][2] * wz)));
+      G[i][0] = fma(c, wx, G[i][0]);
+      G[i][1] = fma(c, wy, G[i][1]);
+      G[i][2] = fma(c, wz, G[i][2]);
+    }
+    const F64 ps = it * fma(wx, nx, fma(wy, ny, wz * nz));
+    comp = ps * (tR - tL);
+    mx = fma(-ps, wx, nx); my = fma(-ps, wy, ny); mz = fma(-ps, wz, nz);
+  }
+  const F64 mS = S * mu, div = F64(2.0 / 3.0) * (G[0][0] + G[1][1] + G[2][2]);
+  const F64 n[3] = {nx, ny, nz};
+  F64 work = 0.0;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    // (G + G^T) n - 2/3 div n
+    F64 t = fma(G[i][0], nx, fma(G[i][1], ny, G[i][2] * nz));
+    t = fma(G[0][i], nx, fma(G[1][i], ny, fma(G[2][i], nz, fma(-div, n[i], t))));
+    t = t * mS;
+    F[2 + i] = F[2 + i] - t;
+    work = fma(t, fma(hr, vL[i], hl * vR[i]), work);
+  }
+  F[1] = F[1] - work;
+  if (f >= m.nfi && (m.fbc[f] == TY_BC_WALL || m.fbc[f] == TY_BC_NOSLIP)) return;  // adiabatic
+  // grad theta . m of each side: (grad p - theta grad rho) . m / rho
+  const F64 gpl = fma(F64(gl[3 * ld]), mx, fma(F64(gl[4 * ld]), my, F64(gl[5 * ld]) * mz));
+  const F64 grl = fma(F64(gl[0]), mx, fma(F64(gl[ld]), my, F64(gl[2 * ld]) * mz));
+  const F64 gpr = fma(F64(gr[3 * ld]), mx, fma(F64(gr[4 * ld]), my, F64(gr[5 * ld]) * mz));
+  const F64 grr = fma(F64(gr[0]), mx, fma(F64(gr[ld]), my, F64(gr[2 * ld]) * mz));
+  const F64 tl = iL * fma(-tL, grl, gpl), tr = iR * fma(-tR, grr, gpr);
+  F[1] = fma(-(mS * F64(o.gig1 * o.iprandtl)), fma(hl, tr, fma(hr, tl, comp)), F[1]);
 }
+#endif
 
-
+#if TY_FAST
+__device__ __forceinline__ void face_flux(const DevMesh& m, const DevState& s, const SpatOpts& o, int f,
+                                          const double* QL, const double* QR, double* __restrict__ flux) {
+  const double nx = d3(m.fn, m.ldf, f, 0), ny = d3(m.fn, m.ldf, f, 1), nz = d3(m.fn, m.ldf, f, 2);
+  const double S = m.fs[f];
+  F64 L[5], R[5], Fx[5];
+#pragma unroll
+  for (int v = 0; v < 5; ++v) { L[v] = QL[v]; R[v] = QR[v]; }
+  if (o.scheme == TY_SCH_ROE) {
+    flux_roe_fast(o, L, R, nx, ny, nz, S, Fx);
+  } else if (o.hll_family == 1) {
+    flux_hllc_fast(o, L, R, nx, ny, nz, S, Fx);
+  } else if (o.scheme == TY_SCH_RUSANOV) {
+    flux_rusanov_fast(o, L, R, nx, ny, nz, S, Fx);
+  } else {
+    double F[5];
+    if (o.hll_family == 2) flux_hlle(o, QL, QR, nx, ny, nz, F);
+    else flux_ausmm(o.gamma, QL, QR, nx, ny, nz, F);
+#pragma unroll
+    for (int v = 0; v < 5; ++v) Fx[v] = S * F[v];
+  }
+  if (o.viscous != TY_VISC_NONE) add_viscous_fast(m, s, o, f, S, Fx);
+#pragma unroll
+  for (int v = 0; v < 5; ++v) flux[v * (size_t)m.ldf + f] = Fx[v].v;
+}
+#else
 __device__ __forceinline__ void face_flux(const DevMesh& m, const DevState& s, const SpatOpts& o, int f,
                                           const double* QL, const double* QR, double* __restrict__ flux) {
   const double nx = d3(m.fn, m.ldf, f, 0), ny = d3(m.fn, m.ldf, f, 1), nz = d3(m.fn, m.ldf, f, 2);
   double F[5];
-  if constexpr (kFast) {
-    if (o.hll_family == 1) flux_hllc_fast(o, QL, QR, nx, ny, nz, F);
-    else if (o.scheme == TY_SCH_RUSANOV) flux_rusanov(o.gamma, QL, QR, nx, ny, nz, F);
-    else if (o.hll_family == 2) flux_hlle(o, QL, QR, nx, ny, nz, F);
-    else if (o.scheme == TY_SCH_AUSMM) flux_ausmm(o.gamma, QL, QR, nx, ny, nz, F);
-    else flux_roe_fast(o, QL, QR, nx, ny, nz, 1.0, F);  // unit surface
-  } else {
-    if (o.hll_family == 1) flux_hllc(o, QL, QR, nx, ny, nz, F);
-    else if (o.scheme == TY_SCH_RUSANOV) flux_rusanov(o.gamma, QL, QR, nx, ny, nz, F);
-    else if (o.hll_family == 2) flux_hlle(o, QL, QR, nx, ny, nz, F);
-    else if (o.scheme == TY_SCH_AUSMM) flux_ausmm(o.gamma, QL, QR, nx, ny, nz, F);
-    else flux_roe(o.gamma, o.entropy_fix, QL, QR, nx, ny, nz, F);
-  }
+  if (o.hll_family == 1) flux_hllc(o, QL, QR, nx, ny, nz, F);
+  else if (o.scheme == TY_SCH_RUSANOV) flux_rusanov(o.gamma, QL, QR, nx, ny, nz, F);
+  else if (o.hll_family == 2) flux_hlle(o, QL, QR, nx, ny, nz, F);
+  else if (o.scheme == TY_SCH_AUSMM) flux_ausmm(o.gamma, QL, QR, nx, ny, nz, F);
+  else flux_roe(o.gamma, o.entropy_fix, QL, QR, nx, ny, nz, F);
   if (o.viscous != TY_VISC_NONE) add_viscous(m, s, o, f, F);
   const double S = m.fs[f];
 #pragma unroll
   for (int v = 0; v < 5; ++v) flux[v * (size_t)m.ldf + f] = S * F[v];
 }
+#endif
 
 // fused face states + flux (no post-limiter)
 __global__ void __launch_bounds__(kBlock) k_face_flux(DevMesh m, DevState s, SpatOpts o) {
@@ -1049,11 +1190,6 @@ __device__ __forceinline__ long long dbits(double x) { return __double_as_longlo
 // pattern back into an FP64 comparison)
 __device__ __forceinline__ bool is_zero(double x) {
   return (((unsigned)__double2hiint(x) << 1) | (unsigned)__double2loint(x)) == 0u;
-}
-
-// |x| without the FP64 instruction of fabs
-__device__ __forceinline__ double abs_bits(double x) {
-  return __hiloint2double(__double2hiint(x) & 0x7fffffff, __double2loint(x));
 }
 
 // |x| as an FP32 number, truncated (relative error below 2^-23) on the integer pipe, when x lies
@@ -1353,7 +1489,7 @@ __global__ void __launch_bounds__(kBlock) k_face_flux_fast(DevMesh m, DevState s
 #pragma unroll
     for (int v = 0; v < 5; ++v) QR[v] = s.cr[v * lf + f];
   }
-  face_flux_fast(m, s, o, f, QL, QR, s.flux);
+  face_flux(m, s, o, f, QL, QR, s.flux);
 }
 
 // ---------------------------------------------------------------------------
