@@ -364,6 +364,14 @@ int run_step(ty_mesh* h, const RkTab& t, double dt, const unsigned long long* dt
   RkStagePlan plans[kMaxStage];
   make_plans(t, plans);
   plans[t.n - 1].store_acc = store_acc ? 1 : 0;
+  if (h->o.mode == TY_MODE_FAST) {  // the final combination starts at its first non-zero term
+    bool started = false;
+    for (int i = 0; i < t.n; ++i) {
+      plans[i].acc_init = started ? 0 : 1;
+      plans[i].has_acc = plans[i].final_stage || plans[i].c_acc != 0.0;
+      started = started || plans[i].c_acc != 0.0;
+    }
+  }
   for (int i = 0; i < t.n; ++i) plans[i].dtloc = dtloc;
   int rc = ensure_pk(h, plans, t.n);
   if (rc) return rc;
@@ -539,7 +547,7 @@ int ty_mesh_create(const ty_mesh_desc* d, int device, ty_mesh** out) {
     return bail(rc);
   // state
   DevState& s = h->s;
-  if ((rc = h->alloc(s.u0, 5 * lc)) || (rc = h->alloc(s.cur, 5 * lc)) || (rc = h->alloc(s.acc, 5 * lc)) ||
+  if ((rc = h->alloc(s.u0, 5 * lc)) || (rc = h->alloc(s.acc, 5 * lc)) ||
       (rc = h->alloc(s.prim, 5 * lc)) || (rc = h->alloc(s.grad, 15 * lc)) || (rc = h->alloc(s.ratio, 3 * lc)) ||
       (rc = h->alloc(s.flux, 5 * lf)) || (rc = h->alloc(s.res, 5 * lc)) || (rc = h->alloc(s.dtbits, 4)) ||
       (rc = h->alloc(s.stage, 5 * (size_t)nci)) ||

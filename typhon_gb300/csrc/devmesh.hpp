@@ -69,7 +69,6 @@ struct DevMesh {
 
 struct DevState {
   double* u0 = nullptr;    // [5][ldc] state at the start of the step (the solution between steps)
-  double* cur = nullptr;   // [5][ldc] state of the current stage
   double* acc = nullptr;   // [5][ldc] Runge-Kutta combination sum coef(n,s) rhs_s
   double* pk[kMaxStage + 1] = {};  // [5][ldc] partial sums of later stage states
   double* prim = nullptr;  // [5][ldc] rho, p, u, v, w (ghosts included)
@@ -102,11 +101,11 @@ struct SpatOpts {
 
 // One Runge-Kutta update applied at the end of a stage: partial sum of the state of stage
 // `target`, P_target <- (u0 or P_target) + c * R.  The partial sum of the next stage is the
-// next stage state (written to cur); later ones are kept in pk[target].
+// next stage state (its primitive variables are stored); later ones are kept in pk[target].
 struct RkOp {
   int target;   // stage index (2..nstage) whose state the term belongs to
   int from_u0;  // 1: first term, start from u0; 0: accumulate into pk[target]
-  int is_next;  // 1: target is the next stage (result goes to cur)
+  int is_next;  // 1: target is the next stage (only its primitive variables are kept)
   double c;
 };
 struct RkStagePlan {

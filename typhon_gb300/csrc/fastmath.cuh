@@ -61,6 +61,9 @@ struct F64 {
   friend __device__ __forceinline__ F64 fma(F64 a, F64 b, F64 c) { return ::fma(a.v, b.v, c.v); }
 };
 
+__device__ __forceinline__ double value(F64 a) { return a.v; }
+__device__ __forceinline__ double value(double a) { return a; }
+
 // 1/a: one third-order step from the hardware seed (3 DFMA).
 __device__ __forceinline__ double rcp_nr(double a) {
   const double x = rcp_seed(a);
