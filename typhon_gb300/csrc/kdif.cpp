@@ -4,8 +4,8 @@
 // (d.n), |d|^2) is computed once on the host in the oracle's operation order.  The implicit
 // step assembles the symmetrised system diag(V/dt) A (symmetric positive definite: A is
 // Typhon's DLU matrix I + dt/V J with the compact Jacobian J_R = -k (d.n) / (Cp |d|^2),
-// J_L = -J_R) and solves it by Jacobi-preconditioned conjugate gradients in FP64 (one fused
-// pair of launches per iteration, kdif.cuh), by the same iteration on FP32 conductances until
+// J_L = -J_R) and solves it by Jacobi-preconditioned conjugate gradients in FP64 (one persistent
+// kernel, kdif.cuh), by the same iteration on FP32 conductances until
 // 1e-6 and then on FP64 ones (mixed), or by FP32 conjugate gradients inside FP64 iterative
 // refinement.
 #include <algorithm>
@@ -201,34 +201,33 @@ int ty_kdif_implicit_step(ty_mesh* h, double dt, const ty_kdif_solve* s, ty_kdif
     // residual is below kSwitch, then restarts on the FP64 conductances from the FP64
     // system's residual
     constexpr double kSwitch = 1e-6;
-    bool a32 = s->solver == TY_KSOLVE_CG_MIXED && s->tol < kSwitch;
+    PcgArgs a{};
+    a.start = 1;
+    a.a32 = s->solver == TY_KSOLVE_CG_MIXED && s->tol < kSwitch ? 1 : 0;
+    a.max_it = s->max_it;
+    a.check = check;
+    a.tol = s->tol;
+    a.sw = kSwitch;
     TY_CU(KD_CALL(h, kdif_ell_build, m, k, dt, q));
-    TY_CU(KD_CALL(h, kdif_fcg_a, m, k, 1, q));
-    TY_CU(KD_CALL(h, kdif_fcg_b, m, k, 1, a32 ? 1 : 0, q));
-    if (int rc = fetch(h, 3, 1)) return rc;
-    const double b2 = P[3];
     double rel = 0.0;
     int it = 0;
-    if (b2 > 0.0) {
-      rel = 1.0;
-      while (it < s->max_it) {
-        TY_CU(KD_CALL(h, kdif_fcg_a, m, k, 0, q));
-        TY_CU(KD_CALL(h, kdif_fcg_b, m, k, 0, a32 ? 1 : 0, q));
-        ++it;
-        if (it % check == 0 || it == s->max_it) {
-          if (int rc = fetch(h, 11, 1)) return rc;
-          rel = std::sqrt(P[11] / b2);
-          if (a32 && rel < kSwitch) {  // restart on the FP64 matrix from the true residual
-            TY_CU(KD_CALL(h, kdif_fcg_replace, m, k, q));
-            TY_CU(KD_CALL(h, kdif_fcg_a, m, k, 2, q));
-            TY_CU(KD_CALL(h, kdif_fcg_b, m, k, 1, 0, q));
-            a32 = false;
-            st->refinements = 1;
-            continue;
-          }
-          if (!a32 && rel < s->tol) break;
-        }
+    for (;;) {
+      a.it0 = it;
+      a.it1 = std::min(s->max_it, it + kPcgChunk);
+      TY_CU(KD_CALL(h, kdif_pcg, m, k, a, q));
+      unsigned timed_out[2] = {0, 0};
+      TY_CU(cudaMemcpyAsync(timed_out, k.count, sizeof(timed_out), cudaMemcpyDeviceToHost, q));
+      if (int rc = fetch(h, kPcgAlpha, 16 - kPcgAlpha)) return rc;
+      if (timed_out[1]) {
+        tyi::set_error("ty_kdif_implicit_step: the grid barrier of the conjugate gradients timed out");
+        return TY_ERR_CUDA;
       }
+      it = (int)P[kPcgIt];
+      rel = P[kPcgB2] > 0.0 ? std::sqrt(P[kPcgRR] / P[kPcgB2]) : 0.0;
+      if (P[kPcgSwitched] != 0.0) st->refinements = 1;
+      a.a32 = P[kPcgA32] != 0.0 ? 1 : 0;
+      a.start = 0;
+      if (P[kPcgDone] != 0.0 || it >= s->max_it) break;
     }
     st->iterations = it;
     st->rel_res = rel;

@@ -264,17 +264,274 @@ __global__ void k_kdif_update_T(DevMesh m, KdifState k) {
   k.T[c] = k.T[c] + k.x[c] / k.cp;
 }
 
-// ---- fused conjugate gradients (single reduction per iteration) ----
+// ---- fused conjugate gradients in one persistent kernel ----
 // Chronopoulos and Gear's arrangement of Jacobi-preconditioned CG: with u = D^-1 r, w = S u,
-// and p and s = S p carried by recurrences, both inner products of an iteration,
-// gamma = r.u and delta = w.u, come from the same iterate, so an iteration is two launches
-// and no host round trip:
-//   A: x += alpha p, r -= alpha s, u = r / diag; gamma, r.r;   beta = gamma / gamma_old
-//   B: w = S u, p = u + beta p, s = w + beta s; delta;         alpha = gamma / (delta - beta gamma / alpha_old)
-// Each launch reduces in a fixed grid (block sums, then the last block to finish sums the
-// block partials in block order): deterministic.  Scalars: scal[8] gamma, [9] alpha,
-// [10] beta, [11] r.r, [12] delta.
-constexpr int kFcgGamma = 8, kFcgAlpha = 9, kFcgBeta = 10, kFcgRR = 11, kFcgDelta = 12;
+// and p and s = S p carried by recurrences, the inner products of an iteration, gamma = r.u,
+// delta = w.u (and r.r when the residual is checked), come from the same iterate:
+//   p = u + beta p, s = w + beta s, x += alpha p, r -= alpha s, u = r / diag;  barrier
+//   w = S u; gamma, delta;  barrier;  beta = gamma / gamma_old,
+//   alpha = gamma / (delta - beta gamma / alpha_old)
+// One cooperative launch runs up to kPcgChunk iterations: the grid is resident, every thread
+// owns up to K cells whose r, p, s and w stay in registers, only u travels through L2 (z), and
+// the scalars are recomputed by every block from the blocks' partial sums, in block order
+// (deterministic).  Separate launches cost 9 us of reduction tails and gaps each, whatever the
+// mesh.  On GB300, us per iteration: 13,182 cells 25 -> 7.1, 750,000 cells 54 -> 29 (FP64 pipe:
+// 17 operations per cell, 20 us), 2,058,000 cells (vectors in memory, K = 0) 105 -> 80.
+constexpr int kPcgThreads = 512;
+constexpr int kPcgPart = 3;  // partial sums per block: gamma, delta, r.r
+constexpr int kPcgBlocks = 4 * 160;
+
+// Barrier over a resident grid: `goal` arrivals in total.  Bounded: false after about two
+// seconds (the caller leaves the kernel and the host sees the error word).
+__device__ __forceinline__ bool grid_barrier(unsigned* count, unsigned goal) {
+  __shared__ int ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(count, 1u);
+    unsigned v = 0;
+    int spins = 0;
+    do {
+      asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+    } while (v < goal && ++spins < (1 << 22));
+    ok = v >= goal;
+    __threadfence();
+  }
+  __syncthreads();
+  return ok != 0;
+}
+
+// Sums of the N per-thread values over the grid, valid in thread 0.  FP64 instructions are
+// scarce (one per 64 clocks, SM quarter and warp), so no warp does what one can do: the values
+// meet in shared memory, 128 threads per value add them down to 128, one warp per value to one;
+// the blocks' sums meet in part and every block adds them in block order.  False when the
+// barrier ran out.
+template <int N>
+__device__ __forceinline__ bool grid_sum(const double (&v)[N], double* tot, double* part, unsigned* count, unsigned goal) {
+  __shared__ double sh[N][kPcgThreads];
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5, nt = blockDim.x;
+#pragma unroll
+  for (int q = 0; q < N; ++q) sh[q][t] = v[q];
+  __syncthreads();
+  if (nt > 128) {
+    const int q = t >> 7, i = t & 127;
+    if (q < N) {
+      double a = sh[q][i];
+      for (int j = i + 128; j < nt; j += 128) a += sh[q][j];
+      sh[q][i] = a;
+    }
+    __syncthreads();
+    if (nt < 128 * N) {  // fewer groups of 128 threads than values
+      for (int r = nt >> 7; r < N; ++r) {
+        if (t < 128) {
+          double a = sh[r][t];
+          for (int j = t + 128; j < nt; j += 128) a += sh[r][j];
+          sh[r][t] = a;
+        }
+      }
+      __syncthreads();
+    }
+  }
+  if (wid < N) {
+    double a = sh[wid][lane];
+#pragma unroll
+    for (int i = 32; i < 128; i += 32) a += sh[wid][lane + i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+    if (lane == 0) part[wid * kPcgBlocks + blockIdx.x] = a;
+  }
+  if (!grid_barrier(count, goal)) return false;
+  if (wid < N) {
+    double a = 0.0;
+    for (int i = lane; i < (int)gridDim.x; i += 32) a += __ldcg(part + wid * kPcgBlocks + i);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+    if (lane == 0) tot[wid] = a;
+  }
+  __syncthreads();
+  return true;
+}
+
+template <int K>
+__global__ void __launch_bounds__(kPcgThreads, K > 0 ? 1 : 2) k_kdif_pcg(int n, int ns, KdifState k, PcgArgs a) {
+  constexpr int KR = K > 0 ? K : 1;
+  double R[KR], P[KR], Q[KR], W[KR];  // r, p, s = S p and w = S u of this thread's cells
+  const int first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  const int cells = K > 0 ? K : (n - first + stride - 1) / stride;
+  unsigned goal = 0;
+  bool a32 = a.a32 != 0;
+  int it = a.it0, done = 0, switched = 0;
+  double alpha, beta, gamma, b2, rr = 0.0;
+  // neighbour lists of this thread's cells, [j][slot][thread]: read every iteration, and the
+  // address of the gather that the FP64 chain waits for
+  extern __shared__ int nbs[];
+#define TY_EACH_CELL                      \
+  _Pragma("unroll") for (int j = 0; j < cells; ++j) { \
+    const int i = first + j * stride;     \
+    const int q = K > 0 ? j : 0;          \
+    (void)q;                              \
+    if (i < n) {
+#define TY_END_CELL \
+    }               \
+  }
+  double* gr = k.r;
+  double* gp = k.p;
+  double* gs = k.s;
+  double* gw = k.q;
+  // u (already in z, visible to every block) -> w and this thread's sums; one copy per precision
+  // of the conductances (a conversion, even predicated off, occupies the FP64 pipe)
+  auto product_of = [&](auto* cond, double (&v)[kPcgPart], bool want_rr) {
+    F64 g = 0.0, dl = 0.0;
+    TY_EACH_CELL
+      const F64 uc = __ldcg(k.z + i);
+      F64 w = F64(__ldg(k.ell_m + i)) * uc;
+      for (int s0 = 0; s0 < ns; s0 += 4) {  // four gathers in flight before the first is used
+        F64 c[4], zn[4];
+#pragma unroll
+        for (int d = 0; d < 4; ++d) {
+          const int sl = s0 + d < ns ? s0 + d : ns - 1;
+          const size_t e = (size_t)sl * n + i;
+          const int nb = K > 0 ? nbs[(j * ns + sl) * blockDim.x + threadIdx.x] : __ldg(k.ell_nb + e);
+          c[d] = (double)__ldg(cond + e);
+          zn[d] = __ldcg(k.z + nb);
+        }
+#pragma unroll
+        for (int d = 0; d < 4; ++d)
+          if (s0 + d < ns) w = fma(c[d], uc - zn[d], w);
+      }
+      const F64 r = K > 0 ? R[q] : gr[i];
+      if (K > 0) W[q] = w.v; else gw[i] = w.v;
+      g = fma(r, uc, g);
+      dl = fma(w, uc, dl);
+    TY_END_CELL
+    v[0] = g.v;
+    v[1] = dl.v;
+    v[2] = 0.0;
+    if (want_rr) {  // every `check` iterations only
+      TY_EACH_CELL
+        const double r = K > 0 ? R[q] : gr[i];
+        v[2] = fma(r, r, v[2]);
+      TY_END_CELL
+    }
+  };
+  auto product = [&](double (&v)[kPcgPart], bool want_rr) {
+    if (a32) product_of(k.ell_a32, v, want_rr);
+    else product_of(k.ell_a, v, want_rr);
+  };
+  double v[kPcgPart];
+  // scalars of the next step, by one thread: sh[0..2] the sums, sh[3] alpha, sh[4] beta, with
+  // 1/alpha = delta/gamma - beta/alpha_old
+  __shared__ double sh[5];
+  double ialpha = 0.0, igamma = 0.0;  // thread 0's: 1/alpha, 1/gamma
+  auto scalars = [&](bool first_step) {
+    if (threadIdx.x == 0) {
+      const double ig = rcp_nr(sh[0]), be = first_step ? 0.0 : sh[0] * igamma;
+      ialpha = fma(sh[1], ig, -(be * ialpha));
+      igamma = ig;
+      sh[3] = rcp_nr(ialpha);
+      sh[4] = be;
+    }
+    __syncthreads();
+    gamma = sh[0];
+    alpha = sh[3];
+    beta = sh[4];
+  };
+  // the iteration's start from the residual in R (or r): u, w, the sums and the first step
+  auto restart = [&]() -> bool {
+    TY_EACH_CELL
+      const double r = K > 0 ? R[q] : gr[i];
+      k.z[i] = r * __ldg(k.dinv + i);
+    TY_END_CELL
+    if (!grid_barrier(k.count, goal += gridDim.x)) return false;
+    product(v, true);
+    if (!grid_sum(v, sh, k.part, k.count, goal += gridDim.x)) return false;
+    scalars(true);
+    return true;
+  };
+  if (K > 0) {
+    TY_EACH_CELL
+      for (int sl = 0; sl < ns; ++sl)
+        nbs[(j * ns + sl) * blockDim.x + threadIdx.x] = __ldg(k.ell_nb + (size_t)sl * n + i);
+    TY_END_CELL
+  }
+  if (a.start) {
+    TY_EACH_CELL
+      k.x[i] = 0.0;
+      const double b = k.bal[i];
+      if (K > 0) { R[q] = b; P[q] = 0.0; Q[q] = 0.0; }
+      else { gr[i] = b; gp[i] = 0.0; gs[i] = 0.0; }
+    TY_END_CELL
+    if (!restart()) { if (threadIdx.x == 0) k.count[1] = 1u; return; }
+    b2 = rr = sh[2];
+    if (!(b2 > 0.0)) done = 1;  // zero right-hand side
+  } else {
+    alpha = k.scal[kPcgAlpha]; beta = k.scal[kPcgBeta]; gamma = k.scal[kPcgGamma]; b2 = k.scal[kPcgB2];
+    ialpha = 1.0 / alpha;
+    igamma = 1.0 / gamma;
+    if (K > 0) {
+      TY_EACH_CELL
+        R[q] = gr[i]; P[q] = gp[i]; Q[q] = gs[i]; W[q] = gw[i];
+      TY_END_CELL
+    }
+  }
+  while (!done && it < a.it1) {
+    TY_EACH_CELL
+      const double u = __ldcg(k.z + i), w = K > 0 ? W[q] : gw[i];
+      const double p = fma(beta, K > 0 ? P[q] : gp[i], u), s = fma(beta, K > 0 ? Q[q] : gs[i], w);
+      const double r = fma(-alpha, s, K > 0 ? R[q] : gr[i]);
+      k.x[i] = fma(alpha, p, k.x[i]);
+      k.z[i] = (F64(r) * F64(__ldg(k.dinv + i))).v;
+      if (K > 0) { P[q] = p; Q[q] = s; R[q] = r; }
+      else { gp[i] = p; gs[i] = s; gr[i] = r; }
+    TY_END_CELL
+    ++it;
+    const bool check = it % a.check == 0 || it == a.max_it;
+    if (!grid_barrier(k.count, goal += gridDim.x)) { if (threadIdx.x == 0) k.count[1] = 1u; return; }
+    product(v, check);
+    if (!grid_sum(v, sh, k.part, k.count, goal += gridDim.x)) { if (threadIdx.x == 0) k.count[1] = 1u; return; }
+    scalars(false);
+    if (check) {
+      rr = sh[2];
+      const double rel = sqrt(rr / b2);
+      if (a32 && rel < a.sw) {
+        // restart on the FP64 conductances from the true residual r = b - S x (continuing the
+        // old directions on the changed operator loses their conjugacy: on a stiff system the
+        // iteration stagnates)
+        a32 = false;
+        switched = 1;
+        TY_EACH_CELL
+          k.z[i] = k.x[i];
+        TY_END_CELL
+        bool ok = grid_barrier(k.count, goal += gridDim.x);
+        if (ok) {
+          double sum[kPcgPart];
+          product(sum, false);  // w = S x
+          TY_EACH_CELL
+            const double r = k.bal[i] - (K > 0 ? W[q] : gw[i]);
+            if (K > 0) { R[q] = r; P[q] = 0.0; Q[q] = 0.0; }
+            else { gr[i] = r; gp[i] = 0.0; gs[i] = 0.0; }
+          TY_END_CELL
+          ok = grid_barrier(k.count, goal += gridDim.x) && restart();
+        }
+        if (!ok) { if (threadIdx.x == 0) k.count[1] = 1u; return; }
+      } else if (!a32 && rel < a.tol) {
+        done = 1;
+      }
+    }
+  }
+  if (K > 0 && !done) {
+    TY_EACH_CELL
+      gr[i] = R[q]; gp[i] = P[q]; gs[i] = Q[q]; gw[i] = W[q];
+    TY_END_CELL
+  }
+#undef TY_EACH_CELL
+#undef TY_END_CELL
+  if (first == 0) {
+    k.scal[kPcgAlpha] = alpha; k.scal[kPcgBeta] = beta; k.scal[kPcgGamma] = gamma; k.scal[kPcgB2] = b2;
+    k.scal[kPcgRR] = rr; k.scal[kPcgIt] = it; k.scal[kPcgDone] = done;
+    k.scal[kPcgA32] = a32 ? 1.0 : 0.0; k.scal[kPcgSwitched] = switched;
+  }
+}
 
 // the symmetrised matrix in difference form (kdif.hpp) and the Jacobi inverse
 __global__ void __launch_bounds__(kBlock) k_kdif_ell(DevMesh m, KdifState k, double dt) {
@@ -300,111 +557,51 @@ __global__ void __launch_bounds__(kBlock) k_kdif_ell(DevMesh m, KdifState k, dou
   k.dinv[c] = 1.0 / d;
 }
 
-// last block of a launch: true in every thread of the block that finished last
-__device__ __forceinline__ bool kd_last_block(unsigned* count) {
-  __shared__ bool last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(count, 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (last) __threadfence();
-  return last;
-}
-// sum of the block partials part[0..nb) in block order (every thread; valid in thread 0)
-__device__ __forceinline__ double kd_sum_partials(const double* part, int nb) {
-  double a = 0.0;
-  for (int i = threadIdx.x; i < nb; i += kRedThreads) a += __ldcg(part + i);
-  return block_sum(a);
-}
-
-// A (first = 1: start, x = 0, r = b; first = 2: restart from the current x and r)
-__global__ void __launch_bounds__(kRedThreads) k_kdif_fcg_a(int n, KdifState k, int first) {
-  const double alpha = first ? 0.0 : k.scal[kFcgAlpha];
-  double g = 0.0, rr = 0.0;
-  for (int i = blockIdx.x * kRedThreads + threadIdx.x; i < n; i += gridDim.x * kRedThreads) {
-    double xi, ri;
-    if (first == 1) { xi = 0.0; ri = k.bal[i]; }
-    else if (first == 2) { xi = k.x[i]; ri = k.r[i]; }
-    else { xi = k.x[i] + alpha * k.p[i]; ri = k.r[i] - alpha * k.s[i]; }
-    const double ui = ri * k.dinv[i];
-    k.x[i] = xi; k.r[i] = ri; k.z[i] = ui;
-    g += ri * ui;
-    rr += ri * ri;
-  }
-  g = block_sum(g);
-  if (threadIdx.x == 0) k.part[blockIdx.x] = g;
-  rr = block_sum(rr);
-  if (threadIdx.x == 0) k.part[kRedBlocks + blockIdx.x] = rr;
-  if (!kd_last_block(k.count)) return;
-  const double gt = kd_sum_partials(k.part, gridDim.x);
-  const double rt = kd_sum_partials(k.part + kRedBlocks, gridDim.x);
-  if (threadIdx.x == 0) {
-    k.scal[kFcgBeta] = first ? 0.0 : gt / k.scal[kFcgGamma];
-    k.scal[kFcgGamma] = gt;
-    k.scal[kFcgRR] = rt;
-    if (first == 1) k.scal[3] = rt;   // |b|^2
-    *k.count = 0u;
-  }
-}
-
-// B: w = S u with FP64 (A32 = false) or FP32 (A32 = true) conductances
-template <bool A32>
-__global__ void __launch_bounds__(kRedThreads) k_kdif_fcg_b(int n, int ns, KdifState k, int first) {
-  const double beta = k.scal[kFcgBeta];
-  double dl = 0.0;
-  for (int c = blockIdx.x * kRedThreads + threadIdx.x; c < n; c += gridDim.x * kRedThreads) {
-    const double uc = k.z[c];
-    double w = k.ell_m[c] * uc;
-    for (int sl = 0; sl < ns; ++sl) {
-      const double a = A32 ? (double)k.ell_a32[sl * (size_t)n + c] : k.ell_a[sl * (size_t)n + c];
-      w = fma(a, uc - k.z[k.ell_nb[sl * (size_t)n + c]], w);
-    }
-    if (first) { k.p[c] = uc; k.s[c] = w; }
-    else { k.p[c] = fma(beta, k.p[c], uc); k.s[c] = fma(beta, k.s[c], w); }
-    dl += w * uc;
-  }
-  dl = block_sum(dl);
-  if (threadIdx.x == 0) k.part[blockIdx.x] = dl;
-  if (!kd_last_block(k.count + 1)) return;
-  const double dt = kd_sum_partials(k.part, gridDim.x);
-  if (threadIdx.x == 0) {
-    const double gm = k.scal[kFcgGamma];
-    k.scal[kFcgDelta] = dt;
-    k.scal[kFcgAlpha] = first ? gm / dt : gm / (dt - beta * gm / k.scal[kFcgAlpha]);
-    k.count[1] = 0u;
-  }
-}
-
-// the true residual r = b - S x of the FP64 system, from which the iteration restarts when
-// the operator changes from FP32 to FP64 conductances (continuing the old directions on the
-// changed operator loses their conjugacy: on this stiff system the iteration stagnates)
-__global__ void __launch_bounds__(kRedThreads) k_kdif_fcg_replace(int n, int ns, KdifState k) {
-  for (int c = blockIdx.x * kRedThreads + threadIdx.x; c < n; c += gridDim.x * kRedThreads) {
-    const double xc = k.x[c];
-    double sx = k.ell_m[c] * xc;
-    for (int sl = 0; sl < ns; ++sl)
-      sx = fma(k.ell_a[sl * (size_t)n + c], xc - k.x[k.ell_nb[sl * (size_t)n + c]], sx);
-    k.r[c] = k.bal[c] - sx;
-  }
-}
-
 // ---- launchers ----
 cudaError_t kdif_ell_build(const DevMesh& m, const KdifState& k, double dt, cudaStream_t st) {
   k_kdif_ell<<<nblk(m.nci), kBlock, 0, st>>>(m, k, dt);
   return cudaGetLastError();
 }
-cudaError_t kdif_fcg_a(const DevMesh& m, const KdifState& k, int first, cudaStream_t st) {
-  k_kdif_fcg_a<<<red_grid(m.nci), kRedThreads, 0, st>>>(m.nci, k, first);
-  return cudaGetLastError();
+template <int K>
+cudaError_t pcg_launch(int n, int ns, const KdifState& k, const PcgArgs& a, int threads, cudaStream_t st) {
+  int dev = 0, sms = 0, per = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const size_t lists = (size_t)K * ns * threads * sizeof(int);
+  cudaError_t e = cudaFuncSetAttribute(k_kdif_pcg<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lists);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_kdif_pcg<K>, threads, lists);
+  if (e != cudaSuccess) return e;
+  if (per < 1) return cudaErrorCooperativeLaunchTooLarge;
+  const int want = (n + threads * std::max(K, 1) - 1) / (threads * std::max(K, 1));
+  const int grid = std::max(1, std::min(want, std::min(K > 0 ? sms : sms * per, kPcgBlocks)));
+  int nn = n, nns = ns;
+  KdifState kk = k;
+  PcgArgs aa = a;
+  void* args[] = {&nn, &nns, &kk, &aa};
+  if ((e = cudaMemsetAsync(k.count, 0, 2 * sizeof(unsigned), st)) != cudaSuccess) return e;
+  return cudaLaunchCooperativeKernel((const void*)k_kdif_pcg<K>, dim3(grid), dim3(threads), args, lists, st);
 }
-cudaError_t kdif_fcg_b(const DevMesh& m, const KdifState& k, int first, int f32, cudaStream_t st) {
-  if (f32) k_kdif_fcg_b<true><<<red_grid(m.nci), kRedThreads, 0, st>>>(m.nci, m.nslot, k, first);
-  else k_kdif_fcg_b<false><<<red_grid(m.nci), kRedThreads, 0, st>>>(m.nci, m.nslot, k, first);
-  return cudaGetLastError();
-}
-cudaError_t kdif_fcg_replace(const DevMesh& m, const KdifState& k, cudaStream_t st) {
-  k_kdif_fcg_replace<<<red_grid(m.nci), kRedThreads, 0, st>>>(m.nci, m.nslot, k);
-  return cudaGetLastError();
+
+// One block of up to 512 threads per SM and K cells per thread, K the smallest of the list that
+// covers the mesh (152 x 512 x 12 = 934,000 cells on GB300), with the block cut to 128 or 256
+// threads where that already spreads the mesh over every SM; beyond that the vectors stay in
+// memory and the grid takes as many blocks as are resident.
+cudaError_t kdif_pcg(const DevMesh& m, const KdifState& k, const PcgArgs& a, cudaStream_t st) {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const long n = m.nci;
+  if (n <= 128L * sms) return pcg_launch<1>(m.nci, m.nslot, k, a, 128, st);
+  if (n <= 256L * sms) return pcg_launch<1>(m.nci, m.nslot, k, a, 256, st);
+  const long per = (n + 512L * sms - 1) / (512L * sms);
+  if (per <= 1) return pcg_launch<1>(m.nci, m.nslot, k, a, 512, st);
+  if (per <= 2) return pcg_launch<2>(m.nci, m.nslot, k, a, 512, st);
+  if (per <= 4) return pcg_launch<4>(m.nci, m.nslot, k, a, 512, st);
+  if (per <= 6) return pcg_launch<6>(m.nci, m.nslot, k, a, 512, st);
+  if (per <= 8) return pcg_launch<8>(m.nci, m.nslot, k, a, 512, st);
+  if (per <= 10) return pcg_launch<10>(m.nci, m.nslot, k, a, 512, st);
+  if (per <= 12) return pcg_launch<12>(m.nci, m.nslot, k, a, 512, st);
+  return pcg_launch<0>(m.nci, m.nslot, k, a, 512, st);
 }
 
 cudaError_t kdif_residual(const DevMesh& m, const KdifState& k, double dt, cudaStream_t st) {

@@ -42,8 +42,20 @@ struct KdifState {
   int* ell_nb = nullptr;        // [nslot][nci]
   double* dinv = nullptr;       // [nci] 1 / diagonal (Jacobi)
   double* s = nullptr;          // [nci] S p (the single-reduction recurrence)
-  unsigned* count = nullptr;    // [2] finished blocks of the two fused kernels (last block reduces)
+  unsigned* count = nullptr;    // [2] arrivals at the persistent kernel's barrier; its error word
 };
+
+// Arguments of the persistent conjugate-gradient kernel: iterations it0 < it <= it1 of at most
+// max_it, from scratch (start) or from the state of the previous launch; the residual is
+// checked every `check` iterations against tol, or against sw while on FP32 conductances (a32).
+struct PcgArgs {
+  int start, a32, it0, it1, max_it, check;
+  double tol, sw;
+};
+constexpr int kPcgChunk = 1000;  // iterations per launch (a launch stays below a tenth of a second)
+// its scalars in KdifState::scal
+constexpr int kPcgAlpha = 7, kPcgBeta = 8, kPcgGamma = 9, kPcgB2 = 10, kPcgRR = 11, kPcgIt = 12, kPcgDone = 13,
+              kPcgA32 = 14, kPcgSwitched = 15;
 
 #define TY_DECLARE_KDIF(NS)                                                                          \
   namespace NS {                                                                                     \
@@ -53,9 +65,7 @@ struct KdifState {
                           cudaStream_t st);                                                           \
   cudaError_t kdif_cg_start(const DevMesh& m, const KdifState& k, int f32, cudaStream_t st);          \
   cudaError_t kdif_ell_build(const DevMesh& m, const KdifState& k, double dt, cudaStream_t st);         \
-  cudaError_t kdif_fcg_a(const DevMesh& m, const KdifState& k, int first, cudaStream_t st);              \
-  cudaError_t kdif_fcg_b(const DevMesh& m, const KdifState& k, int first, int f32, cudaStream_t st);     \
-  cudaError_t kdif_fcg_replace(const DevMesh& m, const KdifState& k, cudaStream_t st);                  \
+  cudaError_t kdif_pcg(const DevMesh& m, const KdifState& k, const PcgArgs& a, cudaStream_t st);         \
   cudaError_t kdif_cg_iter(const DevMesh& m, const KdifState& k, int f32, cudaStream_t st);           \
   cudaError_t kdif_residual64(const DevMesh& m, const KdifState& k, cudaStream_t st);                 \
   cudaError_t kdif_refine(const DevMesh& m, const KdifState& k, cudaStream_t st);                     \
