@@ -10,7 +10,7 @@
 //   3. linear solve (implicit_solve.f90:39-86), then U += dU.
 // Solvers of step 3:
 //   TY_KRYLOV_GMRES   Typhon's bdlu_gmres (SOURCE/MATH/bdlu_gmres.f90:50-217): restarted
-//                     GMRES(NKRYLOV), modified Gram-Schmidt, Givens rotations, x0 = b/diag,
+//                     GMRES(NKRYLOV), modified Gram-Schmidt (two reductions a vector), Givens rotations, x0 = b/diag,
 //                     its stopping test and restart limit, no preconditioner, FP64.
 //   TY_KRYLOV_FGMRES  flexible GMRES(m) with right block-Jacobi preconditioning on the
 //                     assembled BDLU matrix (new), its basis orthogonalised through a measured
@@ -89,10 +89,11 @@ int build_lists(ty_mesh* h) {
       (rc = h->alloc(im.dtloc, (size_t)nci)) || (rc = h->alloc(im.jacL, (size_t)m.nf * kBlk)) ||
       (rc = h->alloc(im.jacR, (size_t)m.nf * kBlk)) || (rc = h->alloc(im.b, 5 * (size_t)nci)) ||
       (rc = h->alloc(im.x, 5 * (size_t)nci)) || (rc = h->alloc(im.r, 5 * (size_t)nci)) ||
-      (rc = h->alloc(im.w, 5 * (size_t)nci)) || (rc = h->alloc(im.part, (size_t)(kMaxKrylov + 1) * kRedBlocks)) ||
-      (rc = h->alloc(im.scal, (size_t)kScalCount)) || (rc = h->alloc(im.done, 1)))
+      (rc = h->alloc(im.w, 5 * (size_t)nci)) || (rc = h->alloc(im.part, (size_t)(2 * kMaxKrylov + 1) * kRedBlocks / 2 + kRedBlocks)) ||
+      (rc = h->alloc(im.scal, (size_t)kScalCount)) || (rc = h->alloc(im.done, 2)) ||
+      (rc = h->alloc(im.mgs_L, (size_t)(kMaxKrylov + 1) * kMaxKrylov)))
     return rc;
-  IMP_CU(cudaMemset(im.done, 0, sizeof(unsigned)));
+  IMP_CU(cudaMemset(im.done, 0, 2 * sizeof(unsigned)));
   IMP_CU(cudaMemcpy(im.cfo, cfo.data(), cfo.size() * sizeof(int), cudaMemcpyHostToDevice));
   IMP_CU(cudaMemcpy(im.cfon, cfon.data(), cfon.size() * sizeof(int), cudaMemcpyHostToDevice));
   if (!im.pinned && cudaMallocHost((void**)&im.pinned, kScalCount * sizeof(double)) != cudaSuccess)
@@ -230,7 +231,7 @@ int gmres_typhon(ty_mesh* h, const ty_imp_params* p, ty_imp_stats* st) {
     IMP_CU(IMP_CALL(h, imp_dot, im.r, im.r, n, im.part, im.scal + kScalMisc, s));
     if (int rc = fetch(h, kScalMisc, 1)) return rc;
     const double beta = std::sqrt(P[kScalMisc]);
-    double fact = 1.0 / beta;
+    const double fact = 1.0 / beta;
     IMP_CU(IMP_CALL(h, imp_scale, im.r, fact, V(0), n, s));
     std::fill(ss.begin(), ss.end(), 0.0);
     ss[1] = beta;
@@ -239,10 +240,8 @@ int gmres_typhon(ty_mesh* h, const ty_imp_params* p, ty_imp_stats* st) {
     for (jk = 1; jk <= nk; ++jk) {
       IMP_CU(IMP_CALL(h, imp_matvec, m, im, V(jk - 1), nullptr, im.w, s, &h->prof));
       ++matvecs;
-      for (int ik = 1; ik <= jk; ++ik)  // h(ik,jk) = (w, v_ik) after w -= h(ik-1,jk) v_(ik-1)
-        IMP_CU(IMP_CALL(h, imp_mgs_pass, ik > 1 ? V(ik - 2) : nullptr, im.scal + std::max(ik - 2, 0), im.w, V(ik - 1), n,
-                        im.part, im.scal + ik - 1, s));
-      IMP_CU(IMP_CALL(h, imp_mgs_pass, V(jk - 1), im.scal + jk - 1, im.w, nullptr, n, im.part, im.scal + jk, s));
+      // h(ik,jk) = (w, v_ik) after w -= h(ik-1,jk) v_(ik-1); h(jk+1,jk)^2 = (w, w); V(jk) = w / h(jk+1,jk)
+      IMP_CU(IMP_CALL(h, imp_mgs_column, im.w, im.V, n, jk, im.mgs_L, im.part, im.scal, im.done + 1, s));
       if (int rc = fetch(h, 0, jk + 1)) return rc;
       for (int ik = 1; ik <= jk; ++ik) H(ik, jk) = P[ik - 1];
       H(jk + 1, jk) = std::sqrt(P[jk]);
@@ -252,10 +251,6 @@ int gmres_typhon(ty_mesh* h, const ty_imp_params* p, ty_imp_stats* st) {
         H(ik + 1, jk) = -qs[ik] * tmp + qc[ik] * H(ik + 1, jk);
       }
       if (H(jk + 1, jk) > eps * 10 * normp1) {
-        if (jk < nk) {
-          fact = 1.0 / H(jk + 1, jk);
-          IMP_CU(IMP_CALL(h, imp_scale, im.w, fact, V(jk), n, s));
-        }
         if (H(jk, jk) == 0) break;
         double tmp = std::sqrt(H(jk, jk) * H(jk, jk) + H(jk + 1, jk) * H(jk + 1, jk));
         qc[jk] = H(jk, jk) / tmp;
@@ -284,6 +279,13 @@ int gmres_typhon(ty_mesh* h, const ty_imp_params* p, ty_imp_stats* st) {
     ss[nkk + 1] = std::sqrt(P[kScalMisc]);
     errgmres = ss[nkk + 1] / normp1;
     nit = nit + 1;
+  }
+  unsigned timed_out = 0;
+  IMP_CU(cudaMemcpy(&timed_out, im.done + 1, sizeof(unsigned), cudaMemcpyDeviceToHost));
+  if (timed_out) {
+    IMP_CU(cudaMemset(im.done + 1, 0, sizeof(unsigned)));
+    tyi::set_error("ty_implicit_step: the Gram-Schmidt kernel's exchange timed out");
+    return TY_ERR_CUDA;
   }
   st->restarts = nit;
   st->matvecs = matvecs;

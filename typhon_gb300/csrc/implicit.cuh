@@ -520,6 +520,43 @@ __global__ void __launch_bounds__(128) k_imp_matvec(DevMesh m, ImpState im, cons
   }
 }
 
+// The same with one thread per row (five consecutive threads a cell, 32 cells a block): chains a
+// fifth as long, so that small meshes fill the SM quarters' FP64 pipes better; the order within
+// a row is the same.
+constexpr int kRowCells = 32;
+__global__ void __launch_bounds__(5 * kRowCells) k_imp_matvec_row(DevMesh m, ImpState im, const double* __restrict__ x,
+                                                               const double* __restrict__ z, double* __restrict__ y) {
+  const int lc = threadIdx.x / 5, i = threadIdx.x - 5 * lc;
+  const int c = blockIdx.x * kRowCells + lc;
+  if (c >= m.nci) return;
+  const size_t n = m.nci;
+  int e = m.nslot > 0 ? im.cfo[c] : -1, nb = e >= 0 ? im.cfon[c] : 0;
+  double acc = z ? z[5 * (size_t)c + i] : 0.0;
+  // the row's product with a block is added (y = A x) or subtracted
+  auto row = [&](const double* __restrict__ A, const double* __restrict__ v, bool first) {
+    double a[5], q[5];
+#pragma unroll
+    for (int j = 0; j < 5; ++j) { a[j] = __ldg(A + 5 * i + j); q[j] = v[j]; }
+    double s = 0.0;
+#pragma unroll
+    for (int j = 0; j < 5; ++j) s = s + a[j] * q[j];
+    acc = z ? acc - s : (first ? s : acc + s);
+  };
+  row(im.diag + (size_t)c * kBlk, x + 5 * (size_t)c, true);
+  for (int sl = 0; sl < m.nslot; ++sl) {
+    if (e < 0 || (e >> 1) >= m.nfi) break;
+    const double* A = ((e & 1) ? im.lower : im.upper) + (size_t)(e >> 1) * kBlk;
+    const double* v = x + 5 * (size_t)nb;
+    if (sl + 1 < m.nslot) {  // the next face's entries while this block is on its way
+      e = im.cfo[(sl + 1) * n + c];
+      nb = e >= 0 ? im.cfon[(sl + 1) * n + c] : 0;
+    }
+    row(A, v, false);
+  }
+  // S A x (the row scale is all ones outside the flexible GMRES)
+  y[5 * (size_t)c + i] = z ? acc : acc * im.rs[i];
+}
+
 // y = S A z with FP32 blocks and FP32 z, FP32 accumulation, FP64 result
 __global__ void __launch_bounds__(128) k_imp_matvec32(DevMesh m, ImpState im, const float* __restrict__ z,
                                                        double* __restrict__ y) {
@@ -704,23 +741,165 @@ __global__ void k_bicg_shift(double* sc) {
   }
 }
 
-// modified Gram-Schmidt pass: w = w - hprev * vprev (when vprev), then partial sums of w . vnext
-__global__ void __launch_bounds__(kRedThreads) k_mgs_pass(const double* __restrict__ vprev,
-                                                           const double* __restrict__ hprev, double* __restrict__ w,
-                                                           const double* __restrict__ vnext, size_t n,
-                                                           double* __restrict__ part) {
-  const double h = vprev ? *hprev : 0.0;
-  double s = 0.0;
-  for (size_t i = blockIdx.x * (size_t)kRedThreads + threadIdx.x; i < n; i += (size_t)gridDim.x * kRedThreads) {
-    double wi = w[i];
-    if (vprev) {
-      wi = wi - h * vprev[i];
-      w[i] = wi;
-    }
-    s += wi * (vnext ? vnext[i] : wi);
+// ---- modified Gram-Schmidt of one Krylov vector in one cooperative launch ----
+// bdlu_gmres.f90:100-118 takes h_i = w . v_i, w -= h_i v_i one vector after the other: jk + 1
+// dependent reductions.  The same h solves (I + L) h = V^T w with L_ij = v_i . v_j (j < i), so the
+// kernel measures V^T w at once, solves the triangle, subtracts V h in the order of i, and
+// measures V^T w and w . w again for the next row of L and h_{jk+1} (the low-synchronisation
+// form of modified Gram-Schmidt of Swirydowicz, Langou, Ananthan, Yang and Thomas, Numer. Linear
+// Algebra Appl. 28, 2021: two reductions a vector, the same loss of orthogonality).
+// The grid is resident and every thread keeps its K entries of w in registers (K = 0: in
+// memory).  No barrier: a block publishes its sums in slots of its own (prefilled with a NaN
+// pattern that no arithmetic produces) and every block reads all slots, waiting (bounded) for
+// those still empty; nothing else travels between blocks.  GB300, 122,825 unknowns, restart 30, us a
+// vector on average: 142 in 2 (jk + 1) launches, 105 with the reductions one after the other in one
+// launch, 35 so (60 with 128 threads a block, 37 with 512).
+constexpr int kMgsThreads = 256;
+constexpr unsigned long long kMgsEmpty = ~0ull;
+constexpr int kMgsSpins = 1 << 22;
+
+template <int K>
+__global__ void __launch_bounds__(kMgsThreads) k_mgs_column(double* w, double* V, size_t n, int jk, double* L,
+                                                            double* slots, double* out, unsigned* err) {
+  constexpr int KR = K > 0 ? K : 1, kWarps = kMgsThreads / 32;
+  extern __shared__ double acc[];  // [jk + 1][kMgsThreads] per-thread sums
+  __shared__ double h[kMaxKrylov + 1];
+  __shared__ int bad;
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5, g = gridDim.x;
+  const size_t first = blockIdx.x * (size_t)kMgsThreads + t, stride = g * (size_t)kMgsThreads;
+  double W[KR];
+  if (t == 0) bad = 0;
+  if constexpr (K > 0) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) W[k] = first + k * stride < n ? w[first + k * stride] : 0.0;
   }
-  s = block_sum(s);
-  if (threadIdx.x == 0) part[blockIdx.x] = s;
+  // this thread's products of w with the vectors 0 .. jk-1 (and with itself) into acc
+  auto products = [&](bool self) {
+    for (int i = 0; i < jk; i += 4) {
+      double s[4] = {0.0, 0.0, 0.0, 0.0};
+      const double* v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[q] = V + (size_t)min(i + q, jk - 1) * n;
+      if constexpr (K > 0) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          if (i + q < jk) {
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+              s[q] = fma(W[k], first + k * stride < n ? v[q][first + k * stride] : 0.0, s[q]);
+          }
+        }
+      } else {
+        for (size_t k = first; k < n; k += stride) {
+          const double wk = w[k];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) s[q] = fma(wk, v[q][k], s[q]);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (i + q < jk) acc[(i + q) * kMgsThreads + t] = s[q];
+    }
+    if (self) {
+      double s = 0.0;
+      if constexpr (K > 0) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) s = fma(W[k], W[k], s);
+      } else {
+        for (size_t k = first; k < n; k += stride) s = fma(w[k], w[k], s);
+      }
+      acc[jk * kMgsThreads + t] = s;
+    }
+    __syncthreads();
+  };
+  // the grid's sums of acc rows 0 .. count-1 into h; every block adds the blocks' sums in block
+  // order.  False after the limit.
+  auto exchange = [&](int count, double* sl) -> bool {
+    for (int i = wid; i < count; i += kWarps) {
+      const double* a = acc + i * kMgsThreads;
+      double s = a[lane];
+#pragma unroll
+      for (int j = 32; j < kMgsThreads; j += 32) s += a[lane + j];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+      if (lane == 0) {
+        unsigned long long b = (unsigned long long)__double_as_longlong(s);
+        if (b == kMgsEmpty) b = 0x7fffffffffffffffull;
+        asm volatile("st.relaxed.gpu.u64 [%0], %1;" ::"l"(sl + (size_t)i * g + blockIdx.x), "l"(b) : "memory");
+      }
+    }
+    for (int i = wid; i < count; i += kWarps) {
+      double s = 0.0;
+      for (int q = lane; q < g; q += 32) {
+        unsigned long long b;
+        int spins = 0;
+        do {
+          asm volatile("ld.relaxed.gpu.u64 %0, [%1];" : "=l"(b) : "l"(sl + (size_t)i * g + q) : "memory");
+        } while (b == kMgsEmpty && ++spins < kMgsSpins);
+        if (b == kMgsEmpty) bad = 1;
+        s += __longlong_as_double((long long)b);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+      if (lane == 0) h[i] = s;
+    }
+    __syncthreads();
+    return bad == 0;  // set at most once: nothing resets it
+  };
+  products(false);
+  if (!exchange(jk, slots)) {
+    if (t == 0) *err = 1u;
+    return;
+  }
+  if (wid == 0) {  // (I + L) h = V^T w, by columns; two entries per lane
+    double d0 = lane < jk ? h[lane] : 0.0, d1 = lane + 32 < jk ? h[lane + 32] : 0.0;
+    for (int i = 0; i < jk; ++i) {
+      const double hi = __shfl_sync(0xffffffffu, i < 32 ? d0 : d1, i & 31);
+      if (lane > i && lane < jk) d0 = fma(-__ldcg(L + lane * kMaxKrylov + i), hi, d0);
+      if (lane + 32 > i && lane + 32 < jk) d1 = fma(-__ldcg(L + (lane + 32) * kMaxKrylov + i), hi, d1);
+    }
+    __syncwarp();
+    if (lane < jk) h[lane] = d0;
+    if (lane + 32 < jk) h[lane + 32] = d1;
+  }
+  __syncthreads();
+  if (blockIdx.x == 0)
+    for (int i = t; i < jk; i += kMgsThreads) out[i] = h[i];
+  if constexpr (K > 0) {
+#pragma unroll 4
+    for (int i = 0; i < jk; ++i) {
+      const double c = -h[i];
+      const double* v = V + (size_t)i * n + first;
+#pragma unroll
+      for (int k = 0; k < K; ++k) W[k] = fma(c, first + k * stride < n ? v[k * stride] : 0.0, W[k]);
+    }
+  } else {
+    for (size_t k = first; k < n; k += stride) {
+      double x = w[k];
+#pragma unroll 4
+      for (int i = 0; i < jk; ++i) x = fma(-h[i], V[(size_t)i * n + k], x);
+      w[k] = x;
+    }
+  }
+  __syncthreads();  // h is read before the second exchange writes it
+  products(true);
+  if (!exchange(jk + 1, slots + (size_t)jk * g)) {
+    if (t == 0) *err = 1u;
+    return;
+  }
+  const double f = 1.0 / sqrt(h[jk]);
+  if (blockIdx.x == 0) {
+    for (int i = t; i < jk; i += kMgsThreads) L[jk * kMaxKrylov + i] = h[i] * f;
+    if (t == 0) out[jk] = h[jk];
+  }
+  double* vn = V + (size_t)jk * n;
+  if constexpr (K > 0) {
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (first + k * stride < n) vn[first + k * stride] = f * W[k];
+  } else {
+    for (size_t k = first; k < n; k += stride) vn[k] = f * w[k];
+  }
 }
 
 // Krylov basis pass of the flexible GMRES (basis vector i at V + i ldv, stored as T):
@@ -981,9 +1160,19 @@ cudaError_t imp_rhs(const DevMesh& m, const DevState& s, const ImpState& im, con
   return cudaGetLastError();
 }
 
+// A row per thread up to 40,000 cells, a cell per thread above, where the row form's narrower
+// loads cost more than its shorter chains gain.  GB300, us per product, cell / row form: 24,565
+// tetrahedra (exact) 24 / 19, 320,000 (fast) 108 / 153.
+constexpr int kRowFormCells = 40000;
+inline void matvec_launch(const DevMesh& m, const ImpState& im, const double* x, const double* z, double* y,
+                          cudaStream_t st) {
+  if (m.nci <= kRowFormCells) k_imp_matvec_row<<<grid_of(m.nci, kRowCells), 5 * kRowCells, 0, st>>>(m, im, x, z, y);
+  else k_imp_matvec<<<grid_of(m.nci, 128), 128, 0, st>>>(m, im, x, z, y);
+}
+
 cudaError_t imp_matvec(const DevMesh& m, const ImpState& im, const double* x, const double* z, double* y,
                        cudaStream_t st, Prof* pr) {
-  pr->launch(K_IMP_MATVEC, st, [&] { k_imp_matvec<<<grid_of(m.nci, 128), 128, 0, st>>>(m, im, x, z, y); });
+  pr->launch(K_IMP_MATVEC, st, [&] { matvec_launch(m, im, x, z, y, st); });
   return cudaGetLastError();
 }
 
@@ -1048,12 +1237,43 @@ cudaError_t imp_asum(const double* a, size_t n, double* part, double* out, cudaS
   return cudaGetLastError();
 }
 
-cudaError_t imp_mgs_pass(const double* vprev, const double* hprev, double* w, const double* vnext, size_t n,
-                         double* part, double* out, cudaStream_t st) {
-  const unsigned g = red_grid(n);
-  k_mgs_pass<<<g, kRedThreads, 0, st>>>(vprev, hprev, w, vnext, n, part);
-  k_red_final<<<1, kRedThreads, 0, st>>>(part, (int)g, kRedBlocks, out);
-  return cudaGetLastError();
+template <int K>
+cudaError_t mgs_launch(double* w, double* V, size_t n, int jk, double* L, double* slots, double* out, unsigned* err,
+                       int sms, cudaStream_t st) {
+  const size_t lists = (size_t)(jk + 1) * kMgsThreads * sizeof(double);
+  cudaError_t e = cudaFuncSetAttribute(k_mgs_column<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lists);
+  if (e != cudaSuccess) return e;
+  int blocks = sms;
+  if (K > 0) {
+    blocks = (int)std::min<size_t>(sms, (n + kMgsThreads * K - 1) / (kMgsThreads * K));
+  } else {  // long vectors in memory: as many blocks as are resident, within the slots
+    int per = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mgs_column<K>, kMgsThreads, lists);
+    if (e != cudaSuccess) return e;
+    blocks = std::min(sms * std::max(per, 1), kRedBlocks / 2);
+  }
+  if ((e = cudaMemsetAsync(slots, 0xff, (size_t)(2 * jk + 1) * blocks * sizeof(double), st)) != cudaSuccess) return e;
+  void* args[] = {&w, &V, &n, &jk, &L, &slots, &out, &err};
+  return cudaLaunchCooperativeKernel((const void*)k_mgs_column<K>, dim3((unsigned)blocks), dim3(kMgsThreads), args, lists,
+                                     st);
+}
+
+// One block per SM with the fewest register entries per thread that cover the vector (152 x 256 x
+// 16 = 622,592 unknowns on GB300); beyond that w stays in memory.
+cudaError_t imp_mgs_column(double* w, double* V, size_t n, int jk, double* L, double* slots, double* out, unsigned* err,
+                           cudaStream_t st) {
+  if (jk < 1 || jk > kMaxKrylov) return cudaErrorInvalidValue;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  sms = std::min(sms, kRedBlocks / 2);
+  const size_t row = (size_t)sms * kMgsThreads;
+  if (n <= row) return mgs_launch<1>(w, V, n, jk, L, slots, out, err, sms, st);
+  if (n <= 2 * row) return mgs_launch<2>(w, V, n, jk, L, slots, out, err, sms, st);
+  if (n <= 4 * row) return mgs_launch<4>(w, V, n, jk, L, slots, out, err, sms, st);
+  if (n <= 8 * row) return mgs_launch<8>(w, V, n, jk, L, slots, out, err, sms, st);
+  if (n <= 16 * row) return mgs_launch<16>(w, V, n, jk, L, slots, out, err, sms, st);
+  return mgs_launch<0>(w, V, n, jk, L, slots, out, err, sms, st);
 }
 
 // blocks of a basis pass: the resident blocks of the whole GPU (at most kRedBlocks), fewer
@@ -1124,11 +1344,11 @@ cudaError_t imp_bicgstab_iter(const DevMesh& m, const ImpState& im, double* x, d
   k_red_part<<<g, kRedThreads, 0, st>>>(r1, r2, n, 0, part);                // rho1 = r1.r2
   k_red_final<<<1, kRedThreads, 0, st>>>(part, (int)g, kRedBlocks, sc + 0);
   k_bicg_p<<<gv, 256, 0, st>>>(r1, v, p, sc, first, n);
-  pr->launch(K_IMP_MATVEC, st, [&] { k_imp_matvec<<<grid_of(m.nci, 128), 128, 0, st>>>(m, im, p, nullptr, v); });
+  pr->launch(K_IMP_MATVEC, st, [&] { matvec_launch(m, im, p, nullptr, v, st); });
   k_red_part<<<g, kRedThreads, 0, st>>>(r2, v, n, 0, part);                 // r2.v
   k_red_final<<<1, kRedThreads, 0, st>>>(part, (int)g, kRedBlocks, sc + 4);
   k_bicg_s<<<gv, 256, 0, st>>>(r1, v, s, sc, n);
-  pr->launch(K_IMP_MATVEC, st, [&] { k_imp_matvec<<<grid_of(m.nci, 128), 128, 0, st>>>(m, im, s, nullptr, t); });
+  pr->launch(K_IMP_MATVEC, st, [&] { matvec_launch(m, im, s, nullptr, t, st); });
   k_bicg_ts<<<g, kRedThreads, 0, st>>>(t, s, n, part);
   k_red_final<<<2, kRedThreads, 0, st>>>(part, (int)g, kRedBlocks, sc + 5);
   k_bicg_update<<<g, kRedThreads, 0, st>>>(x, r1, p, s, t, sc, n, part);

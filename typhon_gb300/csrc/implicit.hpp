@@ -53,8 +53,10 @@ struct ImpState {
   double* Z = nullptr;        // [nk][5 nci] preconditioned basis (flexible GMRES, FP64)
   float* Z32 = nullptr;       // [nk][5 nci] preconditioned basis (mixed precision)
   double* part = nullptr;     // [kMaxKrylov + 1][kRedBlocks] partial sums
+  double* mgs_L = nullptr;    // [kMaxKrylov + 1][kMaxKrylov] products v_i . v_j, j < i (Typhon's GMRES)
   double* scal = nullptr;     // [4 * kMaxKrylov] device scalars (Hessenberg column, step sizes)
-  unsigned* done = nullptr;   // [1] blocks finished in a one-launch reduction (zero between launches)
+  unsigned* done = nullptr;   // [2] blocks finished in a one-launch reduction (zero between launches);
+                              // error word of the Gram-Schmidt kernel's bounded waits
   double* upert = nullptr;    // [5][ldc] perturbed state (Jacobian-free products)
   double* r0 = nullptr;       // [5 nci] residual at the unperturbed state (Jacobian-free)
   double* bs = nullptr;       // [5 nci] right-hand side of the flexible GMRES with its rows scaled
@@ -101,8 +103,8 @@ struct ImpArgs {
                       cudaStream_t st);                                                                 \
   cudaError_t imp_asum(const double* a, size_t n, double* part, double* out, cudaStream_t st);           \
   cudaError_t res_l1(int nci, const double* acc, size_t ld, double* part, double* out, cudaStream_t st);  \
-  cudaError_t imp_mgs_pass(const double* vprev, const double* hprev, double* w, const double* vnext,    \
-                           size_t n, double* part, double* out, cudaStream_t st);                        \
+  cudaError_t imp_mgs_column(double* w, double* V, size_t n, int jk, double* L, double* slots,           \
+                             double* out, unsigned* err, cudaStream_t st);                               \
   cudaError_t imp_basis_pass(double* V, float* V32, size_t ldv, int nv, const double* c,                \
                              const double* src, const double* sp, int extend, size_t n, double* part,   \
                              unsigned* done, double* out, cudaStream_t st, Prof* pr);                   \
