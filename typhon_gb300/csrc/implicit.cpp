@@ -54,6 +54,10 @@ constexpr int kScalY = 2 * kMaxKrylov + 4;    // solution coefficients (kMaxKryl
 constexpr int kScalMisc = 3 * kMaxKrylov + 4; // reductions of the step (16)
 constexpr int kScalCount = 3 * kMaxKrylov + 20;
 
+// leading dimension of the FP64 Krylov basis: whole 16-byte pieces for the sweeps' bulk copies (the
+// vectors they read beside the basis are allocated as long)
+size_t basis_ld(size_t n) { return (n + 1) / 2 * 2; }
+
 template <class T>
 int grow(ty_mesh* h, T*& p, size_t n) {
   if (p) {
@@ -88,8 +92,8 @@ int build_lists(ty_mesh* h) {
   if ((rc = h->alloc(im.cfo, cfo.size())) || (rc = h->alloc(im.cfon, cfon.size())) ||
       (rc = h->alloc(im.dtloc, (size_t)nci)) || (rc = h->alloc(im.jacL, (size_t)m.nf * kBlk)) ||
       (rc = h->alloc(im.jacR, (size_t)m.nf * kBlk)) || (rc = h->alloc(im.b, 5 * (size_t)nci)) ||
-      (rc = h->alloc(im.x, 5 * (size_t)nci)) || (rc = h->alloc(im.r, 5 * (size_t)nci)) ||
-      (rc = h->alloc(im.w, 5 * (size_t)nci)) || (rc = h->alloc(im.part, (size_t)(2 * kMaxKrylov + 1) * kRedBlocks / 2 + kRedBlocks)) ||
+      (rc = h->alloc(im.x, 5 * (size_t)nci)) || (rc = h->alloc(im.r, basis_ld(5 * (size_t)nci))) ||
+      (rc = h->alloc(im.w, basis_ld(5 * (size_t)nci))) || (rc = h->alloc(im.part, (size_t)(2 * kMaxKrylov + 1) * kRedBlocks / 2 + kRedBlocks)) ||
       (rc = h->alloc(im.scal, (size_t)kScalCount)) || (rc = h->alloc(im.done, 2)) ||
       (rc = h->alloc(im.mgs_L, (size_t)(kMaxKrylov + 1) * kMaxKrylov)))
     return rc;
@@ -124,20 +128,20 @@ int ensure_buffers(ty_mesh* h, const ty_imp_params* p) {
       return rc;
     im.fp32_blocks = true;
   }
-  const size_t n = 5 * (size_t)m.nci;
+  const size_t n = 5 * (size_t)m.nci, ldv = basis_ld(n);
   const int nk = p->krylov == TY_KRYLOV_BICGSTAB ? std::max(p->nkrylov, 5) : p->nkrylov;
   const bool gm = p->krylov == TY_KRYLOV_GMRES || p->krylov == TY_KRYLOV_BICGSTAB;  // no preconditioned basis
   // Krylov storage: V (FP64 basis, always), V32 (FP32 basis), Z / Z32 (preconditioned vectors
   // of the flexible GMRES in FP64 / FP32); buffers that exist are regrown with the capacity
   if (im.nk < nk || (need32 && !im.Z32) || (basis32 && !im.V32) || (!need32 && !gm && !im.Z)) {
     const int cap = std::max(nk, im.nk);
-    if ((rc = grow(h, im.V, (size_t)(cap + 1) * n))) return rc;
+    if ((rc = grow(h, im.V, (size_t)(cap + 1) * ldv))) return rc;
     if ((need32 || im.Z32) && (rc = grow(h, im.Z32, (size_t)cap * n))) return rc;
     if ((basis32 || im.V32) && (rc = grow(h, im.V32, (size_t)(cap + 1) * n))) return rc;
     if (((!need32 && !gm) || im.Z) && (rc = grow(h, im.Z, (size_t)cap * n))) return rc;
     im.nk = cap;
   }
-  if ((p->krylov == TY_KRYLOV_FGMRES || p->krylov == TY_KRYLOV_JFNK) && !im.bs && (rc = h->alloc(im.bs, n)))
+  if ((p->krylov == TY_KRYLOV_FGMRES || p->krylov == TY_KRYLOV_JFNK) && !im.bs && (rc = h->alloc(im.bs, ldv)))
     return rc;
   if (p->krylov == TY_KRYLOV_JFNK && !im.jfnk) {
     if ((rc = h->alloc(im.upert, 5 * (size_t)m.ldc)) || (rc = h->alloc(im.r0, n))) return rc;
@@ -166,6 +170,16 @@ int put(ty_mesh* h, int off, const double* v, int k) {
   IMP_CU(cudaMemcpyAsync(h->imp.scal + off, h->imp.pinned + off, k * sizeof(double), cudaMemcpyHostToDevice,
                          h->stream));
   return TY_OK;
+}
+
+// the error word of the kernels' bounded waits (stream idle)
+int check_waits(ty_mesh* h) {
+  unsigned timed_out = 0;
+  IMP_CU(cudaMemcpy(&timed_out, h->imp.done + 1, sizeof(unsigned), cudaMemcpyDeviceToHost));
+  if (!timed_out) return TY_OK;
+  IMP_CU(cudaMemset(h->imp.done + 1, 0, sizeof(unsigned)));
+  tyi::set_error("ty_implicit_step: a wait inside a Krylov kernel timed out");
+  return TY_ERR_CUDA;
 }
 
 // ---- Typhon's bdlu_bicgstab on the device (bdlu_bicgstab.f90:40-80) ----
@@ -280,13 +294,7 @@ int gmres_typhon(ty_mesh* h, const ty_imp_params* p, ty_imp_stats* st) {
     errgmres = ss[nkk + 1] / normp1;
     nit = nit + 1;
   }
-  unsigned timed_out = 0;
-  IMP_CU(cudaMemcpy(&timed_out, im.done + 1, sizeof(unsigned), cudaMemcpyDeviceToHost));
-  if (timed_out) {
-    IMP_CU(cudaMemset(im.done + 1, 0, sizeof(unsigned)));
-    tyi::set_error("ty_implicit_step: the Gram-Schmidt kernel's exchange timed out");
-    return TY_ERR_CUDA;
-  }
+  if (int rc = check_waits(h)) return rc;
   st->restarts = nit;
   st->matvecs = matvecs;
   st->lin_res = errgmres;
@@ -361,7 +369,8 @@ int fgmres(ty_mesh* h, Operator& op, const ty_imp_params* p, ty_imp_stats* st) {
   double* P = im.pinned;
   double* V64 = f32 ? nullptr : im.V;
   float* V32 = f32 ? im.V32 : nullptr;
-  auto Vd = [&](int i) { return V64 ? V64 + (size_t)i * n : nullptr; };
+  const size_t ldv = V64 ? basis_ld(n) : n;
+  auto Vd = [&](int i) { return V64 ? V64 + (size_t)i * ldv : nullptr; };
   auto Vf = [&](int i) { return V32 ? V32 + (size_t)i * n : nullptr; };
   auto Z = [&](int i) { return z32 ? nullptr : im.Z + (size_t)i * n; };
   auto Z32 = [&](int i) { return z32 ? im.Z32 + (size_t)i * n : nullptr; };
@@ -425,11 +434,11 @@ int fgmres(ty_mesh* h, Operator& op, const ty_imp_params* p, ty_imp_stats* st) {
       a[0] = beta;
       int j, nused = 0;
       for (j = 0; j < mk; ++j) {
-        IMP_CU(IMP_CALL(h, imp_basis_pass, V64, V32, n, j, im.scal + kScalCoef, j == 0 ? src : im.w,
+        IMP_CU(IMP_CALL(h, imp_basis_pass, V64, V32, ldv, j, im.scal + kScalCoef, j == 0 ? src : im.w,
                         im.scal + kScalCoef + j, 1, n, im.part, im.done, im.scal + kScalGram, s, &h->prof));
         IMP_CU(IMP_CALL(h, imp_precond, m, im, Vd(j), Vf(j), Z(j), Z32(j), s, &h->prof));
         if (int rc = op.apply(Z(j), Z32(j), im.w, &matvecs)) return rc;
-        IMP_CU(IMP_CALL(h, imp_basis_pass, V64, V32, n, j + 1, nullptr, im.w, nullptr, 0, n, im.part, im.done,
+        IMP_CU(IMP_CALL(h, imp_basis_pass, V64, V32, ldv, j + 1, nullptr, im.w, nullptr, 0, n, im.part, im.done,
                         im.scal + kScalProj, s, &h->prof));
         if (int rc = fetch(h, 0, kScalProj + j + 2)) return rc;
         // column j of the Cholesky factor of G
@@ -486,6 +495,7 @@ int fgmres(ty_mesh* h, Operator& op, const ty_imp_params* p, ty_imp_stats* st) {
       if (std::fabs(a[nused]) <= tol) { ++cycles; break; }
     }
   }
+  if (int rc = check_waits(h)) return rc;
   st->restarts = cycles;
   st->matvecs = matvecs;
   st->lin_res = rel;

@@ -475,49 +475,129 @@ __device__ __forceinline__ void mv5(const double* A, const double* x, double* t)
   }
 }
 
+// ---- 5x5 blocks of 32 cells through shared memory ----
+// A thread that reads its own block, 16 bytes at a time, makes each warp request touch 32 lines
+// (208- or 112-byte strides): the first-level cache, not HBM, then bounds the mat-vec.  Instead
+// the warp copies 32 blocks together (PIECES consecutive lanes one block, asynchronously, one
+// block list ahead of the arithmetic) and every thread reads its block back from shared memory,
+// where both strides are free of bank conflicts.
+template <int PIECES>  // 16-byte pieces of a block: 13 (26 doubles) or 7 (28 floats)
+__device__ __forceinline__ void fetch_blocks(const void* mine, char* stage) {
+  constexpr int PB = 32 / PIECES;  // blocks per request
+  const int lane = threadIdx.x & 31, q = lane / PIECES, piece = lane - q * PIECES;
+#pragma unroll
+  for (int r = 0; r < 32; r += PB) {
+    const int b = r + q;
+    const unsigned long long p = __shfl_sync(0xffffffffu, (unsigned long long)mine, b & 31);
+    if (q < PB && b < 32 && p != 0)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                       (unsigned)__cvta_generic_to_shared(stage + (b * PIECES + piece) * 16)),
+                   "l"((const char*)p + piece * 16)
+                   : "memory");
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
 // y = A x (z == null) or y = z - A x: diagonal block first, then the cell's interior faces in
 // ascending order.  Boundary faces multiply the (zero) ghost unknowns and are skipped.
-__global__ void __launch_bounds__(128) k_imp_matvec(DevMesh m, ImpState im, const double* __restrict__ x,
-                                                     const double* __restrict__ z, double* __restrict__ y) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= m.nci) return;
-  double A[25], xv[5], t[5], yv[5];
+// F32: y = S A x with FP32 blocks and FP32 x, FP32 accumulation, FP64 result.  The FP64 fast mode
+// accumulates every product into the row's sum (25 multiply-adds a block instead of 30 operations).
+// GB300, us per product, own loads -> staged: 250,000 cells FP32 40.5 -> 35.6, 320,000 FP64
+// (fast) 108 -> 90.
+constexpr int kMvThreads = 128;
+template <bool F32>
+__global__ void __launch_bounds__(kMvThreads) k_imp_matvec(DevMesh m, ImpState im, const void* __restrict__ xp,
+                                                            const double* __restrict__ z, double* __restrict__ y) {
+  using T = typename std::conditional<F32, float, double>::type;
+  constexpr int PIECES = F32 ? 7 : 13, kBytes = 32 * PIECES * 16, kStride = F32 ? kBlk32 : kBlk;
+  extern __shared__ __align__(16) char stages[];  // [warps][2][32 blocks]
+  const T* __restrict__ x = (const T*)xp;
+  const T* up = F32 ? (const T*)im.upper32 : (const T*)im.upper;
+  const T* lo = F32 ? (const T*)im.lower32 : (const T*)im.lower;
+  const T* dg = F32 ? (const T*)im.diag32 : (const T*)im.diag;
+  char* mine = stages + (threadIdx.x >> 5) * (2 * kBytes);
+  const int lane = threadIdx.x & 31, c0 = blockIdx.x * kMvThreads + threadIdx.x;
+  const bool on = c0 < m.nci;
+  const int c = on ? c0 : m.nci - 1;
+  const size_t n = m.nci;
+  // entry of a slot: its block and neighbour, null past the cell's interior faces
+  const T* A = nullptr;
+  int nb = c;
+  bool more = on;
+  auto entry = [&](int sl) {
+    const int e = more && sl < m.nslot ? im.cfo[sl * n + c] : -1;
+    more = e >= 0 && (e >> 1) < m.nfi;
+    A = more ? ((e & 1) ? lo : up) + (size_t)(e >> 1) * kStride : nullptr;
+    nb = more ? im.cfon[sl * n + c] : c;
+  };
+  fetch_blocks<PIECES>(on ? dg + (size_t)c * kStride : nullptr, mine);
+  T xv[5], yv[5];
 #pragma unroll
   for (int v = 0; v < 5; ++v) xv[v] = x[5 * (size_t)c + v];
-  load_block(im.diag + (size_t)c * kBlk, A);
-  mv5(A, xv, t);
-  if (z) {
+  bool have = on;
+  for (int s = 0; s <= m.nslot; ++s) {  // block list 0: the diagonal; s: slot s - 1
+    const bool cur = have;
+    T xn[5];
+    entry(s);  // the next list's block and x while this one is on its way
+    have = A != nullptr;
+    const bool any = __any_sync(0xffffffffu, have);
+    if (any) {
+      fetch_blocks<PIECES>(A, mine + ((s + 1) & 1) * kBytes);
 #pragma unroll
-    for (int v = 0; v < 5; ++v) yv[v] = z[5 * (size_t)c + v] - t[v];
-  } else {
-#pragma unroll
-    for (int v = 0; v < 5; ++v) yv[v] = t[v];
-  }
-  for (int sl = 0; sl < m.nslot; ++sl) {
-    const int e = im.cfo[sl * (size_t)m.nci + c];
-    if (e < 0) break;
-    const int f = e >> 1;
-    if (f >= m.nfi) break;
-    const int nb = im.cfon[sl * (size_t)m.nci + c];
-    load_block(((e & 1) ? im.lower : im.upper) + (size_t)f * kBlk, A);
-#pragma unroll
-    for (int v = 0; v < 5; ++v) xv[v] = x[5 * (size_t)nb + v];
-    mv5(A, xv, t);
-    if (z) {
-#pragma unroll
-      for (int v = 0; v < 5; ++v) yv[v] = yv[v] - t[v];
+      for (int v = 0; v < 5; ++v) xn[v] = x[5 * (size_t)nb + v];
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
     } else {
-#pragma unroll
-      for (int v = 0; v < 5; ++v) yv[v] = yv[v] + t[v];
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
-  }
-  if (z) {
+    __syncwarp();
+    if (cur) {
+      const T* B = (const T*)(mine + (s & 1) * kBytes + lane * PIECES * 16);
+      T a[28];
+      if constexpr (F32) {
 #pragma unroll
-    for (int v = 0; v < 5; ++v) y[5 * (size_t)c + v] = yv[v];
-  } else {  // S A x (the row scale is all ones outside the flexible GMRES)
+        for (int k = 0; k < 7; ++k) {
+          const float4 t = reinterpret_cast<const float4*>(B)[k];
+          a[4 * k] = t.x; a[4 * k + 1] = t.y; a[4 * k + 2] = t.z; a[4 * k + 3] = t.w;
+        }
+      } else {
 #pragma unroll
-    for (int v = 0; v < 5; ++v) y[5 * (size_t)c + v] = yv[v] * im.rs[v];
+        for (int k = 0; k < 13; ++k) {
+          const double2 t = reinterpret_cast<const double2*>(B)[k];
+          a[2 * k] = t.x; a[2 * k + 1] = t.y;
+        }
+      }
+      if constexpr (F32 || kFast) {
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+          T q = s == 0 ? T(0) : yv[i];
+          if (!F32 && s == 0 && z) q = (T)z[5 * (size_t)c + i];
+#pragma unroll
+          for (int j = 0; j < 5; ++j) {
+            if constexpr (F32) q = fmaf(a[i * 5 + j], xv[j], q);
+            else q = fma(a[i * 5 + j], z ? -xv[j] : xv[j], q);
+          }
+          yv[i] = q;
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+          T q = T(0);
+#pragma unroll
+          for (int j = 0; j < 5; ++j) q = q + a[i * 5 + j] * xv[j];
+          if (s == 0) yv[i] = z ? z[5 * (size_t)c + i] - q : q;
+          else yv[i] = z ? yv[i] - q : yv[i] + q;
+        }
+      }
+    }
+    if (!any) break;
+    __syncwarp();  // the stage is free for the list after next
+#pragma unroll
+    for (int v = 0; v < 5; ++v) xv[v] = xn[v];
   }
+  if (!on) return;
+  // S A x (the row scale is all ones outside the flexible GMRES)
+#pragma unroll
+  for (int v = 0; v < 5; ++v) y[5 * (size_t)c + v] = !F32 && z ? (double)yv[v] : (double)yv[v] * im.rs[v];
 }
 
 // The same with one thread per row (five consecutive threads a cell, 32 cells a block): chains a
@@ -555,43 +635,6 @@ __global__ void __launch_bounds__(5 * kRowCells) k_imp_matvec_row(DevMesh m, Imp
   }
   // S A x (the row scale is all ones outside the flexible GMRES)
   y[5 * (size_t)c + i] = z ? acc : acc * im.rs[i];
-}
-
-// y = S A z with FP32 blocks and FP32 z, FP32 accumulation, FP64 result
-__global__ void __launch_bounds__(128) k_imp_matvec32(DevMesh m, ImpState im, const float* __restrict__ z,
-                                                       double* __restrict__ y) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= m.nci) return;
-  float A[28], xv[5], yv[5];
-#pragma unroll
-  for (int v = 0; v < 5; ++v) xv[v] = z[5 * (size_t)c + v];
-  load_block32(im.diag32 + (size_t)c * kBlk32, A);
-#pragma unroll
-  for (int i = 0; i < 5; ++i) {
-    float s = 0.f;
-#pragma unroll
-    for (int j = 0; j < 5; ++j) s = fmaf(A[i * 5 + j], xv[j], s);
-    yv[i] = s;
-  }
-  for (int sl = 0; sl < m.nslot; ++sl) {
-    const int e = im.cfo[sl * (size_t)m.nci + c];
-    if (e < 0) break;
-    const int f = e >> 1;
-    if (f >= m.nfi) break;
-    const int nb = im.cfon[sl * (size_t)m.nci + c];
-    load_block32(((e & 1) ? im.lower32 : im.upper32) + (size_t)f * kBlk32, A);
-#pragma unroll
-    for (int v = 0; v < 5; ++v) xv[v] = z[5 * (size_t)nb + v];
-#pragma unroll
-    for (int i = 0; i < 5; ++i) {
-      float s = yv[i];
-#pragma unroll
-      for (int j = 0; j < 5; ++j) s = fmaf(A[i * 5 + j], xv[j], s);
-      yv[i] = s;
-    }
-  }
-#pragma unroll
-  for (int v = 0; v < 5; ++v) y[5 * (size_t)c + v] = (double)yv[v] * im.rs[v];
 }
 
 // z = D^-1 S^-1 v, the block-Jacobi preconditioner of the flexible GMRES on its row-scaled
@@ -902,89 +945,188 @@ __global__ void __launch_bounds__(kMgsThreads) k_mgs_column(double* w, double* V
   }
 }
 
-// Krylov basis pass of the flexible GMRES (basis vector i at V + i ldv, stored as T):
-//   extend 0: out_i = V_i . src (i < nv), out_nv = src . src
-//   extend 1: v = (src - sum_{i<nv} c_i V_i) s is stored as V_nv (rounded to T), then
-//             out_i = V_i . v (i < nv), out_nv = v . v, of the stored values
-// An FP64 basis is swept in FP64; an FP32 basis (mixed-precision solve) in FP32 arithmetic
-// with FP64 block sums.  The first form projects A z_j on the basis; the second forms the next
-// basis vector and the new column of the basis' Gram matrix in the same sweep, so one iteration reads the basis
-// twice and synchronises with the host once.  One row per thread per trip: the row's basis
-// entries are loaded together and kept in registers; the per-thread sums live in shared
-// memory.  Each block reduces its sums once, writes one partial per output, and the last block
-// to finish adds the partials in block order: one launch, the same result for the same grid.
-template <int J, class T>
-__global__ void __launch_bounds__(kCgsThreads) k_basis_pass(T* V, size_t ldv, int nv, const double* __restrict__ c,
+// Krylov basis pass of the flexible GMRES (basis vector i at V + i ldv):
+//   project: out_i = V_i . src (i < nv), out_nv = src . src
+//   extend:  v = (src - sum_{i<nv} c_i V_i) s is stored as V_nv (rounded to the basis' type), then
+//            out_i = V_i . v (i < nv), out_nv = v . v, of the stored values
+// An FP64 basis is swept in FP64; an FP32 basis (mixed-precision solve) in FP32 arithmetic with
+// FP64 block sums.  The first form projects A z_j on the basis; the second forms the next basis
+// vector and the new column of the basis' Gram matrix in the same sweep, so one iteration reads
+// the basis twice and synchronises with the host once.  Each block reduces its sums once, writes
+// one partial per output, and the last block to finish adds the partials in block order: one
+// launch, the same result for the same grid.
+
+// The end of a sweep: acc [nout][T] per-thread sums -> one partial per output and block -> out.
+template <int T>
+__device__ __forceinline__ void finish_sums(const double* acc, int nout, double* __restrict__ part,
+                                            unsigned* __restrict__ done, double* __restrict__ out) {
+  __shared__ bool last;
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  for (int i = wid; wid < T / 32 && i < nout; i += T / 32) {
+    double x = 0.0;
+#pragma unroll
+    for (int q = 0; q < T / 32; ++q) x += acc[(size_t)i * T + q * 32 + lane];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    if (lane == 0) part[(size_t)i * kRedBlocks + blockIdx.x] = x;
+  }
+  __threadfence();
+  __syncthreads();
+  if (t == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int i = wid; wid < T / 32 && i < nout; i += T / 32) {
+    const double* p = part + (size_t)i * kRedBlocks;
+    double x = 0.0;
+    for (unsigned b = lane; b < gridDim.x; b += 32) x += __ldcg(p + b);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    if (lane == 0) out[i] = x;
+  }
+  if (t == 0) *done = 0u;  // ready for the next launch on the stream
+}
+
+// ---- bulk copies into shared memory (TMA) with their completion barrier ----
+__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(unsigned long long* b, unsigned count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(b)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(unsigned long long* b) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(b)) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(unsigned long long* b, unsigned bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(b)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned bytes, unsigned long long* b) {
+  asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_addr(dst)),
+               "l"(src), "r"(bytes), "r"(smem_addr(b))
+               : "memory");
+}
+// waits (bounded) for the phase of the given parity; false after the limit
+__device__ __forceinline__ bool mbar_wait(unsigned long long* b, unsigned parity) {
+  unsigned ok = 0;
+  for (int i = 0; i < (1 << 20) && !ok; ++i)
+    asm volatile("{.reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p;}"
+                 : "=r"(ok)
+                 : "r"(smem_addr(b)), "r"(parity)
+                 : "memory");
+  return ok != 0;
+}
+
+// The FP64 sweep.  Bound by the FP64 pipe (nv + 1 multiply-adds a row, 2 nv + 2 when it extends):
+// compiled per form and per even J >= nv (predicated-off slots occupy the pipe), one block of
+// two warps per SM quarter, its tiles of 256 rows of the nv + 1 vectors brought to shared memory
+// by a ninth warp's bulk copies several tiles ahead, so that neither registers nor occupancy
+// limit the loads in flight.  One block per SM also because a block's reduction costs (nv + 1) (T/32 + 5) additions
+// and the last block adds a partial per block: 15 us of a 66 us sweep when eight blocks per SM did.
+// The vectors are padded to 16 bytes (ldv a multiple of 2, src at least ldv long).  GB300, project /
+// extend: 1,250,000 rows, J = 14, 53 / 77 us with loads to registers, 46 / 81 us so; 1,600,000
+// rows, 24 vectors, 427 / 159 (the compiler spread the loads out) -> 88 / 169.
+constexpr int kSweepThreads = 256;
+template <int J>
+constexpr int kSweepStages = J <= 8 ? 8 : (J <= 16 ? 4 : 3);
+
+template <int J, bool EXTEND>
+__global__ void __launch_bounds__(kSweepThreads + 32) k_basis_pass(double* V, size_t ldv, int nv,
+                                                               const double* __restrict__ c,
+                                                               const double* __restrict__ src,
+                                                               const double* __restrict__ sp, size_t n,
+                                                               double* __restrict__ part, unsigned* __restrict__ done,
+                                                               double* __restrict__ out) {
+  constexpr int T = kSweepThreads, S = kSweepStages<J>;
+  extern __shared__ __align__(16) double buf[];  // [S][J + 1][T]: the vectors 0 .. nv-1, then src
+  __shared__ __align__(8) unsigned long long full[S], empty[S];
+  __shared__ double cl[J];
+  const int t = threadIdx.x;
+  if (EXTEND && t < J) cl[t] = t < nv ? -c[t] : 0.0;
+  const double sc = EXTEND ? *sp : 1.0;
+  const int tiles = (int)((n + T - 1) / T), mine = (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+  auto load = [&](int i) {  // this block's tile i into its stage (one thread)
+    const size_t k0 = (size_t)(blockIdx.x + i * gridDim.x) * T;
+    const unsigned bytes = (unsigned)(min((size_t)T, ldv - k0) * sizeof(double));
+    double* d = buf + (size_t)(i % S) * (J + 1) * T;
+    unsigned long long* b = &full[i % S];
+    mbar_expect(b, bytes * (nv + 1));
+    for (int v = 0; v < nv; ++v) bulk_load(d + v * T, V + v * ldv + k0, bytes, b);
+    bulk_load(d + J * T, src + k0, bytes, b);
+  };
+  if (t == 0) {
+    for (int i = 0; i < S; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], T / 32);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (nv < J && t < T) {  // the padding slot of an odd nv
+    for (int i = 0; i < S; ++i) buf[(size_t)i * (J + 1) * T + nv * T + t] = 0.0;
+    if (nv + 1 < J)
+      for (int i = 0; i < S; ++i) buf[(size_t)i * (J + 1) * T + (nv + 1) * T + t] = 0.0;
+  }
+  __syncthreads();
+  bool ok = true;
+  if (t == T)  // the producer: one thread of the ninth warp
+    for (int i = 0; i < mine; ++i) {
+      if (i >= S) ok = mbar_wait(&empty[i % S], (i / S - 1) & 1) && ok;
+      load(i);
+    }
+  double* vout = V + (size_t)nv * ldv;
+  double ad[J], cr[EXTEND && J <= 20 ? J : 1], xx = 0.0;
+#pragma unroll
+  for (int i = 0; i < J; ++i) {
+    ad[i] = 0.0;
+    if (EXTEND && J <= 20) cr[i] = cl[i];
+  }
+  for (int i = 0; i < (t < T ? mine : 0); ++i) {
+    const int st = i % S;
+    ok = mbar_wait(&full[st], (i / S) & 1) && ok;
+    const double* d = buf + (size_t)st * (J + 1) * T + t;
+    const size_t k = (size_t)(blockIdx.x + i * gridDim.x) * T + t;
+    if (k < n) {
+      double x = d[J * T], b[J];
+#pragma unroll
+      for (int v = 0; v < J; ++v) b[v] = d[v * T];
+      if constexpr (EXTEND) {
+#pragma unroll
+        for (int v = 0; v < J; ++v) x = fma(J <= 20 ? cr[v] : cl[v], b[v], x);
+        x = x * sc;
+        vout[k] = x;
+      }
+#pragma unroll
+      for (int v = 0; v < J; ++v) ad[v] = fma(b[v], x, ad[v]);
+      xx = fma(x, x, xx);
+    }
+    __syncwarp();
+    if ((t & 31) == 0) mbar_arrive(&empty[st]);
+  }
+  if (!ok) done[1] = 1u;
+  __syncthreads();  // every copy has been waited for: the stages become the per-thread sums
+  if (t < T) {
+#pragma unroll
+    for (int i = 0; i < J; ++i) buf[i * T + t] = ad[i];
+    buf[nv * T + t] = xx;
+  }
+  __syncthreads();
+  finish_sums<T>(buf, nv + 1, part, done, out);
+}
+
+template <int J>
+__global__ void __launch_bounds__(kCgsThreads) k_basis_pass32(float* V, size_t ldv, int nv, const double* __restrict__ c,
                                                              const double* __restrict__ src,
                                                              const double* __restrict__ sp, int extend, size_t n,
                                                              double* __restrict__ part, unsigned* __restrict__ done,
                                                              double* __restrict__ out) {
   __shared__ double cl[J];
   __shared__ double acc[J + 1][kCgsThreads];
-  __shared__ bool last;
   const int t = threadIdx.x;
   if (t < J) cl[t] = (extend && t < nv) ? c[t] : 0.0;
 #pragma unroll
   for (int i = 0; i <= J; ++i) acc[i][t] = 0.0;
   const double sc = extend ? *sp : 1.0;
   __syncthreads();
-  T* vout = V + (size_t)nv * ldv;
-  if constexpr (std::is_same<T, double>::value && J <= 16) {
-    // short bases: per-thread sums in registers, written to shared memory once
-    double ad[J];
-#pragma unroll
-    for (int i = 0; i < J; ++i) ad[i] = 0.0;
-    double xx = 0.0;
-    for (size_t k = blockIdx.x * (size_t)kCgsThreads + t; k < n; k += (size_t)gridDim.x * kCgsThreads) {
-      double v[J];
-      const double* pv = V + k;
-#pragma unroll
-      for (int i = 0; i < J; ++i) {
-        v[i] = i < nv ? *pv : 0.0;
-        pv += ldv;
-      }
-      double x = src[k];
-      if (extend) {
-#pragma unroll
-        for (int i = 0; i < J; ++i)
-          if (i < nv) x = x - cl[i] * v[i];
-        x = x * sc;
-        vout[k] = x;
-      }
-#pragma unroll
-      for (int i = 0; i < J; ++i)
-        if (i < nv) ad[i] += v[i] * x;
-      xx += x * x;
-    }
-#pragma unroll
-    for (int i = 0; i < J; ++i)
-      if (i < nv) acc[i][t] = ad[i];
-    acc[nv][t] = xx;
-  } else if constexpr (std::is_same<T, double>::value) {
-    double xx = 0.0;
-    for (size_t k = blockIdx.x * (size_t)kCgsThreads + t; k < n; k += (size_t)gridDim.x * kCgsThreads) {
-      double v[J];
-      const double* pv = V + k;
-#pragma unroll
-      for (int i = 0; i < J; ++i) {
-        v[i] = i < nv ? *pv : 0.0;
-        pv += ldv;
-      }
-      double x = src[k];
-      if (extend) {
-#pragma unroll
-        for (int i = 0; i < J; ++i)
-          if (i < nv) x = x - cl[i] * v[i];
-        x = x * sc;
-        vout[k] = x;
-      }
-#pragma unroll
-      for (int i = 0; i < J; ++i)
-        if (i < nv) acc[i][t] += v[i] * x;
-      xx += x * x;
-    }
-    acc[nv][t] = xx;
-  } else {
+  float* vout = V + (size_t)nv * ldv;
+  {
     // FP32 basis: FP32 arithmetic per row (GB300 issues FP32 at about 60x its FP64 rate),
     // per-thread sums in FP32 registers over the thread's rows, FP64 from the block sums on
     float cf[J], af[J];
@@ -1033,31 +1175,7 @@ __global__ void __launch_bounds__(kCgsThreads) k_basis_pass(T* V, size_t ldv, in
     acc[nv][t] = (double)xx;
   }
   __syncthreads();
-  const int nout = nv + 1;
-  const int lane = t & 31, wid = t >> 5;
-  for (int i = wid; i < nout; i += kCgsThreads / 32) {
-    double x = 0.0;
-#pragma unroll
-    for (int q = 0; q < kCgsThreads / 32; ++q) x += acc[i][q * 32 + lane];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) part[(size_t)i * kRedBlocks + blockIdx.x] = x;
-  }
-  __threadfence();
-  __syncthreads();
-  if (t == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  for (int i = wid; i < nout; i += kCgsThreads / 32) {
-    const double* p = part + (size_t)i * kRedBlocks;
-    double x = 0.0;
-    for (unsigned b = lane; b < gridDim.x; b += 32) x += __ldcg(p + b);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) out[i] = x;
-  }
-  if (t == 0) *done = 0u;  // ready for the next launch on the stream
+  finish_sums<kCgsThreads>(&acc[0][0], nv + 1, part, done, out);
 }
 
 __global__ void k_scale(const double* __restrict__ w, double s, double* __restrict__ v, size_t n) {
@@ -1160,14 +1278,21 @@ cudaError_t imp_rhs(const DevMesh& m, const DevState& s, const ImpState& im, con
   return cudaGetLastError();
 }
 
+template <bool F32>
+void mv_staged(const DevMesh& m, const ImpState& im, const void* x, const double* z, double* y, cudaStream_t st) {
+  constexpr int bytes = kMvThreads / 32 * 2 * 32 * (F32 ? 7 : 13) * 16;
+  cudaFuncSetAttribute(k_imp_matvec<F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  k_imp_matvec<F32><<<grid_of(m.nci, kMvThreads), kMvThreads, bytes, st>>>(m, im, x, z, y);
+}
+
 // A row per thread up to 40,000 cells, a cell per thread above, where the row form's narrower
 // loads cost more than its shorter chains gain.  GB300, us per product, cell / row form: 24,565
-// tetrahedra (exact) 24 / 19, 320,000 (fast) 108 / 153.
+// tetrahedra (exact) 24 / 19, 320,000 (fast) 90 (108 before its blocks were staged) / 153.
 constexpr int kRowFormCells = 40000;
 inline void matvec_launch(const DevMesh& m, const ImpState& im, const double* x, const double* z, double* y,
                           cudaStream_t st) {
   if (m.nci <= kRowFormCells) k_imp_matvec_row<<<grid_of(m.nci, kRowCells), 5 * kRowCells, 0, st>>>(m, im, x, z, y);
-  else k_imp_matvec<<<grid_of(m.nci, 128), 128, 0, st>>>(m, im, x, z, y);
+  else mv_staged<false>(m, im, x, z, y, st);
 }
 
 cudaError_t imp_matvec(const DevMesh& m, const ImpState& im, const double* x, const double* z, double* y,
@@ -1178,7 +1303,7 @@ cudaError_t imp_matvec(const DevMesh& m, const ImpState& im, const double* x, co
 
 cudaError_t imp_matvec32(const DevMesh& m, const ImpState& im, const float* z, double* y, cudaStream_t st,
                          Prof* pr) {
-  pr->launch(K_IMP_MATVEC, st, [&] { k_imp_matvec32<<<grid_of(m.nci, 128), 128, 0, st>>>(m, im, z, y); });
+  pr->launch(K_IMP_MATVEC, st, [&] { mv_staged<true>(m, im, z, nullptr, y, st); });
   return cudaGetLastError();
 }
 
@@ -1276,63 +1401,66 @@ cudaError_t imp_mgs_column(double* w, double* V, size_t n, int jk, double* L, do
   return mgs_launch<0>(w, V, n, jk, L, slots, out, err, sms, st);
 }
 
-// blocks of a basis pass: the resident blocks of the whole GPU (at most kRedBlocks), fewer
-// for short vectors; a fixed function of n and the device, so sums repeat from run to run
-template <int J, class T>
-unsigned basis_grid(size_t n) {
-  static const unsigned cap = [] {
-    int dev = 0, sms = 0, per = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_basis_pass<J, T>, kCgsThreads, 0);
-    const long c = (long)std::max(sms, 1) * std::max(per, 1);
-    return (unsigned)std::min<long>(c, kRedBlocks);
-  }();
-  const size_t g = (n + kCgsThreads - 1) / kCgsThreads;
-  return (unsigned)std::max<size_t>(1, std::min<size_t>(g, cap));
+// Blocks of a sweep: a fixed function of n and the device, so that sums repeat from run to run.
+inline unsigned sm_count() {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return (unsigned)std::max(1, std::min(sms, kRedBlocks));
 }
 
-template <int J, class T>
-void basis_launch_j(T* V, size_t ldv, int nv, const double* c, const double* src, const double* sp, int extend,
-                    size_t n, double* part, unsigned* done, double* out, cudaStream_t st) {
-  k_basis_pass<J, T><<<basis_grid<J, T>(n), kCgsThreads, 0, st>>>(V, ldv, nv, c, src, sp, extend, n, part, done, out);
+template <int J>
+cudaError_t basis_launch_j(double* V, size_t ldv, int nv, const double* c, const double* src, const double* sp,
+                           int extend, size_t n, double* part, unsigned* done, double* out, cudaStream_t st) {
+  const unsigned g = (unsigned)std::max<size_t>(1, std::min<size_t>((n + kSweepThreads - 1) / kSweepThreads, sm_count()));
+  const size_t sums = (size_t)kSweepStages<J> * (J + 1) * kSweepThreads * sizeof(double);
+  auto* k = extend ? k_basis_pass<J, true> : k_basis_pass<J, false>;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sums);
+  if (e != cudaSuccess) return e;
+  k<<<g, kSweepThreads + 32, sums, st>>>(V, ldv, nv, c, src, sp, n, part, done, out);
+  return cudaGetLastError();
 }
 
-// The unrolled loops of a sweep run J slots per entry whatever nv is, so an FP64 sweep (bound
-// by the FP64 pipe) takes the smallest even J >= nv; an FP32 sweep (bound by HBM) takes 8, 16
-// or 32.
-template <class T>
-void basis_launch(T* V, size_t ldv, int nv, const double* c, const double* src, const double* sp, int extend,
-                  size_t n, double* part, unsigned* done, double* out, cudaStream_t st) {
-  if constexpr (std::is_same<T, double>::value) {
-    switch ((nv + 1) / 2) {
-      case 0:
-      case 1: basis_launch_j<2>(V, ldv, nv, c, src, sp, extend, n, part, done, out, st); return;
-      case 2: basis_launch_j<4>(V, ldv, nv, c, src, sp, extend, n, part, done, out, st); return;
-      case 3: basis_launch_j<6>(V, ldv, nv, c, src, sp, extend, n, part, done, out, st); return;
-      case 4: basis_launch_j<8>(V, ldv, nv, c, src, sp, extend, n, part, done, out, st); return;
-      case 5: basis_launch_j<10>(V, ldv, nv, c, src, sp, extend, n, part, done, out, st); return;
-      case 6: basis_launch_j<12>(V, ldv, nv, c, src, sp, extend, n, part, done, out, st); return;
-      case 7: basis_launch_j<14>(V, ldv, nv, c, src, sp, extend, n, part, done, out, st); return;
-      case 8: basis_launch_j<16>(V, ldv, nv, c, src, sp, extend, n, part, done, out, st); return;
-      default: basis_launch_j<kMaxCgs>(V, ldv, nv, c, src, sp, extend, n, part, done, out, st); return;
-    }
-  } else {
-    if (nv <= 8) basis_launch_j<8>(V, ldv, nv, c, src, sp, extend, n, part, done, out, st);
-    else if (nv <= 16) basis_launch_j<16>(V, ldv, nv, c, src, sp, extend, n, part, done, out, st);
-    else basis_launch_j<kMaxCgs>(V, ldv, nv, c, src, sp, extend, n, part, done, out, st);
+// the smallest even J >= nv
+template <int J = 2>
+cudaError_t basis_launch(double* V, size_t ldv, int nv, const double* c, const double* src, const double* sp, int extend,
+                         size_t n, double* part, unsigned* done, double* out, cudaStream_t st) {
+  if constexpr (J < kMaxCgs) {
+    if (nv > J) return basis_launch<J + 2>(V, ldv, nv, c, src, sp, extend, n, part, done, out, st);
   }
+  return basis_launch_j<J>(V, ldv, nv, c, src, sp, extend, n, part, done, out, st);
+}
+
+// an FP32 sweep, bound by HBM, takes 8, 16 or 32 slots and every resident block
+template <int J>
+cudaError_t basis_launch32_j(float* V, size_t ldv, int nv, const double* c, const double* src, const double* sp,
+                             int extend, size_t n, double* part, unsigned* done, double* out, cudaStream_t st) {
+  static const unsigned cap = [] {
+    int per = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_basis_pass32<J>, kCgsThreads, 0);
+    return (unsigned)std::min<long>((long)sm_count() * std::max(per, 1), kRedBlocks);
+  }();
+  const size_t g = std::max<size_t>(1, std::min<size_t>((n + kCgsThreads - 1) / kCgsThreads, cap));
+  k_basis_pass32<J><<<(unsigned)g, kCgsThreads, 0, st>>>(V, ldv, nv, c, src, sp, extend, n, part, done, out);
+  return cudaGetLastError();
+}
+inline cudaError_t basis_launch32(float* V, size_t ldv, int nv, const double* c, const double* src, const double* sp,
+                                  int extend, size_t n, double* part, unsigned* done, double* out, cudaStream_t st) {
+  if (nv <= 8) return basis_launch32_j<8>(V, ldv, nv, c, src, sp, extend, n, part, done, out, st);
+  if (nv <= 16) return basis_launch32_j<16>(V, ldv, nv, c, src, sp, extend, n, part, done, out, st);
+  return basis_launch32_j<kMaxCgs>(V, ldv, nv, c, src, sp, extend, n, part, done, out, st);
 }
 
 cudaError_t imp_basis_pass(double* V, float* V32, size_t ldv, int nv, const double* c, const double* src,
                            const double* sp, int extend, size_t n, double* part, unsigned* done, double* out,
                            cudaStream_t st, Prof* pr) {
   if (nv < 0 || nv > kMaxCgs) return cudaErrorInvalidValue;
+  cudaError_t e = cudaSuccess;
   pr->launch(K_IMP_ORTHO, st, [&] {
-    if (V32) basis_launch(V32, ldv, nv, c, src, sp, extend, n, part, done, out, st);
-    else basis_launch(V, ldv, nv, c, src, sp, extend, n, part, done, out, st);
+    e = V32 ? basis_launch32(V32, ldv, nv, c, src, sp, extend, n, part, done, out, st)
+            : basis_launch(V, ldv, nv, c, src, sp, extend, n, part, done, out, st);
   });
-  return cudaGetLastError();
+  return e;
 }
 
 cudaError_t imp_bicgstab_iter(const DevMesh& m, const ImpState& im, double* x, double* r1, const double* r2,

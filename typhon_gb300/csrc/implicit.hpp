@@ -48,7 +48,7 @@ struct ImpState {
   double* x = nullptr;        // [5 nci] solution (the update)
   double* r = nullptr;        // [5 nci]
   double* w = nullptr;        // [5 nci]
-  double* V = nullptr;        // [nk + 1][5 nci] Krylov basis
+  double* V = nullptr;        // [nk + 1][5 nci, padded to even for the flexible GMRES] Krylov basis
   float* V32 = nullptr;       // [nk + 1][5 nci] Krylov basis of the mixed-precision flexible GMRES
   double* Z = nullptr;        // [nk][5 nci] preconditioned basis (flexible GMRES, FP64)
   float* Z32 = nullptr;       // [nk][5 nci] preconditioned basis (mixed precision)
@@ -56,7 +56,7 @@ struct ImpState {
   double* mgs_L = nullptr;    // [kMaxKrylov + 1][kMaxKrylov] products v_i . v_j, j < i (Typhon's GMRES)
   double* scal = nullptr;     // [4 * kMaxKrylov] device scalars (Hessenberg column, step sizes)
   unsigned* done = nullptr;   // [2] blocks finished in a one-launch reduction (zero between launches);
-                              // error word of the Gram-Schmidt kernel's bounded waits
+                              // error word of the bounded waits inside the Krylov kernels
   double* upert = nullptr;    // [5][ldc] perturbed state (Jacobian-free products)
   double* r0 = nullptr;       // [5 nci] residual at the unperturbed state (Jacobian-free)
   double* bs = nullptr;       // [5 nci] right-hand side of the flexible GMRES with its rows scaled
