@@ -25,11 +25,8 @@ int ty_residual_device(ty_mesh* h, double dt, double* R) {
   if (!R) return TY_ERR_ARG;
   if ((rc = ensure_prim(h))) return rc;
   if ((rc = stage_faces(h))) return rc;
-  cudaError_t e = ADJ_CALL(h, residual_gather, h->m, h->s, dt, nullptr, h->stream, &h->prof);
+  cudaError_t e = ADJ_CALL(h, residual_gather, h->m, h->s, dt, nullptr, R, h->m.nci, h->stream, &h->prof);
   if (e != cudaSuccess) return cuda_fail(e, "residual gather");
-  const size_t n = h->m.nci;
-  TY_CU(cudaMemcpy2DAsync(R, n * sizeof(double), h->s.res, h->m.ldc * sizeof(double), n * sizeof(double), 5,
-                          cudaMemcpyDeviceToDevice, h->stream));
   return TY_OK;
 }
 

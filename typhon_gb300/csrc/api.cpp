@@ -258,9 +258,12 @@ int build_viscous_geometry(ty_mesh* h) {
 namespace tyi {
 
 int check_err(ty_mesh* h) {
-  int e[2] = {0, 0};
-  TY_CU(cudaMemcpyAsync(e, h->s.err, 2 * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  // time-step slots and error word lie together: one copy to pinned memory, one wait
+  unsigned long long* host = h->ctl_host + 4;
+  TY_CU(cudaMemcpyAsync(host, h->s.dtbits, 6 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, h->stream));
   TY_CU(cudaStreamSynchronize(h->stream));
+  int e[2];
+  std::memcpy(e, host + 4, sizeof(e));
   if (e[0] != 0) {
     TY_CU(cudaMemsetAsync(h->s.err, 0, 4 * sizeof(int), h->stream));
     tyi::set_error(std::string(ty_error_string(e[0])) + " at cell " + std::to_string(e[1]));
@@ -269,13 +272,16 @@ int check_err(ty_mesh* h) {
   return TY_OK;
 }
 
-int set_dt_slot(ty_mesh* h, int slot, double v) {
-  unsigned long long b;
-  std::memcpy(&b, &v, 8);
-  // pinned staging word per slot keeps the copy asynchronous and ordered on the stream
-  unsigned long long* host = reinterpret_cast<unsigned long long*>(h->dtbits_host) + slot;
-  *host = b;
-  TY_CU(cudaMemcpyAsync(h->s.dtbits + slot, host, 8, cudaMemcpyHostToDevice, h->stream));
+double fetched_dt(const ty_mesh* h, int slot) {
+  double v;
+  std::memcpy(&v, h->ctl_host + 4 + slot, 8);
+  return v;
+}
+
+int reset_dt_slots(ty_mesh* h, int slot, int count) {
+  // pinned staging words that always hold the largest finite double: asynchronous and ordered
+  TY_CU(cudaMemcpyAsync(h->s.dtbits + slot, h->ctl_host, count * sizeof(unsigned long long), cudaMemcpyHostToDevice,
+                        h->stream));
   return TY_OK;
 }
 
@@ -357,9 +363,10 @@ int ensure_pk(ty_mesh* h, const RkStagePlan* plans, int n) {
 }
 
 // one RK step; dt either host value or device slot dtbits_cur.  dtbits_next: where the
-// final stage writes the next step's stability time step (or null).
+// final stage writes the next step's stability time step (or null); dtbits_reset: a slot that it
+// sets back to the largest finite double, the target of the step after.
 int run_step(ty_mesh* h, const RkTab& t, double dt, const unsigned long long* dtbits_cur,
-             unsigned long long* dtbits_next, double cfl, bool store_acc = false,
+             unsigned long long* dtbits_next, unsigned long long* dtbits_reset, double cfl, bool store_acc = false,
              const double* dtloc = nullptr) {
   RkStagePlan plans[kMaxStage];
   make_plans(t, plans);
@@ -389,7 +396,7 @@ int run_step(ty_mesh* h, const RkTab& t, double dt, const unsigned long long* dt
       if (e != cudaSuccess) return cuda_fail(e, "ghost rows");
     }
     cudaError_t e = MODE_CALL(h, rk_update, h->m, h->s, h->o, plans[i], dt, dtbits_cur,
-                              i == t.n - 1 ? dtbits_next : nullptr, cfl, h->stream, &h->prof);
+                              i == t.n - 1 ? dtbits_next : nullptr, dtbits_reset, cfl, h->stream, &h->prof);
     if (e != cudaSuccess) return cuda_fail(e, "rk update");
   }
   h->prim_valid = true;  // the final update wrote the primitive variables of u0
@@ -549,16 +556,18 @@ int ty_mesh_create(const ty_mesh_desc* d, int device, ty_mesh** out) {
   DevState& s = h->s;
   if ((rc = h->alloc(s.u0, 5 * lc)) || (rc = h->alloc(s.acc, 5 * lc)) ||
       (rc = h->alloc(s.prim, 5 * lc)) || (rc = h->alloc(s.grad, 15 * lc)) || (rc = h->alloc(s.ratio, 3 * lc)) ||
-      (rc = h->alloc(s.flux, 5 * lf)) || (rc = h->alloc(s.res, 5 * lc)) || (rc = h->alloc(s.dtbits, 4)) ||
-      (rc = h->alloc(s.stage, 5 * (size_t)nci)) ||
-      (rc = h->alloc(s.err, 4)))
+      (rc = h->alloc(s.flux, 5 * lf)) || (rc = h->alloc(s.res, 5 * lc)) || (rc = h->alloc(s.dtbits, 6)) ||
+      (rc = h->alloc(s.stage, 5 * (size_t)nci)))
     return bail(rc);
+  s.err = reinterpret_cast<int*>(s.dtbits + 4);  // behind the time-step slots: read with them
   TY_CU(cudaMemset(s.u0, 0, 5 * lc * sizeof(double)));
   TY_CU(cudaMemset(s.grad, 0, 15 * lc * sizeof(double)));
   TY_CU(cudaMemset(s.prim, 0, 5 * lc * sizeof(double)));
   TY_CU(cudaMemset(s.err, 0, 4 * sizeof(int)));
   TY_CU(cudaMemset(s.ratio, 0, 3 * lc * sizeof(double)));
-  if (cudaMallocHost((void**)&h->dtbits_host, 4 * sizeof(double)) != cudaSuccess) return bail(TY_ERR_NOMEM);
+  // [0..3] the largest finite double (reset values), [4..9] slots and error word read back
+  if (cudaMallocHost((void**)&h->ctl_host, 10 * sizeof(unsigned long long)) != cudaSuccess) return bail(TY_ERR_NOMEM);
+  for (int i = 0; i < 4; ++i) h->ctl_host[i] = 0x7fefffffffffffffull;
   h->nslot = nslot;
   m.ghost_copy = ng > 0 && !h->nonperiodic_bc;
   *out = h;
@@ -570,7 +579,8 @@ int ty_mesh_destroy(ty_mesh* h) {
   cudaSetDevice(h->device);
   if (h->stream) cudaStreamSynchronize(h->stream);
   for (void* p : h->allocs) cudaFree(p);
-  if (h->dtbits_host) cudaFreeHost(h->dtbits_host);
+  if (h->ctl_host) cudaFreeHost(h->ctl_host);
+  if (h->steady_host) cudaFreeHost(h->steady_host);
   if (h->imp.pinned) cudaFreeHost(h->imp.pinned);
   if (h->kd.pinned) cudaFreeHost(h->kd.pinned);
   if (h->own_stream) cudaStreamDestroy(h->own_stream);
@@ -764,14 +774,11 @@ int ty_timestep(ty_mesh* h, double cfl, double* dt_out) {
   int rc = ready(h);
   if (rc) return rc;
   if (!dt_out || !(cfl > 0.0)) return TY_ERR_ARG;
-  if ((rc = set_dt_slot(h, 2, 1.7976931348623157e308))) return rc;
+  if ((rc = reset_dt_slots(h, 2, 1))) return rc;
   cudaError_t e = MODE_CALL(h, timestep, h->m, h->s, h->o, h->s.u0, cfl, h->s.dtbits + 2, h->stream, &h->prof);
   if (e != cudaSuccess) return cuda_fail(e, "timestep");
-  unsigned long long b = 0;
-  TY_CU(cudaMemcpyAsync(&b, h->s.dtbits + 2, 8, cudaMemcpyDeviceToHost, h->stream));
   if ((rc = check_err(h))) return rc;
-  double dt;
-  std::memcpy(&dt, &b, 8);
+  const double dt = fetched_dt(h, 2);
   if (dt != dt) return TY_ERR_NANDT;
   *dt_out = dt;
   return TY_OK;
@@ -782,14 +789,13 @@ int ty_residual(ty_mesh* h, double dt, double* R_out) {
   if (rc) return rc;
   if ((rc = ensure_prim(h))) return rc;
   if ((rc = stage_faces(h))) return rc;
-  cudaError_t e = MODE_CALL(h, residual_gather, h->m, h->s, dt, nullptr, h->stream, &h->prof);
+  cudaError_t e = MODE_CALL(h, residual_gather, h->m, h->s, dt, nullptr, h->s.res, h->m.ldc, h->stream, &h->prof);
   if (e != cudaSuccess) return cuda_fail(e, "residual gather");
   if (R_out) {
     const int n = h->m.nci;
     TY_CU(cudaMemcpy2DAsync(R_out, n * sizeof(double), h->s.res, h->m.ldc * sizeof(double), n * sizeof(double), 5,
                             cudaMemcpyDeviceToHost, h->stream));
   }
-  TY_CU(cudaStreamSynchronize(h->stream));
   return check_err(h);
 }
 
@@ -798,8 +804,7 @@ int ty_rk_step(ty_mesh* h, int32_t method, double dt) {
   if (rc) return rc;
   RkTab t;
   if (!rk_table(method, t) || !(dt >= 0.0)) return TY_ERR_ARG;
-  if ((rc = run_step(h, t, dt, nullptr, nullptr, 0.0))) return rc;
-  TY_CU(cudaStreamSynchronize(h->stream));
+  if ((rc = run_step(h, t, dt, nullptr, nullptr, nullptr, 0.0))) return rc;
   return check_err(h);
 }
 
@@ -809,23 +814,17 @@ int ty_rk_steps(ty_mesh* h, int32_t method, double cfl, int32_t nsteps, double* 
   RkTab t;
   if (!rk_table(method, t) || nsteps < 0 || !(cfl > 0.0)) return TY_ERR_ARG;
   if (nsteps == 0) return TY_OK;
-  // slot 0/1 alternate: step n reads slot n%2, its last stage writes the next dt into the other
-  if ((rc = set_dt_slot(h, 0, 1.7976931348623157e308))) return rc;
+  // three slots in turn: step n reads slot n % 3, its last stage writes the next dt into the
+  // following one and resets the third, which the step after will write
+  if ((rc = reset_dt_slots(h, 0, 3))) return rc;
   cudaError_t e = MODE_CALL(h, timestep, h->m, h->s, h->o, h->s.u0, cfl, h->s.dtbits, h->stream, &h->prof);
   if (e != cudaSuccess) return cuda_fail(e, "timestep");
-  for (int n = 0; n < nsteps; ++n) {
-    int cur = n & 1, nxt = cur ^ 1;
-    if ((rc = set_dt_slot(h, nxt, 1.7976931348623157e308))) return rc;
-    if ((rc = run_step(h, t, 0.0, h->s.dtbits + cur, h->s.dtbits + nxt, cfl))) return rc;
-  }
-  if (dt_last) {
-    unsigned long long b;
-    TY_CU(cudaMemcpyAsync(&b, h->s.dtbits + ((nsteps - 1) & 1), 8, cudaMemcpyDeviceToHost, h->stream));
-    TY_CU(cudaStreamSynchronize(h->stream));
-    std::memcpy(dt_last, &b, 8);
-  }
-  TY_CU(cudaStreamSynchronize(h->stream));
-  return check_err(h);
+  for (int n = 0; n < nsteps; ++n)
+    if ((rc = run_step(h, t, 0.0, h->s.dtbits + n % 3, h->s.dtbits + (n + 1) % 3, h->s.dtbits + (n + 2) % 3, cfl)))
+      return rc;
+  rc = check_err(h);
+  if (dt_last) *dt_last = fetched_dt(h, (nsteps - 1) % 3);
+  return rc;
 }
 
 int ty_steady_iteration(ty_mesh* h, int32_t method, double cfl, int32_t local_dt, double* dt_out, double* res_l1) {
@@ -834,8 +833,9 @@ int ty_steady_iteration(ty_mesh* h, int32_t method, double cfl, int32_t local_dt
   RkTab t;
   if (!rk_table(method, t) || !(cfl > 0.0) || !res_l1) return TY_ERR_ARG;
   if (!h->steady_red && (rc = h->alloc(h->steady_red, 3 * (size_t)tyk::kRedBlocks + 3))) return rc;
+  if (!h->steady_host && cudaMallocHost((void**)&h->steady_host, 3 * sizeof(double)) != cudaSuccess) return TY_ERR_NOMEM;
   if (local_dt && !h->steady_dtloc && (rc = h->alloc(h->steady_dtloc, (size_t)h->m.nci))) return rc;
-  if ((rc = set_dt_slot(h, 0, 1.7976931348623157e308))) return rc;
+  if ((rc = reset_dt_slots(h, 0, 1))) return rc;
   cudaError_t e;
   if (local_dt) {  // calc_ns_timestep per cell, kept per cell (calc_zonetimestep.f90:93-117, loc_stab_cond)
     tyk::ImpState im = h->imp;
@@ -845,19 +845,16 @@ int ty_steady_iteration(ty_mesh* h, int32_t method, double cfl, int32_t local_dt
     e = MODE_CALL(h, timestep, h->m, h->s, h->o, h->s.u0, cfl, h->s.dtbits, h->stream, &h->prof);
   }
   if (e != cudaSuccess) return cuda_fail(e, "timestep");
-  if ((rc = run_step(h, t, 0.0, h->s.dtbits, nullptr, cfl, true, local_dt ? h->steady_dtloc : nullptr))) return rc;
+  if ((rc = run_step(h, t, 0.0, h->s.dtbits, nullptr, nullptr, cfl, true, local_dt ? h->steady_dtloc : nullptr))) return rc;
   double* out = h->steady_red + 3 * (size_t)tyk::kRedBlocks;
   e = MODE_CALL(h, res_l1, h->m.nci, h->s.acc, (size_t)h->m.ldc, h->steady_red, out, h->stream);
   if (e != cudaSuccess) return cuda_fail(e, "residual sums");
-  TY_CU(cudaMemcpyAsync(res_l1, out, 3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  if (dt_out) {
-    unsigned long long b;
-    TY_CU(cudaMemcpyAsync(&b, h->s.dtbits, 8, cudaMemcpyDeviceToHost, h->stream));
-    TY_CU(cudaStreamSynchronize(h->stream));
-    std::memcpy(dt_out, &b, 8);
-  }
-  TY_CU(cudaStreamSynchronize(h->stream));
-  return check_err(h);
+  double* host = h->steady_host;
+  TY_CU(cudaMemcpyAsync(host, out, 3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+  rc = check_err(h);
+  std::memcpy(res_l1, host, 3 * sizeof(double));
+  if (dt_out) *dt_out = fetched_dt(h, 0);
+  return rc;
 }
 
 int ty_ghost_state_set(ty_mesh* h, const double* cons_ghost) {

@@ -174,10 +174,12 @@ struct GhostRk {
   cudaError_t residual_faces(const DevMesh& m, const DevState& s, const SpatOpts& o,               \
                              cudaStream_t st, Prof* pr);                                           \
   cudaError_t residual_gather(const DevMesh& m, const DevState& s, double dt,                      \
-                              const unsigned long long* dtbits, cudaStream_t st, Prof* pr);        \
+                              const unsigned long long* dtbits, double* out, int ld,               \
+                              cudaStream_t st, Prof* pr);                                          \
   cudaError_t rk_update(const DevMesh& m, const DevState& s, const SpatOpts& o,                    \
                         const RkStagePlan& plan, double dt, const unsigned long long* dtbits,      \
-                        unsigned long long* dtbits_next, double cfl, cudaStream_t st, Prof* pr);   \
+                        unsigned long long* dtbits_next, unsigned long long* dtbits_reset,         \
+                        double cfl, cudaStream_t st, Prof* pr);                                    \
   cudaError_t timestep(const DevMesh& m, const DevState& s, const SpatOpts& o, const double* cons, \
                        double cfl, unsigned long long* dtbits, cudaStream_t st, Prof* pr);         \
   cudaError_t unpack_state(const DevMesh& m, const DevState& s, cudaStream_t st);                  \

@@ -53,7 +53,7 @@ struct ty_mesh {
   std::vector<int> cf;  // [nslot][nci]
   int lsq_gradmeth = -1, geo_highres = -1;
   bool visc_ready = false;
-  double* dtbits_host = nullptr;  // pinned
+  unsigned long long* ctl_host = nullptr;  // pinned: reset values, then slots and error word read back
   Prof prof;
   tyk::ImpState imp;  // implicit-step matrices and Krylov workspace (allocated on first use)
   tyk::KdifState kd;  // heat-conduction state (ty_kdif_setup)
@@ -82,6 +82,7 @@ struct ty_mesh {
   double* gprim = nullptr;
   bool ghost_rows = false;
   double* steady_red = nullptr;  // [3 kRedBlocks + 3] partial and final residual sums of ty_steady_iteration
+  double* steady_host = nullptr;   // [3] pinned
   double* steady_dtloc = nullptr;  // [nci] per-cell time step of ty_steady_iteration (local_dt)
   cudaStream_t own_stream = nullptr;
 
@@ -109,8 +110,9 @@ struct ty_mesh {
 
 namespace tyi {
 // shared steps of the pipelines (api.cpp)
-int check_err(ty_mesh* h);                       // read and clear the device error word
-int set_dt_slot(ty_mesh* h, int slot, double v); // dtbits[slot] = v (stream-ordered)
+int check_err(ty_mesh* h);                       // wait; read the time-step slots and the device error word (cleared)
+double fetched_dt(const ty_mesh* h, int slot);   // time-step slot as of the last check_err
+int reset_dt_slots(ty_mesh* h, int slot, int count);  // slots = largest finite double (stream-ordered)
 int ensure_prim(ty_mesh* h);                     // primitive variables of the resident state
 int ready(ty_mesh* h);                           // parameters and state present; device set
 int stage_faces(ty_mesh* h);                     // ghost states .. face fluxes of s.prim

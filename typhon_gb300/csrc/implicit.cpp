@@ -532,7 +532,7 @@ int ty_implicit_step(ty_mesh* h, const ty_imp_params* p, ty_imp_stats* st) {
   cudaStream_t s = h->stream;
   const size_t n = 5 * (size_t)m.nci;
   // 1. time step
-  if ((rc = set_dt_slot(h, 0, DBL_MAX))) return rc;
+  if ((rc = reset_dt_slots(h, 0, 1))) return rc;
   IMP_CU(IMP_CALL(h, imp_dtloc, m, S, h->o, im, p->cfl, S.dtbits, s));
   if ((rc = check_err(h))) return rc;
   // 2. residual, Jacobians, assembly

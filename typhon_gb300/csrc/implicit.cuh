@@ -459,7 +459,9 @@ __global__ void __launch_bounds__(kBlock) k_imp_rhs(DevMesh m, DevState s, ImpSt
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= m.nci) return;
   double R[5];
-  gather_residual(m, s, c, R);
+  int es[kMaxSlot];
+  face_list(m, c, es);
+  gather_residual(m, s, es, R);
   const double coef = imp_dt(im, a, c) / m.cvol[c];
 #pragma unroll
   for (int v = 0; v < 5; ++v) out[5 * (size_t)c + v] = coef * R[v];
