@@ -468,41 +468,48 @@ __device__ void adj_recon_f(const DevMesh& m, const SpatOpts& o, const AdjSide& 
     }
     return;
   }
-  // G . CF - g (u . CF) = G . w with w = CF - (u . CF) u, the no-limiter weights (recw)
+  // G . CF - g (u . CF) = G . w with w = CF - (u . CF) u, the no-limiter weights (recw).
+  // With D = a^2 + b^2, MUSCL (a = 2g - b): phi = 2g ab/D, dphi/db = (2g/D)^2 (a - b) 2g,
+  // dphi/dg = 2 ab/D - (2g/D)^2 2 (a - b) b; MUSCL-UNS (a = g): phi = ab (a + b)/D,
+  // dphi/da = b^2 (b^2 - a^2 + 2ab)/D^2, dphi/db = a^2 (a^2 - b^2 + 2ab)/D^2.  ab > 0 is read from
+  // its upper word (normal numbers), and the derivatives are selected, not branched to.
   const bool uns = o.highres == TY_HRES_MUSCLUNS;
-  const double ux = m.uLR[F], uy = m.uLR[lf + F], uz = m.uLR[2 * lf + F];
+  const F64 ux = m.uLR[F], uy = m.uLR[lf + F], uz = m.uLR[2 * lf + F];
   const double* w = m.recw + (4 * sd.side) * lf + F;
-  const double wx = w[0], wy = w[lf], wz = w[2 * lf];
+  const F64 wx = w[0], wy = w[lf], wz = w[2 * lf];
   const double* CF = sd.side ? m.RF : m.LF;
-  const double uc = ux * CF[F] + uy * CF[lf + F] + uz * CF[2 * lf + F];
-  const double idLR = sd.side ? -m.invdLR[F] : m.invdLR[F];
-  double ruc[3];
+  const F64 uc = fma(ux, F64(CF[F]), fma(uy, F64(CF[lf + F]), uz * F64(CF[2 * lf + F])));
+  const F64 idLR = sd.side ? -m.invdLR[F] : m.invdLR[F];
+  F64 nruc[3];  // -r (u . CF): kept with its sign, a negation of its own would be an FP64 instruction
 #pragma unroll
-  for (int k = 0; k < 3; ++k) ruc[k] = O[20 + k] * uc;
+  for (int k = 0; k < 3; ++k) nruc[k] = F64(O[20 + k]) * -uc;
 #pragma unroll
   for (int v = 0; v < 5; ++v) {
-    const double gx = O[5 + 3 * v], gy = O[6 + 3 * v], gz = O[7 + 3 * v];
-    const double g = gx * ux + gy * uy + gz * uz;
-    const double LR = (N[v] - O[v]) * idLR;
-    const double a = uns ? g : 2.0 * g - LR, b = LR;
-    const double ab = a * b;
-    const double rc = ruc[v < 2 ? v : 2];
-    // phi = a b (a + b) / D, D = a^2 + b^2; dphi/da = b^2 (b^2 - a^2 + 2ab) / D^2,
-    // dphi/db = a^2 (a^2 - b^2 + 2ab) / D^2
-    double phi = 0.0, cgv = -rc, cqv = 0.0;
-    if (ab > 0.0) {
-      const double a2 = a * a, b2 = b * b, iD = rcp_nr(a2 + b2);
-      phi = ab * (a + b) * iD;
-      const double dl = b2 - a2;
-      const double X = b2 * fma(2.0, ab, dl), Y = a2 * fma(2.0, ab, -dl);  // D^2 dphi/da, D^2 dphi/db
-      const double k1 = rc * (iD * iD);
-      cgv = uns ? fma(X, k1, -rc) : fma(2.0 * X, k1, -rc);
-      cqv = (uns ? Y : Y - X) * k1 * idLR;
+    const F64 gx = O[5 + 3 * v], gy = O[6 + 3 * v], gz = O[7 + 3 * v], qo = O[v];
+    const F64 g = fma(gx, ux, fma(gy, uy, gz * uz)), b = (F64(N[v]) - qo) * idLR;
+    const F64 nrc = nruc[v < 2 ? v : 2];
+    F64 phi, cgv, cqv;
+    bool pos;
+    if (uns) {
+      const F64 ab = g * b, a2 = g * g, b2 = b * b, iD = rcp_nr(a2 + b2), dl = b2 - a2, h = ab + ab;
+      pos = __double2hiint(ab.v) >= 1 << 20;
+      const F64 k1 = nrc * (iD * iD);
+      phi = ab * (g + b) * iD;
+      cgv = fma(-(b2 * (h + dl)), k1, nrc);
+      cqv = (a2 * (h - dl)) * k1 * -idLR;
+    } else {
+      const F64 g2 = g + g, a = g2 - b, ab = a * b, iD = rcp_nr(fma(a, a, b * b));
+      pos = __double2hiint(ab.v) >= 1 << 20;
+      const F64 t = ab * iD, mm = g2 * iD, k = mm * (mm * (a - b)) * nrc;
+      phi = g2 * t;
+      cgv = fma(b + b, k, fma(-(t + t), nrc, nrc));
+      cqv = g2 * k * -idLR;
     }
-    const double inc = fma(phi, uc, gx * wx + gy * wy + gz * wz);
-    q[v] = fma(O[20 + (v < 2 ? v : 2)], inc, O[v]);
-    cg[v] = cgv;
-    cq[v] = cqv;
+    phi = pos ? phi.v : 0.0;
+    const F64 inc = fma(phi, uc, fma(gx, wx, fma(gy, wy, gz * wz)));
+    q[v] = fma(F64(O[20 + (v < 2 ? v : 2)]), inc, qo).v;
+    cg[v] = pos ? cgv.v : nrc.v;
+    cq[v] = pos ? cqv.v : 0.0;
   }
 }
 
@@ -525,17 +532,17 @@ __device__ void adj_recon_b(const DevMesh& m, const SpatOpts& o, const AdjSide& 
     }
     return;
   }
-  const double ux = m.uLR[F], uy = m.uLR[lf + F], uz = m.uLR[2 * lf + F];
+  const F64 ux = m.uLR[F], uy = m.uLR[lf + F], uz = m.uLR[2 * lf + F];
   const double* CF = sd.side ? m.RF : m.LF;
-  const double cx = CF[F], cy = CF[lf + F], cz = CF[2 * lf + F];
+  const F64 cx = CF[F], cy = CF[lf + F], cz = CF[2 * lf + F];
 #pragma unroll
   for (int v = 0; v < 5; ++v) {
-    const double db = O[20 + (v < 2 ? v : 2)] * Qb[v], gb = cg[v] * Qb[v], dqb = cq[v] * Qb[v];
-    own[v] = Qb[v] - dqb;
-    oth[v] = dqb;
-    G[3 * v] = db * cx + gb * ux;
-    G[3 * v + 1] = db * cy + gb * uy;
-    G[3 * v + 2] = db * cz + gb * uz;
+    const F64 b = Qb[v], db = F64(O[20 + (v < 2 ? v : 2)]) * b, gb = F64(cg[v]) * b, dqb = F64(cq[v]) * b;
+    own[v] = (b - dqb).v;
+    oth[v] = dqb.v;
+    G[3 * v] = fma(db, cx, gb * ux).v;
+    G[3 * v + 1] = fma(db, cy, gb * uy).v;
+    G[3 * v + 2] = fma(db, cz, gb * uz).v;
   }
 }
 
@@ -546,8 +553,118 @@ __device__ __forceinline__ void adj_store_g(double* rec, const double G[15]) {
   o[7] = make_double2(G[14], 0.0);
 }
 
+struct HllcSuper {
+  double vqb, q0b, pb, reb, m0;
+};
+// Reverse of the flux of one side alone (supersonic faces): a call, so that it is not
+// if-converted into the subsonic path.
+__device__ __noinline__ HllcSuper hllc_vjp_super(double vq, double q0, double p, double re, double A, double B, double C) {
+  return {A * q0 + B * (re + p), A * vq, B * vq + C, B * vq, vq * q0};
+}
+
+// hllc_vjp (adjoint_flux.cuh) for the fast mode: Lb, Rb = (dF/dL, dF/dR)^T Fb of the same flux, in
+// the regrouped form of flux_hllc_fast and traversed backwards.  One reverse of the side that
+// gives the flux, picked by selects and added to that side's results; the wave speeds reversed
+// through T = p/rho and k_r (am^2 = g (k_l T_l + k_r T_r) + (g - 1)/2 k_l k_r |du|^2, vm = vn_l + k_r
+// dvn, d k_r = k_l k_r d ln(rho_r/rho_l)/2) and not through enthalpies; reciprocal roots serve as
+// root and as its derivative's divisor.  About 190 FP64 operations for 340, none of them a
+// comparison or predicated off, all DFMA (F64).
+__device__ __forceinline__ void hllc_vjp_fast(const SpatOpts& o, const double* QL, const double* QR, double nxd,
+                                              double nyd, double nzd, const double* Fbd, double* QLb, double* QRb) {
+  const F64 g = o.gamma, hg1 = 0.5 * (o.gamma - 1.0), ig1 = o.ig1;
+  const F64 n[3] = {nxd, nyd, nzd};
+  F64 L[5], R[5], Fb[5];
+#pragma unroll
+  for (int v = 0; v < 5; ++v) { L[v] = QL[v]; R[v] = QR[v]; Fb[v] = Fbd[v]; }
+  // forward
+  const F64 P = L[0] * R[0], y = rsqrt_nr(P), y2 = y * y, rroe = P * y, inv = rcp_nr(L[0] + rroe);
+  const F64 kl = L[0] * inv, kr = rroe * inv, kk = kl * kr;
+  const F64 iL = y2 * R[0], iR = y2 * L[0], TL = L[1] * iL, TR = R[1] * iR;
+  const F64 d[3] = {R[2] - L[2], R[3] - L[3], R[4] - L[4]};
+  const F64 dd = fma(d[0], d[0], fma(d[1], d[1], d[2] * d[2]));
+  const F64 vnl = fma(L[2], n[0], fma(L[3], n[1], L[4] * n[2])), vnr = fma(R[2], n[0], fma(R[3], n[1], R[4] * n[2]));
+  const F64 dvn = vnr - vnl, vm = fma(kr, dvn, vnl);
+  const F64 al2 = g * TL, ar2 = g * TR, am2 = fma(g, fma(kl, TL, kr * TR), hg1 * (kk * dd));
+  const F64 yl = rsqrt_nr(al2), yr = rsqrt_nr(ar2), ym = rsqrt_nr(am2);
+  const F64 am = am2 * ym, l1 = fma(-al2, yl, vnl), l2 = vm - am, r1 = fma(ar2, yr, vnr), r2 = vm + am;
+  const bool slm = order_key(l2.v) < order_key(l1.v), srm = order_key(r1.v) < order_key(r2.v);
+  const F64 sl = slm ? l2 : l1, sr = srm ? r2 : r1;
+  const F64 dl = sl - vnl, dr = sr - vnr, rql = L[0] * dl, rqr = R[0] * dr;
+  const F64 iden = rcp_nr(rqr - rql);
+  const F64 Sst = (fma(rqr, vnr, fma(-rql, vnl, L[1])) - R[1]) * iden;
+  const bool supl = !is_neg(sl.v), supr = !supl && (is_neg(sr.v) || __double2hiint(sr.v) == 0);
+  const bool left = supl || (!supr && !is_neg(Sst.v));
+  const F64 q0 = left ? L[0] : R[0], p = left ? L[1] : R[1];
+  const F64 q[3] = {left ? L[2] : R[2], left ? L[3] : R[3], left ? L[4] : R[4]};
+  const F64 vq = left ? vnl : vnr;
+  const F64 hq = F64(0.5) * fma(q[0], q[0], fma(q[1], q[1], q[2] * q[2])), re = fma(ig1, p, hq * q0);
+  // reverse: F = (m0, E, m0 q + c n); A, B, C the adjoints of m0, E, c
+  const F64 A = fma(Fb[2], q[0], fma(Fb[3], q[1], fma(Fb[4], q[2], Fb[0]))), B = Fb[1];
+  const F64 C = fma(Fb[2], n[0], fma(Fb[3], n[1], Fb[4] * n[2]));
+  // adjoints of the side's vn, s (at fixed rho s), rho, p, rho E; of S*'s numerator; of rho_k (s_k - vn_k)
+  F64 vqb, sqb = 0.0, q0b = 0.0, pb, reb, m0, Nb = 0.0, rqlb = 0.0, rqrb = 0.0;
+  if (supl || supr) {
+    const HllcSuper h = hllc_vjp_super(vq.v, q0.v, p.v, re.v, A.v, B.v, C.v);
+    vqb = h.vqb; q0b = h.q0b; pb = h.pb; reb = h.reb; m0 = h.m0;
+  } else {
+    const F64 sq = left ? sl : sr, ds = left ? dl : dr, rq = left ? rql : rqr;
+    const F64 i = rcp_nr(sq - Sst), dv = Sst - vq, dp = rq * dv, pst = p + dp, w = Sst * i;
+    const F64 E1 = fma(re, ds, fma(pst, Sst, -(p * vq)));  // E = w E1 + S* p*
+    m0 = w * rq;
+    const F64 wb = fma(B, E1, fma(A, rq, C * dp)), E1b = B * w, BE = B + E1b;
+    const F64 pstb = fma(BE, Sst, C), dpb = fma(C, w, pstb), dpr = dpb * rq;
+    pb = fma(-E1b, vq, pstb);
+    reb = E1b * ds;
+    const F64 t = wb * i, tw = t * w, er = E1b * re;
+    sqb = er - tw;
+    vqb = fma(-E1b, re + p, -dpr);
+    Nb = (fma(BE, pst, dpr) + (t + tw)) * iden;
+    const F64 rqb = fma(A, w, dpb * dv);
+    rqlb = Nb * (Sst - vnl);
+    rqrb = Nb * (vnr - Sst);
+    const F64 b = (left ? rqlb : rqrb) + rqb;
+    rqlb = left ? b : rqlb;
+    rqrb = left ? rqrb : b;
+  }
+  const auto add = [left](F64& l, F64& r, F64 x) {
+    const F64 s = (left ? l : r) + x;
+    l = left ? s : l;
+    r = left ? r : s;
+  };
+  const F64 dlb = rqlb * L[0], drb = rqrb * R[0];
+  F64 slb = dlb, srb = drb, vnlb = fma(-Nb, rql, -dlb), vnrb = fma(Nb, rqr, -drb);
+  F64 rlb = rqlb * dl, rrb = rqrb * dr, plb = Nb, prb = -Nb;
+  add(slb, srb, sqb);
+  add(vnlb, vnrb, vqb);
+  add(rlb, rrb, fma(hq, reb, q0b));
+  add(plb, prb, fma(ig1, reb, pb));
+  // wave speeds
+  const F64 zero = 0.0, slmb = slm ? slb : zero, srmb = srm ? srb : zero;
+  const F64 vmb = slmb + srmb, Hb = F64(0.5) * ((srmb - slmb) * ym), gH = g * Hb, hg = 0.5 * o.gamma;
+  const F64 TLb = fma(gH, kl, -(slm ? zero : slb) * (hg * yl)), TRb = fma(gH, kr, (srm ? zero : srb) * (hg * yr));
+  vnlb = fma(vmb, kl, vnlb + (slm ? zero : slb));
+  vnrb = fma(vmb, kr, vnrb + (srm ? zero : srb));
+  const F64 hH = hg1 * Hb, e = F64(2.0) * (hH * kk);
+  const F64 krb = fma(vmb, dvn, fma(gH, TR - TL, hH * ((kl - kr) * dd))), hk = F64(0.5) * (krb * kk);
+  QLb[0] = fma(-iL, fma(TLb, TL, hk), rlb).v;
+  QRb[0] = fma(iR, fma(-TRb, TR, hk), rrb).v;
+  QLb[1] = fma(TLb, iL, plb).v;
+  QRb[1] = fma(TRb, iR, prb).v;
+  const F64 kq = q0 * reb;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const F64 ed = e * d[k];
+    F64 l = fma(vnlb, n[k], -ed), r = fma(vnrb, n[k], ed);
+    const F64 s = fma(m0, Fb[2 + k], fma(kq, q[k], left ? l : r));
+    QLb[2 + k] = (left ? s : l).v;
+    QRb[2 + k] = (left ? r : s).v;
+  }
+}
+
 // per face: lambda_F, the flux products at the reconstructed states, both reconstructions
-// reversed, summed per destination cell into the face record
+// reversed, summed per destination cell into the face record.  Bound by the FP64 pipe: HLLC with
+// van Albada issues 649 FP64 instructions a face (787 as plain double with branches), 327,680
+// faces in 406 us (552), the pipe 87 % busy at three warps per SM quarter.
 template <int SCH>
 __device__ __forceinline__ void adj_face2f(const DevMesh& m, const SpatOpts& o, const double* __restrict__ crec,
                                            double* __restrict__ frec, int f) {
@@ -560,14 +677,14 @@ __device__ __forceinline__ void adj_face2f(const DevMesh& m, const SpatOpts& o, 
   const double S = m.fs[f];
   double Fb[5], QL[5], QR[5], cg0[5], cq0[5], cg1[5], cq1[5];
 #pragma unroll
-  for (int v = 0; v < 5; ++v) Fb[v] = interior ? S * (B[23 + v] - A[23 + v]) : -S * A[23 + v];
+  for (int v = 0; v < 5; ++v) Fb[v] = (F64(S) * ((interior ? F64(B[23 + v]) : F64(0.0)) - F64(A[23 + v]))).v;
   const AdjSide s0{A, B, f, 0}, s1{B, A, F1, interior ? 1 : 0};
   adj_recon_f(m, o, s0, QL, cg0, cq0);
   adj_recon_f(m, o, s1, QR, cg1, cq1);
   double QLb[5] = {0, 0, 0, 0, 0}, QRb[5] = {0, 0, 0, 0, 0};
   const size_t lf = m.ldf;
   const double nx = m.fn[f], ny = m.fn[lf + f], nz = m.fn[2 * lf + f];
-  if constexpr (SCH == TY_SCH_HLLC) hllc_vjp(o.gamma, QL, QR, nx, ny, nz, Fb, QLb, QRb);
+  if constexpr (SCH == TY_SCH_HLLC) hllc_vjp_fast(o, QL, QR, nx, ny, nz, Fb, QLb, QRb);
   else if constexpr (SCH == TY_SCH_RUSANOV) rusanov_vjp(o.gamma, QL, QR, nx, ny, nz, Fb, QLb, QRb);
   else roe_vjp(o.gamma, o.entropy_fix, QL, QR, nx, ny, nz, Fb, QLb, QRb);
   double* rec = frec + (size_t)f * kAdjFace;
@@ -580,7 +697,7 @@ __device__ __forceinline__ void adj_face2f(const DevMesh& m, const SpatOpts& o, 
   // other cell; to the right-state cell the converse
   double d[12];
 #pragma unroll
-  for (int v = 0; v < 5; ++v) { d[v] = own0[v] + oth1[v]; d[5 + v] = own1[v] + oth0[v]; }
+  for (int v = 0; v < 5; ++v) { d[v] = (F64(own0[v]) + F64(oth1[v])).v; d[5 + v] = (F64(own1[v]) + F64(oth0[v])).v; }
   d[10] = 0.0; d[11] = 0.0;
   double2* oq = reinterpret_cast<double2*>(rec + 32);
 #pragma unroll
@@ -606,7 +723,8 @@ __global__ void __launch_bounds__(128, 3) k_adj_face2f_roe(DevMesh m, SpatOpts o
 // weights: the cell's own term is added to qb [5][ldc], and the term of each neighbour
 // (G_c = Wown q_c + sum over slots wo_slot q_nb) is written to ctb [nf][2][5] at the face and
 // this cell's side, for the neighbour's gather (k_adj_cell3f).  NS >= nslot: the slot loop is
-// unrolled so that every record load is issued before the first is used.
+// unrolled so that every record load is issued before the first is used.  163,840 tetrahedra:
+// 73 us with additions as DADD, 68 as F64 (FP64 pipe 82 % busy).
 template <int NS>
 __global__ void __launch_bounds__(kBlock) k_adj_cell2f(DevMesh m, const double* __restrict__ frec,
                                                        const double* __restrict__ wtab, double* __restrict__ qb,
@@ -625,7 +743,7 @@ __global__ void __launch_bounds__(kBlock) k_adj_cell2f(DevMesh m, const double* 
     rf[2 * sl + 1] = (e >= 0 && !side && f >= m.nfi) ? m.part[f] : -1;
     rs[2 * sl + 1] = 1;
   }
-  double q[5] = {0, 0, 0, 0, 0}, g[16];
+  F64 q[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, g[16];
 #pragma unroll
   for (int k = 0; k < 16; ++k) g[k] = 0.0;
 #pragma unroll
@@ -636,29 +754,29 @@ __global__ void __launch_bounds__(kBlock) k_adj_cell2f(DevMesh m, const double* 
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const double2 t = rg[k];
-      g[2 * k] += t.x;
-      g[2 * k + 1] += t.y;
+      g[2 * k] = g[2 * k] + t.x;
+      if (k < 7) g[2 * k + 1] = g[2 * k + 1] + t.y;  // the sixteenth is padding
     }
 #pragma unroll
-    for (int v = 0; v < 5; ++v) q[v] += r[32 + 5 * rs[i] + v];
+    for (int v = 0; v < 5; ++v) q[v] = q[v] + r[32 + 5 * rs[i] + v];
   }
   {
-    const double wx = wtab[c], wy = wtab[n + c], wz = wtab[2 * n + c];
+    const F64 wx = wtab[c], wy = wtab[n + c], wz = wtab[2 * n + c];
 #pragma unroll
-    for (int v = 0; v < 5; ++v) q[v] += wx * g[3 * v] + wy * g[3 * v + 1] + wz * g[3 * v + 2];
+    for (int v = 0; v < 5; ++v) q[v] = fma(wx, g[3 * v], fma(wy, g[3 * v + 1], fma(wz, g[3 * v + 2], q[v])));
   }
   const size_t ld = m.ldc;
 #pragma unroll
-  for (int v = 0; v < 5; ++v) qb[v * ld + c] = q[v];
+  for (int v = 0; v < 5; ++v) qb[v * ld + c] = q[v].v;
 #pragma unroll
   for (int sl = 0; sl < NS; ++sl) {
     const int f = rf[2 * sl];
     if (f < 0) continue;
     const double* w = wtab + (3 + 3 * (size_t)sl) * n + c;
-    const double wx = w[0], wy = w[n], wz = w[2 * n];
+    const F64 wx = w[0], wy = w[n], wz = w[2 * n];
     double* o = ctb + (size_t)f * 10 + 5 * rs[2 * sl];
 #pragma unroll
-    for (int v = 0; v < 5; ++v) o[v] = wx * g[3 * v] + wy * g[3 * v + 1] + wz * g[3 * v + 2];
+    for (int v = 0; v < 5; ++v) o[v] = fma(wx, g[3 * v], fma(wy, g[3 * v + 1], wz * g[3 * v + 2])).v;
   }
 }
 
@@ -801,7 +919,7 @@ __global__ void __launch_bounds__(128) k_adj_face1f(DevMesh m, SpatOpts o, const
   double QLb[5] = {0, 0, 0, 0, 0}, QRb[5] = {0, 0, 0, 0, 0};
   const size_t lf = m.ldf;
   const double nx = m.fn[f], ny = m.fn[lf + f], nz = m.fn[2 * lf + f];
-  if constexpr (SCH == TY_SCH_HLLC) hllc_vjp(o.gamma, QL, QR, nx, ny, nz, Fb, QLb, QRb);
+  if constexpr (SCH == TY_SCH_HLLC) hllc_vjp_fast(o, QL, QR, nx, ny, nz, Fb, QLb, QRb);
   else if constexpr (SCH == TY_SCH_RUSANOV) rusanov_vjp(o.gamma, QL, QR, nx, ny, nz, Fb, QLb, QRb);
   else roe_vjp(o.gamma, o.entropy_fix, QL, QR, nx, ny, nz, Fb, QLb, QRb);
   if (!two) {
