@@ -687,6 +687,7 @@ int ty_set_params(ty_mesh* h, const ty_spat_params* p) {
   h->o.inv_entropy_fix = p->entropy_fix > 0.0 ? 1.0 / p->entropy_fix : 0.0;
   h->o.ig1 = 1.0 / (p->gamma - 1.0);
   h->o.gig1 = p->gamma * h->o.ig1;
+  h->o.gdg1 = p->gamma / (p->gamma - 1.0);
   h->o.roe_sub = 1.0 - p->entropy_fix;
   h->o.irgas = p->rgas != 0.0 ? 1.0 / p->rgas : 0.0;
   h->o.iprandtl = p->prandtl != 0.0 ? 1.0 / p->prandtl : 0.0;

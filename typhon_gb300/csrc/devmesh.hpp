@@ -87,7 +87,8 @@ struct SpatOpts {
   int scheme, highres, limiter, postlim, gradmeth, mode;
   double gamma, entropy_fix;
   double inv_entropy_fix;  // 1 / entropy_fix (fast-mode Roe flux)
-  double ig1, gig1;        // 1 / (gamma - 1), gamma / (gamma - 1) (fast-mode fluxes)
+  double ig1, gig1;        // 1 / (gamma - 1), gamma times it (fast-mode fluxes)
+  double gdg1;             // gamma / (gamma - 1), divided (exact-mode fluxes)
   double roe_sub;          // 1 - entropy_fix: |u.n| up to this times a is outside the entropy fix
   double irgas, iprandtl;  // 1 / rgas, 1 / prandtl (0 when not set)
   // HLL family (TY_SCH_HLLC / HLLE and their B, K, KB variants): 1 HLLC, 2 HLLE, 0 other;

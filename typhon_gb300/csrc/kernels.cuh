@@ -318,70 +318,149 @@ __global__ void k_ghost_prim(DevMesh m, double* __restrict__ prim, SpatOpts o) {
   prim[4 * ld + g] = vz;
 }
 
+// Comparisons of doubles run on the FP64 pipe (a minimum is a comparison and a select); on bit
+// patterns they run on the integer pipe.
+__device__ __forceinline__ long long order_key(double x) {  // orders like x
+  const long long b = __double_as_longlong(x);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+__device__ __forceinline__ double min_bits(double a, double b) { return order_key(a) < order_key(b) ? a : b; }
+__device__ __forceinline__ double max_bits(double a, double b) { return order_key(a) < order_key(b) ? b : a; }
+__device__ __forceinline__ bool is_neg(double x) { return __double2hiint(x) < 0; }  // sign bit
+// x without the sign (fabs of a stored value is an FP64 instruction)
+__device__ __forceinline__ double abs_bits(double x) {
+  return __hiloint2double(__double2hiint(x) & 0x7fffffff, __double2loint(x));
+}
+
+__device__ __forceinline__ long long dbits(double x) { return __double_as_longlong(x); }
+
+// x == 0 on the integer pipe (on the 32-bit halves: the compiler turns a test of the 64-bit
+// pattern back into an FP64 comparison)
+__device__ __forceinline__ bool is_zero(double x) {
+  return (((unsigned)__double2hiint(x) << 1) | (unsigned)__double2loint(x)) == 0u;
+}
+
+// |x| as an FP32 number, truncated (relative error below 2^-23) on the integer pipe, when x lies
+// in [2^-60, 2^60); ok is cleared otherwise.
+__device__ __forceinline__ float trunc32(double x, bool& ok) {
+  const int hi = __double2hiint(x) & 0x7fffffff;
+  ok = ok && (unsigned)(hi - ((1023 - 60) << 20)) < (unsigned)(120 << 20);
+  return __uint_as_float(__funnelshift_l((unsigned)__double2loint(x), (unsigned)hi, 3) - ((1023u - 127u) << 23));
+}
+
+// Exact mode: double arithmetic issued as F64 (fastmath.cuh: the same rounded values, and at
+// -fmad=false nothing is contracted); the fast mode's compiler contracts plain doubles itself.
+using X64 = typename std::conditional<kFast, double, F64>::type;
+
+// a / b correctly rounded for several a and one b: with y = 1/b correctly rounded, q0 = a y
+// corrected once by its residual is within an ulp of a/b, and corrected again it is the
+// correctly rounded quotient (P. Markstein, "Computation of elementary functions on the IBM
+// RISC System/6000 processor", IBM J. Res. Dev. 34 (1990): q + (a - b q) y with exact residual).
+// Five fused multiply-adds where an IEEE division issues about ten FP64 instructions.  Exponents are limited so that no residual leaves the normal range; zeros
+// keep their sign (q0); anything else sets `bad` and is divided by div_ieee.
+struct Divisor {
+  F64 b, y;
+  bool ok;
+};
+__device__ __forceinline__ Divisor divisor(double b) {
+  return {b, 1.0 / b, ((unsigned)(__double2hiint(b) >> 20) & 0x7ffu) - 823u <= 400u};
+}
+__device__ __forceinline__ F64 quotient(F64 a, const Divisor& d, bool& bad) {
+  const unsigned hi = (unsigned)__double2hiint(a.v);
+  const bool zero = ((hi << 1) | (unsigned)__double2loint(a.v)) == 0u;
+  bad = bad || !d.ok || (!zero && ((hi >> 20) & 0x7ffu) - 323u > 1400u);
+  const F64 q0 = a * d.y, q1 = fma(fma(-d.b, q0, a), d.y, q0), q2 = fma(fma(-d.b, q1, a), d.y, q1);
+  return zero ? q0.v : q2.v;
+}
+__device__ __noinline__ double div_ieee(double a, double b) { return a / b; }
+__device__ __forceinline__ F64 quotient(F64 a, const Divisor& d) {
+  bool bad = false;
+  F64 q = quotient(a, d, bad);
+  if (bad) q = div_ieee(a.v, d.b.v);
+  return q;
+}
+
+// A cell's face list read ahead of its use (and of the wait): one trip to L2 less.
+__device__ __forceinline__ void face_list(const DevMesh& m, int c, int es[kMaxSlot]) {
+#pragma unroll
+  for (int sl = 0; sl < kMaxSlot; ++sl) es[sl] = sl < m.nslot ? m.cf[sl * (size_t)m.nci + c] : -1;
+}
+
 // ---------------------------------------------------------------------------
 // least-squares gradient: b_c = sum_f (q(fc2) - q(fc1)) d_f over the cell's faces in colour
 // order, then the Cholesky solve (exact) or, in fast mode, the precomputed A^-1 d weights.
+// The solve divides by three numbers, ten times each: their reciprocals once and quotient().
+// 87,880 tetrahedra: 95 us with IEEE divisions, 60 us.
+__device__ __noinline__ double3 cholesky_ieee(double x1, double x2, double x3, double L11, double L21, double L31,
+                                              double L22, double L32, double L33) {
+  x1 = x1 / L11;
+  x2 = x2 - L21 * x1;
+  x2 = x2 / L22;
+  x3 = x3 - L31 * x1;
+  x3 = x3 - L32 * x2;
+  x3 = x3 / L33;
+  x3 = x3 / L33;
+  x2 = x2 - L32 * x3;
+  x2 = x2 / L22;
+  x1 = x1 - L21 * x2;
+  x1 = x1 - L31 * x3;
+  x1 = x1 / L11;
+  return make_double3(x1, x2, x3);
+}
+
 __global__ void __launch_bounds__(kBlock) k_grad(DevMesh m, DevState s) {
-  pdl_wait();
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= m.nci) return;
-  const size_t ld = m.ldc;
-  double b[15];
+  int es[kMaxSlot];
+  face_list(m, c, es);
+  pdl_wait();
+  const size_t ld = m.ldc, n = m.nci;
+  X64 b[15];
 #pragma unroll
   for (int k = 0; k < 15; ++k) b[k] = 0.0;
   const double* __restrict__ prim = s.prim;
-  for (int sl = 0; sl < m.nslot; ++sl) {
-    int e = m.cf[sl * (size_t)m.nci + c];
+#pragma unroll
+  for (int sl = 0; sl < kMaxSlot; ++sl) {
+    const int e = es[sl];
     if (e < 0) break;
-    int f = e >> 1;
-    int i1 = m.fc1[f], i2 = m.fc2[f];
-    if constexpr (kFast) {
-      const int side = e & 1;
-      const double wx = d3(m.lsqw, m.ldf, f, 3 * side), wy = d3(m.lsqw, m.ldf, f, 3 * side + 1),
-                   wz = d3(m.lsqw, m.ldf, f, 3 * side + 2);
+    const int f = e >> 1;
+    const int i1 = m.fc1[f], i2 = m.fc2[f];
+    const int side = kFast ? e & 1 : 0;
+    const double* w = kFast ? m.lsqw : m.dcg;
+    const X64 wx = d3(w, m.ldf, f, 3 * side), wy = d3(w, m.ldf, f, 3 * side + 1), wz = d3(w, m.ldf, f, 3 * side + 2);
 #pragma unroll
-      for (int v = 0; v < 5; ++v) {
-        double dsca = prim[v * ld + i2] - prim[v * ld + i1];
-        b[3 * v] = fma(dsca, wx, b[3 * v]);
-        b[3 * v + 1] = fma(dsca, wy, b[3 * v + 1]);
-        b[3 * v + 2] = fma(dsca, wz, b[3 * v + 2]);
-      }
-    } else {
-      const double dx = d3(m.dcg, m.ldf, f, 0), dy = d3(m.dcg, m.ldf, f, 1), dz = d3(m.dcg, m.ldf, f, 2);
-#pragma unroll
-      for (int v = 0; v < 5; ++v) {
-        double dsca = prim[v * ld + i2] - prim[v * ld + i1];
-        b[3 * v] = b[3 * v] + dsca * dx;
-        b[3 * v + 1] = b[3 * v + 1] + dsca * dy;
-        b[3 * v + 2] = b[3 * v + 2] + dsca * dz;
-      }
+    for (int v = 0; v < 5; ++v) {
+      const X64 dsca = X64(prim[v * ld + i2]) - X64(prim[v * ld + i1]);
+      b[3 * v] = b[3 * v] + dsca * wx;
+      b[3 * v + 1] = b[3 * v + 1] + dsca * wy;
+      b[3 * v + 2] = b[3 * v + 2] + dsca * wz;
     }
   }
   if constexpr (!kFast) {
-    const double L11 = m.lsq[c], L21 = m.lsq[m.nci + c], L31 = m.lsq[2 * (size_t)m.nci + c];
-    const double L22 = m.lsq[3 * (size_t)m.nci + c], L32 = m.lsq[4 * (size_t)m.nci + c];
-    const double L33 = m.lsq[5 * (size_t)m.nci + c];
+    const F64 L21 = m.lsq[n + c], L31 = m.lsq[2 * n + c], L32 = m.lsq[4 * n + c];
+    const Divisor L11 = divisor(m.lsq[c]), L22 = divisor(m.lsq[3 * n + c]), L33 = divisor(m.lsq[5 * n + c]);
     // cholesky_solve (MATRIX.f90:79-111), column per variable
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
-      double x1 = b[3 * v], x2 = b[3 * v + 1], x3 = b[3 * v + 2];
-      x1 = x1 / L11;
-      x2 = x2 - L21 * x1;
-      x2 = x2 / L22;
-      x3 = x3 - L31 * x1;
-      x3 = x3 - L32 * x2;
-      x3 = x3 / L33;
-      x3 = x3 / L33;
-      x2 = x2 - L32 * x3;
-      x2 = x2 / L22;
-      x1 = x1 - L21 * x2;
-      x1 = x1 - L31 * x3;
-      x1 = x1 / L11;
-      b[3 * v] = x1; b[3 * v + 1] = x2; b[3 * v + 2] = x3;
+      bool bad = false;
+      const F64 y1 = quotient(b[3 * v], L11, bad);
+      const F64 y2 = quotient(b[3 * v + 1] - L21 * y1, L22, bad);
+      const F64 y3 = quotient((b[3 * v + 2] - L31 * y1) - L32 * y2, L33, bad);
+      const F64 x3 = quotient(y3, L33, bad);
+      const F64 x2 = quotient(y2 - L32 * x3, L22, bad);
+      const F64 x1 = quotient((y1 - L21 * x2) - L31 * x3, L11, bad);
+      double3 x = make_double3(x1.v, x2.v, x3.v);
+      if (bad)
+        x = cholesky_ieee(value(b[3 * v]), value(b[3 * v + 1]), value(b[3 * v + 2]), L11.b.v, L21.v, L31.v, L22.b.v, L32.v,
+                          L33.b.v);
+      s.grad[3 * v * ld + c] = x.x;
+      s.grad[(3 * v + 1) * ld + c] = x.y;
+      s.grad[(3 * v + 2) * ld + c] = x.z;
     }
-  }
+  } else {
 #pragma unroll
-  for (int k = 0; k < 15; ++k) s.grad[k * ld + c] = b[k];
+    for (int k = 0; k < 15; ++k) s.grad[k * ld + c] = value(b[k]);
+  }
 }
 
 __global__ void k_ghost_grad(DevMesh m, double* __restrict__ grad) {
@@ -420,42 +499,53 @@ __global__ void k_ghost_grad(DevMesh m, double* __restrict__ grad) {
 
 // ---------------------------------------------------------------------------
 // High-order face state on one side of face f (side 0: cell fc1 "L", side 1: cell fc2 "R").
-__device__ void recon(const DevMesh& m, const DevState& s, const SpatOpts& o, int f, int side, double q[5]) {
-  const size_t ld = m.ldc;
+// LR: (q(fc2) - q(fc1)) / |C_L C_R|, the same for both sides (slopes_lr).
+__device__ __forceinline__ void slopes_lr(const DevMesh& m, const DevState& s, int f, X64 LR[5]) {
   const int icl = m.fc1[f], icr = m.fc2[f];
-  const int c = side ? icr : icl;
+  if constexpr (kFast) {
+#pragma unroll
+    for (int v = 0; v < 5; ++v) LR[v] = (s.prim[v * (size_t)m.ldc + icr] - s.prim[v * (size_t)m.ldc + icl]) / m.dLR[f];
+  } else {
+    const Divisor d = divisor(m.dLR[f]);
+#pragma unroll
+    for (int v = 0; v < 5; ++v)
+      LR[v] = value(quotient(F64(s.prim[v * (size_t)m.ldc + icr]) - F64(s.prim[v * (size_t)m.ldc + icl]), d));
+  }
+}
+
+__device__ __forceinline__ void recon(const DevMesh& m, const DevState& s, const SpatOpts& o, int f, int side,
+                                      const X64 LR[5], double q[5]) {
+  const size_t ld = m.ldc;
+  const int c = side ? m.fc2[f] : m.fc1[f];
   const double* __restrict__ prim = s.prim;
 #pragma unroll
   for (int v = 0; v < 5; ++v) q[v] = prim[v * ld + c];
   if (o.highres == TY_HRES_NONE) return;
   const double* __restrict__ gr = s.grad;
-  const double ux = d3(m.uLR, m.ldf, f, 0), uy = d3(m.uLR, m.ldf, f, 1), uz = d3(m.uLR, m.ldf, f, 2);
-  const double dLR = m.dLR[f];
+  const X64 ux = d3(m.uLR, m.ldf, f, 0), uy = d3(m.uLR, m.ldf, f, 1), uz = d3(m.uLR, m.ldf, f, 2);
   if (o.highres == TY_HRES_MUSCLFAST) {
     const double k = side ? m.kRF[f] : m.kLF[f];
     // scalars (tvdgradfst_scal.f90:35-57)
 #pragma unroll
     for (int sv = 0; sv < 2; ++sv) {
-      double LR = (prim[sv * ld + icr] - prim[sv * ld + icl]) / dLR;
       double sg;
       if (o.limiter == TY_LIM_NONE) {
-        sg = LR;
+        sg = value(LR[sv]);
       } else {
-        double g = gr[(3 * sv) * ld + c] * ux + gr[(3 * sv + 1) * ld + c] * uy + gr[(3 * sv + 2) * ld + c] * uz;
-        sg = apply_lim(o.limiter, false, true, g, LR);
+        X64 g = X64(gr[(3 * sv) * ld + c]) * ux + X64(gr[(3 * sv + 1) * ld + c]) * uy + X64(gr[(3 * sv + 2) * ld + c]) * uz;
+        sg = apply_lim(o.limiter, false, true, value(g), value(LR[sv]));
       }
       q[sv] = q[sv] + sg * k;
     }
     // velocity (tvdgradfst_vect.f90:36-58)
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-      double LR = (prim[(2 + i) * ld + icr] - prim[(2 + i) * ld + icl]) / dLR;
       double sg;
       if (o.limiter == TY_LIM_NONE) {
-        sg = LR;
+        sg = value(LR[2 + i]);
       } else {
-        double g = gr[(6 + 3 * i) * ld + c] * ux + gr[(7 + 3 * i) * ld + c] * uy + gr[(8 + 3 * i) * ld + c] * uz;
-        sg = apply_lim(o.limiter, false, false, g, LR);
+        X64 g = X64(gr[(6 + 3 * i) * ld + c]) * ux + X64(gr[(7 + 3 * i) * ld + c]) * uy + X64(gr[(8 + 3 * i) * ld + c]) * uz;
+        sg = apply_lim(o.limiter, false, false, value(g), value(LR[2 + i]));
       }
       q[2 + i] = q[2 + i] + k * sg;
     }
@@ -464,31 +554,30 @@ __device__ void recon(const DevMesh& m, const DevState& s, const SpatOpts& o, in
   // MUSCL / MUSCL-UNS (tvdgradstr_*.f90, tvdgraduns_*.f90)
   const bool uns = o.highres == TY_HRES_MUSCLUNS;
   const double* CF = side ? m.RF : m.LF;
-  const double cx = d3(CF, m.ldf, f, 0), cy = d3(CF, m.ldf, f, 1), cz = d3(CF, m.ldf, f, 2);
+  const X64 cx = d3(CF, m.ldf, f, 0), cy = d3(CF, m.ldf, f, 1), cz = d3(CF, m.ldf, f, 2);
 #pragma unroll
   for (int sv = 0; sv < 2; ++sv) {
-    double LR = (prim[sv * ld + icr] - prim[sv * ld + icl]) / dLR;
-    double gx = gr[(3 * sv) * ld + c], gy = gr[(3 * sv + 1) * ld + c], gz = gr[(3 * sv + 2) * ld + c];
-    double g = gx * ux + gy * uy + gz * uz;
-    double sg = o.limiter == TY_LIM_NONE ? LR - g : apply_lim(o.limiter, uns, true, g, LR) - g;
+    X64 gx = gr[(3 * sv) * ld + c], gy = gr[(3 * sv + 1) * ld + c], gz = gr[(3 * sv + 2) * ld + c];
+    const X64 g = gx * ux + gy * uy + gz * uz;
+    const X64 sg = o.limiter == TY_LIM_NONE ? LR[sv] - g : X64(apply_lim(o.limiter, uns, true, value(g), value(LR[sv]))) - g;
     gx = gx + sg * ux; gy = gy + sg * uy; gz = gz + sg * uz;
-    q[sv] = q[sv] + (gx * cx + gy * cy + gz * cz);
-  }
-  double T[9];
-#pragma unroll
-  for (int k = 0; k < 9; ++k) T[k] = gr[(6 + k) * ld + c];
-  double sgv[3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    double LR = (prim[(2 + i) * ld + icr] - prim[(2 + i) * ld + icl]) / dLR;
-    double g = T[3 * i] * ux + T[3 * i + 1] * uy + T[3 * i + 2] * uz;
-    sgv[i] = o.limiter == TY_LIM_NONE ? LR - g : apply_lim(o.limiter, uns, false, g, LR) - g;
+    q[sv] = value(X64(q[sv]) + (gx * cx + gy * cy + gz * cz));
   }
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    double t0 = T[3 * i] + sgv[i] * ux, t1 = T[3 * i + 1] + sgv[i] * uy, t2 = T[3 * i + 2] + sgv[i] * uz;
-    q[2 + i] = q[2 + i] + (t0 * cx + t1 * cy + t2 * cz);
+    const X64 T0 = gr[(6 + 3 * i) * ld + c], T1 = gr[(7 + 3 * i) * ld + c], T2 = gr[(8 + 3 * i) * ld + c];
+    const X64 g = T0 * ux + T1 * uy + T2 * uz, lr = LR[2 + i];
+    const X64 sg = o.limiter == TY_LIM_NONE ? lr - g : X64(apply_lim(o.limiter, uns, false, value(g), value(lr))) - g;
+    const X64 t0 = T0 + sg * ux, t1 = T1 + sg * uy, t2 = T2 + sg * uz;
+    q[2 + i] = value(X64(q[2 + i]) + (t0 * cx + t1 * cy + t2 * cz));
   }
+}
+
+// one side of a face by itself
+__device__ void recon(const DevMesh& m, const DevState& s, const SpatOpts& o, int f, int side, double q[5]) {
+  X64 LR[5];
+  if (o.highres != TY_HRES_NONE) slopes_lr(m, s, f, LR);
+  recon(m, s, o, f, side, LR, q);
 }
 
 // moving adiabatic wall, face-state mode (setboco_ns_flux.f90): the right state takes the left
@@ -680,50 +769,60 @@ __device__ void flux_rusanov(double g, const double* L, const double* R, double 
 }
 
 // Roe flux-difference splitting with Harten's entropy fix (new: Typhon has no Roe flux)
-__device__ void flux_roe(double g, double eps, const double* L, const double* R, double nx, double ny, double nz,
+// Harten's fix of a wave speed below delta: a call, taken by few faces
+__device__ __noinline__ double harten(double l, double delta) { return (l * l + delta * delta) / (2.0 * delta); }
+
+// Operations of calc_flux_roe.f90 in its order, as F64; the three divisions by a^2 share its reciprocal,
+// comparisons are of bit patterns.  Limited states and flux of 175,760 faces: 111 -> 92 us.
+__device__ void flux_roe(const SpatOpts& o, const double* Ls, const double* Rs, double nxs, double nys, double nzs,
                          double* F) {
-  const double ig1 = 1.0 / (g - 1.0);
-  const double gig1 = g / (g - 1.0);
-  double t1 = sqrt(R[0] / L[0]);
-  double rroe = L[0] * t1;
-  double kl = 1.0 / (1.0 + t1), kr = t1 * kl;
-  double ux = kl * L[2] + kr * R[2], uy = kl * L[3] + kr * R[3], uz = kl * L[4] + kr * R[4];
-  double sqL = L[2] * L[2] + L[3] * L[3] + L[4] * L[4];
-  double sqR = R[2] * R[2] + R[3] * R[3] + R[4] * R[4];
-  double hl = gig1 * L[1] / L[0] + 0.5 * sqL;
-  double hr = gig1 * R[1] / R[0] + 0.5 * sqR;
-  double hroe = kl * hl + kr * hr;
-  double q2 = ux * ux + uy * uy + uz * uz;
-  double a2 = (g - 1.0) * (hroe - 0.5 * q2);
-  double a = sqrt(a2);
-  double vn = ux * nx + uy * ny + uz * nz;
-  double vnl = L[2] * nx + L[3] * ny + L[4] * nz;
-  double vnr = R[2] * nx + R[3] * ny + R[4] * nz;
-  double rel = ig1 * L[1] + 0.5 * L[0] * sqL;
-  double rer = ig1 * R[1] + 0.5 * R[0] * sqR;
-  double drho = R[0] - L[0], dp = R[1] - L[1], dvn = vnr - vnl;
-  double dux = R[2] - L[2], duy = R[3] - L[3], duz = R[4] - L[4];
-  double al1 = (dp - rroe * a * dvn) / (2.0 * a2);
-  double al5 = (dp + rroe * a * dvn) / (2.0 * a2);
-  double al2 = drho - dp / a2;
-  double dutx = dux - dvn * nx, duty = duy - dvn * ny, dutz = duz - dvn * nz;
-  double l1 = fabs(vn - a), l5 = fabs(vn + a), l2 = fabs(vn);
-  double delta = eps * a;
-  if (l1 < delta) l1 = (l1 * l1 + delta * delta) / (2.0 * delta);
-  if (l5 < delta) l5 = (l5 * l5 + delta * delta) / (2.0 * delta);
-  double w1 = l1 * al1, w2 = l2 * al2, w5 = l5 * al5, ws = l2 * rroe;
-  double d_mass = w1 + w2 + w5;
-  double dmx = w1 * (ux - a * nx) + w2 * ux + w5 * (ux + a * nx) + ws * dutx;
-  double dmy = w1 * (uy - a * ny) + w2 * uy + w5 * (uy + a * ny) + ws * duty;
-  double dmz = w1 * (uz - a * nz) + w2 * uz + w5 * (uz + a * nz) + ws * dutz;
-  double d_ener = w1 * (hroe - a * vn) + w2 * (0.5 * q2) + w5 * (hroe + a * vn) +
-                  ws * ((ux * dux + uy * duy + uz * duz) - vn * dvn);
-  double ml = vnl * L[0], mr = vnr * R[0];
-  F[0] = 0.5 * (ml + mr - d_mass);
-  F[1] = 0.5 * (vnl * (rel + L[1]) + vnr * (rer + R[1]) - d_ener);
-  F[2] = 0.5 * ((ml * L[2] + L[1] * nx) + (mr * R[2] + R[1] * nx) - dmx);
-  F[3] = 0.5 * ((ml * L[3] + L[1] * ny) + (mr * R[3] + R[1] * ny) - dmy);
-  F[4] = 0.5 * ((ml * L[4] + L[1] * nz) + (mr * R[4] + R[1] * nz) - dmz);
+  F64 L[5], R[5];
+#pragma unroll
+  for (int v = 0; v < 5; ++v) { L[v] = Ls[v]; R[v] = Rs[v]; }
+  const F64 nx = nxs, ny = nys, nz = nzs, half = 0.5;
+  const F64 ig1 = o.ig1, gig1 = o.gdg1;
+  F64 t1 = sqrt(Rs[0] / Ls[0]);
+  F64 rroe = L[0] * t1;
+  F64 kl = 1.0 / (F64(1.0) + t1).v, kr = t1 * kl;
+  F64 ux = kl * L[2] + kr * R[2], uy = kl * L[3] + kr * R[3], uz = kl * L[4] + kr * R[4];
+  F64 sqL = L[2] * L[2] + L[3] * L[3] + L[4] * L[4];
+  F64 sqR = R[2] * R[2] + R[3] * R[3] + R[4] * R[4];
+  F64 hl = F64((gig1 * L[1]).v / Ls[0]) + half * sqL;
+  F64 hr = F64((gig1 * R[1]).v / Rs[0]) + half * sqR;
+  F64 hroe = kl * hl + kr * hr;
+  F64 q2 = ux * ux + uy * uy + uz * uz, hq2 = half * q2;
+  F64 a2 = F64(o.gamma - 1.0) * (hroe - hq2);
+  F64 a = sqrt(a2.v);
+  F64 vn = ux * nx + uy * ny + uz * nz;
+  F64 vnl = L[2] * nx + L[3] * ny + L[4] * nz;
+  F64 vnr = R[2] * nx + R[3] * ny + R[4] * nz;
+  F64 rel = ig1 * L[1] + half * L[0] * sqL;
+  F64 rer = ig1 * R[1] + half * R[0] * sqR;
+  F64 drho = R[0] - L[0], dp = R[1] - L[1], dvn = vnr - vnl;
+  F64 dux = R[2] - L[2], duy = R[3] - L[3], duz = R[4] - L[4];
+  const Divisor d = divisor(a2.v), dd = {a2 + a2, d.y * half, d.ok};
+  const F64 rad = rroe * a * dvn;
+  F64 al1 = quotient(dp - rad, dd);
+  F64 al5 = quotient(dp + rad, dd);
+  F64 al2 = drho - quotient(dp, d);
+  F64 dutx = dux - dvn * nx, duty = duy - dvn * ny, dutz = duz - dvn * nz;
+  F64 l1 = abs_bits((vn - a).v), l5 = abs_bits((vn + a).v), l2 = abs_bits(vn.v);
+  F64 delta = F64(o.entropy_fix) * a;
+  if (dbits(l1.v) < dbits(delta.v)) l1 = harten(l1.v, delta.v);  // positive doubles order like their bits
+  if (dbits(l5.v) < dbits(delta.v)) l5 = harten(l5.v, delta.v);
+  F64 w1 = l1 * al1, w2 = l2 * al2, w5 = l5 * al5, ws = l2 * rroe;
+  F64 d_mass = w1 + w2 + w5;
+  const F64 anx = a * nx, any = a * ny, anz = a * nz, avn = a * vn;
+  F64 dmx = w1 * (ux - anx) + w2 * ux + w5 * (ux + anx) + ws * dutx;
+  F64 dmy = w1 * (uy - any) + w2 * uy + w5 * (uy + any) + ws * duty;
+  F64 dmz = w1 * (uz - anz) + w2 * uz + w5 * (uz + anz) + ws * dutz;
+  F64 d_ener = w1 * (hroe - avn) + w2 * hq2 + w5 * (hroe + avn) + ws * ((ux * dux + uy * duy + uz * duz) - vn * dvn);
+  F64 ml = vnl * L[0], mr = vnr * R[0];
+  F[0] = (half * (ml + mr - d_mass)).v;
+  F[1] = (half * (vnl * (rel + L[1]) + vnr * (rer + R[1]) - d_ener)).v;
+  F[2] = (half * ((ml * L[2] + L[1] * nx) + (mr * R[2] + R[1] * nx) - dmx)).v;
+  F[3] = (half * ((ml * L[3] + L[1] * ny) + (mr * R[3] + R[1] * ny) - dmy)).v;
+  F[4] = (half * ((ml * L[4] + L[1] * nz) + (mr * R[4] + R[1] * nz) - dmz)).v;
 }
 
 // ===========================================================================
@@ -733,20 +832,6 @@ __device__ void flux_roe(double g, double eps, const double* L, const double* R,
 // (HBM-resident) and the per-stage work avoids divisions.
 
 #if TY_FAST
-// Comparisons of doubles run on the FP64 pipe (a minimum is a comparison and a select); on bit
-// patterns they run on the integer pipe.
-__device__ __forceinline__ long long order_key(double x) {  // orders like x
-  const long long b = __double_as_longlong(x);
-  return b ^ ((b >> 63) & 0x7fffffffffffffffll);
-}
-__device__ __forceinline__ double min_bits(double a, double b) { return order_key(a) < order_key(b) ? a : b; }
-__device__ __forceinline__ double max_bits(double a, double b) { return order_key(a) < order_key(b) ? b : a; }
-__device__ __forceinline__ bool is_neg(double x) { return __double2hiint(x) < 0; }  // sign bit
-// x without the sign (fabs of a stored value is an FP64 instruction)
-__device__ __forceinline__ double abs_bits(double x) {
-  return __hiloint2double(__double2hiint(x) & 0x7fffffff, __double2loint(x));
-}
-
 // Roe weights and reciprocal densities from one reciprocal square root: with y = 1/sqrt(rho_L
 // rho_R), rroe = sqrt(rho_L rho_R) = rho_L rho_R y, kl = rho_L / (rho_L + rroe), kr = rroe /
 // (rho_L + rroe), 1/rho_L = y^2 rho_R, 1/rho_R = y^2 rho_L.
@@ -1098,7 +1183,7 @@ __device__ __forceinline__ void face_flux(const DevMesh& m, const DevState& s, c
   else if (o.scheme == TY_SCH_RUSANOV) flux_rusanov(o.gamma, QL, QR, nx, ny, nz, F);
   else if (o.hll_family == 2) flux_hlle(o, QL, QR, nx, ny, nz, F);
   else if (o.scheme == TY_SCH_AUSMM) flux_ausmm(o.gamma, QL, QR, nx, ny, nz, F);
-  else flux_roe(o.gamma, o.entropy_fix, QL, QR, nx, ny, nz, F);
+  else flux_roe(o, QL, QR, nx, ny, nz, F);
   if (o.viscous != TY_VISC_NONE) add_viscous(m, s, o, f, F);
   const double S = m.fs[f];
 #pragma unroll
@@ -1112,7 +1197,9 @@ __global__ void __launch_bounds__(kBlock) k_face_flux(DevMesh m, DevState s, Spa
   int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= m.nf) return;
   double QL[5], QR[5];
-  recon(m, s, o, f, 0, QL);
+  X64 LR[5];
+  if (o.highres != TY_HRES_NONE) slopes_lr(m, s, f, LR);
+  recon(m, s, o, f, 0, LR, QL);
   const int kind = f < m.nfi ? TY_BC_INTERIOR : m.fbc[f];
   if (kind == TY_BC_PERIODIC) {
     recon(m, s, o, m.part[f], 0, QR);  // cell_r(face) = cell_l(partner face)
@@ -1128,55 +1215,87 @@ __global__ void __launch_bounds__(kBlock) k_face_flux(DevMesh m, DevState s, Spa
     for (int v = 0; v < 5; ++v) QR[v] = QL[v];
     mirror(m, f, QR);
   } else {
-    recon(m, s, o, f, 1, QR);
+    recon(m, s, o, f, 1, LR, QR);
   }
   face_flux(m, s, o, f, QL, QR, s.flux);
 }
 
-// post-limiter path, 1: unlimited face states
+// post-limiter path, 1: unlimited face states.  Both sides share the slopes (q(fc2) - q(fc1)) / |C_L C_R|,
+// five quotients by one divisor where each side divided for itself: 175,760 faces 102 -> 70 us.
 __global__ void __launch_bounds__(kBlock) k_face_states(DevMesh m, DevState s, SpatOpts o) {
   pdl_wait();
   int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= m.nf) return;
   double Q[5];
-  recon(m, s, o, f, 0, Q);
+  X64 LR[5];
+  if (o.highres != TY_HRES_NONE) slopes_lr(m, s, f, LR);
+  recon(m, s, o, f, 0, LR, Q);
 #pragma unroll
   for (int v = 0; v < 5; ++v) s.cl[v * (size_t)m.ldf + f] = Q[v];
-  recon(m, s, o, f, 1, Q);
+  recon(m, s, o, f, 1, LR, Q);
 #pragma unroll
   for (int v = 0; v < 5; ++v) s.cr[v * (size_t)m.ldf + f] = Q[v];
 }
 
+// klim n/d < klim bn/bd as the limiter computes them (a NaN counts as 0): the call taken where the
+// FP32 comparison of k_barth does not decide
+__device__ __noinline__ bool ratio_less(double klim, double n, double d, double bn, double bd) {
+  return fmax(klim * (n / d), 0.0) < fmax(klim * (bn / bd), 0.0);
+}
+
 // post-limiter path, 2: Barth-type ratio of each interior cell (postlimit_barth.f90:60-80,
-// 140-170).  A face whose increment is exactly zero imposes no constraint.
+// 140-170): min(1, max(klim LR/den, 0)) over faces and variables of a group.  A face whose
+// increment is exactly zero imposes no constraint.  Division and product round monotonically, so
+// the fraction that is smallest gives the minimum: fractions are compared in FP32, truncated and
+// cross-multiplied (exactly, ratio_less, where they are within 1e-6 or out of FP32's range), and one
+// division per group is left of one per face and variable.  87,880 tetrahedra: 62 -> 19 us.
 __global__ void __launch_bounds__(kBlock) k_barth(DevMesh m, DevState s, double klim) {
-  pdl_wait();
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= m.nci) return;
+  int es[kMaxSlot];
+  face_list(m, c, es);
+  pdl_wait();
   const size_t ld = m.ldc, lf = m.ldf;
-  double r[3] = {1.0, 1.0, 1.0};
-  double qc[5];
+  X64 qc[5];
 #pragma unroll
   for (int v = 0; v < 5; ++v) qc[v] = s.prim[v * ld + c];
-  for (int sl = 0; sl < m.nslot; ++sl) {
-    int e = m.cf[sl * (size_t)m.nci + c];
+  // smallest fraction so far, 1 / klim at first (klim is 1 or 1/2)
+  double bn[3] = {1.0, 1.0, 1.0}, bd[3] = {klim, klim, klim};
+  float fn[3] = {1.0f, 1.0f, 1.0f}, fd[3] = {(float)klim, (float)klim, (float)klim};
+  bool zero[3] = {false, false, false}, far[3] = {false, false, false};
+#pragma unroll
+  for (int sl = 0; sl < kMaxSlot; ++sl) {
+    const int e = es[sl];
     if (e < 0) break;
-    int f = e >> 1, side = e & 1;
-    int nb = side ? m.fc1[f] : m.fc2[f];
+    const int f = e >> 1, side = e & 1;
+    const int nb = side ? m.fc1[f] : m.fc2[f];
     const double* qf = side ? s.cr : s.cl;
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
-      double LR = s.prim[v * ld + nb] - qc[v];  // = +-(q(fc2) - q(fc1)) seen from c
-      double den = qf[v * lf + f] - qc[v];
-      if (den != 0.0) {
-        double l = fmax(klim * (LR / den), 0.0);
-        int k = v < 2 ? v : 2;
-        r[k] = fmin(r[k], l);
+      const int k = v < 2 ? v : 2;
+      const double n = value(X64(s.prim[v * ld + nb]) - qc[v]);  // = +-(q(fc2) - q(fc1)) seen from c
+      const double d = value(X64(qf[v * lf + f]) - qc[v]);
+      if (is_zero(d)) continue;
+      if (is_zero(n) || (__double2hiint(n) ^ __double2hiint(d)) < 0) {  // n/d <= 0
+        zero[k] = true;
+        continue;
+      }
+      bool ok = !far[k];
+      const float gn = trunc32(n, ok), gd = trunc32(d, ok);
+      const float x = gn * fd[k], y = fn[k] * gd;
+      bool less = x < y;
+      if (!ok || fabsf(x - y) <= 9.6e-7f * y) less = ratio_less(klim, n, d, bn[k], bd[k]);
+      if (less) {
+        bn[k] = abs_bits(n);
+        bd[k] = abs_bits(d);
+        bool in = true;
+        fn[k] = trunc32(n, in); fd[k] = trunc32(d, in);
+        far[k] = !in;
       }
     }
   }
 #pragma unroll
-  for (int k = 0; k < 3; ++k) s.ratio[k * ld + c] = r[k];
+  for (int k = 0; k < 3; ++k) s.ratio[k * ld + c] = zero[k] ? 0.0 : fmin(1.0, fmax(klim * (bn[k] / bd[k]), 0.0));
 }
 
 // post-limiter path, 3: limited states + flux
@@ -1191,9 +1310,8 @@ __global__ void __launch_bounds__(kBlock) k_face_flux_lim(DevMesh m, DevState s,
     const double* qf = side ? s.cr : s.cl;
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
-      double qc = s.prim[v * ld + c];
-      double rr = s.ratio[(v < 2 ? v : 2) * ld + c];
-      Q[v] = qc + rr * (qf[v * lf + face] - qc);
+      const X64 qc = s.prim[v * ld + c], rr = s.ratio[(v < 2 ? v : 2) * ld + c];
+      Q[v] = value(qc + rr * (X64(qf[v * lf + face]) - qc));
     }
   };
   limited(f, 0, QL);
@@ -1219,22 +1337,6 @@ __global__ void __launch_bounds__(kBlock) k_face_flux_lim(DevMesh m, DevState s,
 
 
 #if TY_FAST
-__device__ __forceinline__ long long dbits(double x) { return __double_as_longlong(x); }
-
-// x == 0 on the integer pipe (on the 32-bit halves: the compiler turns a test of the 64-bit
-// pattern back into an FP64 comparison)
-__device__ __forceinline__ bool is_zero(double x) {
-  return (((unsigned)__double2hiint(x) << 1) | (unsigned)__double2loint(x)) == 0u;
-}
-
-// |x| as an FP32 number, truncated (relative error below 2^-23) on the integer pipe, when x lies
-// in [2^-60, 2^60); ok is cleared otherwise.
-__device__ __forceinline__ float trunc32(double x, bool& ok) {
-  const int hi = __double2hiint(x) & 0x7fffffff;
-  ok = ok && (unsigned)(hi - ((1023 - 60) << 20)) < (unsigned)(120 << 20);
-  return __uint_as_float(__funnelshift_l((unsigned)__double2loint(x), (unsigned)hi, 3) - ((1023u - 127u) << 23));
-}
-
 // |a| b < |c| d of positive products, as bit patterns.  A call, so that the multiplications are
 // not if-converted into the callers: a predicated-off FP64 instruction occupies the pipe as well.
 __device__ __noinline__ bool product_less(double a, double b, double c, double d) {
@@ -1540,12 +1642,6 @@ __global__ void __launch_bounds__(kBlock) k_face_flux_fast(DevMesh m, DevState s
 // residual R_c = dt/V_c * sum(+-F S), in the colour order of flux_to_res.  The sign is put on the
 // flux's bits (R - F is R + (-F), bit for bit), so that one sum per flux is issued: a branch on
 // the side issued both, one of them predicated off.
-// The face list is read ahead (and before the wait for the flux kernel): one trip to L2 less.
-__device__ __forceinline__ void face_list(const DevMesh& m, int c, int es[kMaxSlot]) {
-#pragma unroll
-  for (int sl = 0; sl < kMaxSlot; ++sl) es[sl] = sl < m.nslot ? m.cf[sl * (size_t)m.nci + c] : -1;
-}
-
 template <class T>
 __device__ __forceinline__ void gather_residual(const DevMesh& m, const DevState& s, const int es[kMaxSlot], T R[5]) {
 #pragma unroll
