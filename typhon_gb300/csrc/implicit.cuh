@@ -23,12 +23,22 @@
 namespace tyk {
 namespace TY_KNS {
 
+// quotient and root of the Jacobians: IEEE in exact mode, Newton-Raphson (fastmath.cuh) in fast mode
+__device__ __forceinline__ double jac_div(double a, double b) {
+  if constexpr (kFast) return a * rcp_nr(b);
+  return a / b;
+}
+__device__ __forceinline__ double jac_sqrt(double a) {
+  if constexpr (kFast) return sqrt_nr(a);
+  return sqrt(a);
+}
+
 // Jacobian of the physical flux along n, row-major (calc_jacflux.f90:49-77); q = (rho, p, u)
-__device__ void jacflux(double g, const double* q, double nx, double ny, double nz, double vn, double* J) {
-  const double g1 = g - 1.0, ig1 = 1.0 / g1;
+__device__ void jacflux(double g, double ig1, const double* q, double nx, double ny, double nz, double vn, double* J) {
+  const double g1 = g - 1.0;
   const double u[3] = {q[2], q[3], q[4]}, t[3] = {nx, ny, nz};
   const double v2 = u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
-  const double en = ig1 * q[1] / q[0] + .5 * v2;
+  const double en = jac_div(ig1 * q[1], q[0]) + .5 * v2;
   J[0] = 0.0; J[1] = 0.0; J[2] = t[0]; J[3] = t[1]; J[4] = t[2];
   J[5] = vn * (g1 * v2 - g * en);
   J[6] = vn * g;
@@ -56,9 +66,9 @@ __device__ void face_jacobians(const SpatOpts& o, const double* L, const double*
   const double g = o.gamma;
   const double vnl = L[2] * nx + L[3] * ny + L[4] * nz;
   const double vnr = R[2] * nx + R[3] * ny + R[4] * nz;
-  const double al = sqrt(g * L[1] / L[0]), ar = sqrt(g * R[1] / R[0]);
-  jacflux(g, L, nx, ny, nz, vnl, JL);
-  jacflux(g, R, nx, ny, nz, vnr, JR);
+  const double al = jac_sqrt(jac_div(g * L[1], L[0])), ar = jac_sqrt(jac_div(g * R[1], R[0]));
+  jacflux(g, o.ig1, L, nx, ny, nz, vnl, JL);
+  jacflux(g, o.ig1, R, nx, ny, nz, vnr, JR);
   if (o.scheme == TY_SCH_RUSANOV) {  // calc_jac_rusanov.f90: (A_L + ray I)/2, (A_R - ray I)/2
     const double ray = fmax(fabs(vnl) + al, fabs(vnr) + ar);
 #pragma unroll
@@ -69,39 +79,39 @@ __device__ void face_jacobians(const SpatOpts& o, const double* L, const double*
   }
   double sl, sr;
   if (o.hll_family != 0) {  // the HLLC / HLLE family's wave speeds (calc_flux_hllc.f90:86-124, calc_flux_hlle.f90:83-120)
-    const double gig1 = g / (g - 1.0);
-    double t1 = sqrt(R[0] / L[0]);
+    const double gig1 = o.gdg1;
+    double t1 = jac_sqrt(jac_div(R[0], L[0]));
     double roe_rho = L[0] * t1;
-    double kl = 1.0 / (1.0 + t1);
+    double kl = jac_div(1.0, 1.0 + t1);
     double kr = t1 * kl;
     double rux = kl * L[2] + kr * R[2], ruy = kl * L[3] + kr * R[3], ruz = kl * L[4] + kr * R[4];
     double sqL = L[2] * L[2] + L[3] * L[3] + L[4] * L[4];
     double sqR = R[2] * R[2] + R[3] * R[3] + R[4] * R[4];
-    double h1 = gig1 * L[1] / L[0] + 0.5 * sqL;
-    double h2 = gig1 * R[1] / R[0] + 0.5 * sqR;
+    double h1 = jac_div(gig1 * L[1], L[0]) + 0.5 * sqL;
+    double h2 = jac_div(gig1 * R[1], R[0]) + 0.5 * sqR;
     h1 = kl * h1 + kr * h2;
-    double roe_p = (h1 - 0.5 * (rux * rux + ruy * ruy + ruz * ruz)) * roe_rho / gig1;
+    double roe_p = jac_div((h1 - 0.5 * (rux * rux + ruy * ruy + ruz * ruz)) * roe_rho, gig1);
     double vm = rux * nx + ruy * ny + ruz * nz;
-    double am = sqrt(g * roe_p / roe_rho);
+    double am = jac_sqrt(jac_div(g * roe_p, roe_rho));
     hll_speeds(o, vnl, vnr, al, ar, vm, am, sl, sr);
     if (o.hll_family == 1) {  // calc_flux_hllc.f90 passes min(sl, 0), max(sr, 0) to calc_jac_hll
       sl = fmin(sl, 0.0);
       sr = fmax(sr, 0.0);
     }
   } else {  // Roe flux: HLL Jacobian with Einfeldt's speeds from the Roe average (new)
-    double t1 = sqrt(R[0] / L[0]);
-    double kl = 1.0 / (1.0 + t1), kr = t1 * kl;
+    double t1 = jac_sqrt(jac_div(R[0], L[0]));
+    double kl = jac_div(1.0, 1.0 + t1), kr = t1 * kl;
     double ux = kl * L[2] + kr * R[2], uy = kl * L[3] + kr * R[3], uz = kl * L[4] + kr * R[4];
-    double hl = g / (g - 1.0) * L[1] / L[0] + 0.5 * (L[2] * L[2] + L[3] * L[3] + L[4] * L[4]);
-    double hr = g / (g - 1.0) * R[1] / R[0] + 0.5 * (R[2] * R[2] + R[3] * R[3] + R[4] * R[4]);
-    double am = sqrt((g - 1.0) * (kl * hl + kr * hr - 0.5 * (ux * ux + uy * uy + uz * uz)));
+    double hl = jac_div(o.gdg1 * L[1], L[0]) + 0.5 * (L[2] * L[2] + L[3] * L[3] + L[4] * L[4]);
+    double hr = jac_div(o.gdg1 * R[1], R[0]) + 0.5 * (R[2] * R[2] + R[3] * R[3] + R[4] * R[4]);
+    double am = jac_sqrt((g - 1.0) * (kl * hl + kr * hr - 0.5 * (ux * ux + uy * uy + uz * uz)));
     double vm = ux * nx + uy * ny + uz * nz;
     sl = fmin(fmin(vnl - al, vm - am), 0.0);
     sr = fmax(fmax(vnr + ar, vm + am), 0.0);
   }
 #pragma unroll
   for (int i = 0; i < 5; ++i) { JL[i * 6] = JL[i * 6] - sl; JR[i * 6] = JR[i * 6] - sr; }
-  const double cl = sr / (sr - sl), cr = -sl / (sr - sl);
+  const double cl = jac_div(sr, sr - sl), cr = jac_div(-sl, sr - sl);
 #pragma unroll
   for (int k = 0; k < 25; ++k) { JL[k] = cl * JL[k]; JR[k] = cr * JR[k]; }
 }
@@ -171,13 +181,24 @@ __device__ void implicit_face_states(const DevMesh& m, const DevState& s, const 
   }
 }
 
-// J dt / V of build_implicit_bdlu.f90:51-55: two roundings per entry in exact mode, a product
-// with the per-cell quotient q = dt / V in fast mode
-#if TY_FAST
-#define TY_DTV(J, dt, V, q) ((J) * (q))
-#else
-#define TY_DTV(J, dt, V, q) ((J) * (dt) / (V))
-#endif
+// J dt / V of build_implicit_bdlu.f90:51-55: two roundings per entry in exact mode (the 25
+// quotients by V through its reciprocal), a product with the per-cell quotient dt / V in fast mode
+__device__ __forceinline__ void scaled_block(const double* J, double dt, double V, double* U) {
+  if constexpr (kFast) {
+    const double q = dt / V;
+#pragma unroll
+    for (int k = 0; k < 25; ++k) U[k] = J[k] * q;
+  } else {
+    const Divisor d = divisor(V);
+    bool bad = false;
+#pragma unroll
+    for (int k = 0; k < 25; ++k) U[k] = value(quotient(F64(J[k]) * F64(dt), d, bad));
+    if (bad) {
+#pragma unroll
+      for (int k = 0; k < 25; ++k) U[k] = div_ieee(J[k] * dt, V);
+    }
+  }
+}
 
 __device__ __forceinline__ double imp_dt(const ImpState& im, const ImpArgs& a, int c) {
   return a.local_dt ? im.dtloc[c] : __longlong_as_double((long long)*a.dtg);
@@ -265,11 +286,11 @@ __global__ void __launch_bounds__(128) k_imp_face(DevMesh m, DevState s, SpatOpt
     const double dHL = m.vgeo[f], dHR = m.vgeo[lf + f];
     const double wx = m.vgeo[2 * lf + f], wy = m.vgeo[3 * lf + f], wz = m.vgeo[4 * lf + f];
     const double rL = s.prim[icl], rR = s.prim[icr], pL = s.prim[ld + icl], pR = s.prim[ld + icr];
-    const double TL = pL / (rL * r), TR = pR / (rR * r);
+    const double TL = jac_div(pL, rL * r), TR = jac_div(pR, rR * r);
     const double TH = dHR * TL + dHL * TR;
     const double rhoH = dHR * rL + dHL * rR;
     const double mu = viscosity(o, rhoH, TH);
-    const double id = mu / (dHR * rL + dHL * rR) / sqrt(wx * wx + wy * wy + wz * wz);
+    const double id = jac_div(jac_div(mu, dHR * rL + dHL * rR), jac_sqrt(wx * wx + wy * wy + wz * wz));
 #pragma unroll
     for (int i = 0; i < 5; ++i) {
       JR[i * 6] = JR[i * 6] - id;
@@ -335,17 +356,11 @@ __global__ void __launch_bounds__(128) k_imp_face(DevMesh m, DevState s, SpatOpt
   if (f < m.nfi) {
     const int c1 = m.fc1[f], c2 = m.fc2[f];
     const double dt1 = imp_dt(im, a, c1), dt2 = imp_dt(im, a, c2);
-    const double V1 = m.cvol[c1], V2 = m.cvol[c2];
     double U[25];
-#if TY_FAST
-    const double q1 = dt1 / V1, q2 = dt2 / V2;
-#endif
-#pragma unroll
-    for (int k = 0; k < 25; ++k) U[k] = +TY_DTV(JR[k], dt1, V1, q1);
+    scaled_block(JR, dt1, m.cvol[c1], U);
     if (a.want64) store_block(im.upper + (size_t)f * kBlk, U);
     if (a.want32) store_block32(im.upper32 + (size_t)f * kBlk32, U);
-#pragma unroll
-    for (int k = 0; k < 25; ++k) U[k] = -TY_DTV(JL[k], dt2, V2, q2);
+    scaled_block(JL, -dt2, m.cvol[c2], U);
     if (a.want64) store_block(im.lower + (size_t)f * kBlk, U);
     if (a.want32) store_block32(im.lower32 + (size_t)f * kBlk32, U);
   }
@@ -407,23 +422,16 @@ __global__ void __launch_bounds__(128) k_imp_diag(DevMesh m, ImpState im, ImpArg
 #pragma unroll
   for (int i = 0; i < 5; ++i) D[i * 6] = 1.0;
   const double dt = imp_dt(im, a, c), V = m.cvol[c];
-#if TY_FAST
-  const double q = dt / V;  // one division per cell; exact mode keeps Typhon's (J dt) / V per entry
-#endif
   for (int sl = 0; sl < m.nslot; ++sl) {
     const int e = im.cfo[sl * (size_t)m.nci + c];
     if (e < 0) break;
     const int f = e >> 1;
     double J[25];
-    if (e & 1) {
-      load_block(im.jacR + (size_t)f * kBlk, J);
+    load_block(((e & 1) ? im.jacR : im.jacL) + (size_t)f * kBlk, J);
+    double U[25];
+    scaled_block(J, (e & 1) ? -dt : dt, V, U);
 #pragma unroll
-      for (int k = 0; k < 25; ++k) D[k] = D[k] - TY_DTV(J[k], dt, V, q);
-    } else {
-      load_block(im.jacL + (size_t)f * kBlk, J);
-#pragma unroll
-      for (int k = 0; k < 25; ++k) D[k] = D[k] + TY_DTV(J[k], dt, V, q);
-    }
+    for (int k = 0; k < 25; ++k) D[k] = value(X64(D[k]) + X64(U[k]));
   }
   if (a.want64) store_block(im.diag + (size_t)c * kBlk, D);
   if (a.want32) store_block32(im.diag32 + (size_t)c * kBlk32, D);
@@ -613,13 +621,13 @@ __global__ void __launch_bounds__(5 * kRowCells) k_imp_matvec_row(DevMesh m, Imp
   if (c >= m.nci) return;
   const size_t n = m.nci;
   int e = m.nslot > 0 ? im.cfo[c] : -1, nb = e >= 0 ? im.cfon[c] : 0;
-  double acc = z ? z[5 * (size_t)c + i] : 0.0;
+  X64 acc = z ? z[5 * (size_t)c + i] : 0.0;
   // the row's product with a block is added (y = A x) or subtracted
   auto row = [&](const double* __restrict__ A, const double* __restrict__ v, bool first) {
-    double a[5], q[5];
+    X64 a[5], q[5];
 #pragma unroll
     for (int j = 0; j < 5; ++j) { a[j] = __ldg(A + 5 * i + j); q[j] = v[j]; }
-    double s = 0.0;
+    X64 s = 0.0;
 #pragma unroll
     for (int j = 0; j < 5; ++j) s = s + a[j] * q[j];
     acc = z ? acc - s : (first ? s : acc + s);
@@ -636,7 +644,7 @@ __global__ void __launch_bounds__(5 * kRowCells) k_imp_matvec_row(DevMesh m, Imp
     row(A, v, false);
   }
   // S A x (the row scale is all ones outside the flexible GMRES)
-  y[5 * (size_t)c + i] = z ? acc : acc * im.rs[i];
+  y[5 * (size_t)c + i] = value(z ? acc : acc * X64(im.rs[i]));
 }
 
 // z = D^-1 S^-1 v, the block-Jacobi preconditioner of the flexible GMRES on its row-scaled

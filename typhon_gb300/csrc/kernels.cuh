@@ -183,6 +183,10 @@ __global__ void k_prim(DevMesh m, const double* __restrict__ cons, double* __res
 __device__ __forceinline__ double viscosity(const SpatOpts& o, double rho, double T) {
   if (o.visc_law == TY_VISC_KINEMATIC) return o.visc_kin * rho;
   const double mu0 = 0.0000168, T0 = 273.00, S = 110.50;
+  if constexpr (kFast) {
+    const double x = T * (1.0 / T0);
+    return mu0 * (T0 + S) * (x * sqrt_nr(x)) * rcp_nr(T + S);
+  }
   return mu0 * pow(T / T0, 1.5) * (T0 + S) / (T + S);
 }
 
@@ -503,8 +507,9 @@ __global__ void k_ghost_grad(DevMesh m, double* __restrict__ grad) {
 __device__ __forceinline__ void slopes_lr(const DevMesh& m, const DevState& s, int f, X64 LR[5]) {
   const int icl = m.fc1[f], icr = m.fc2[f];
   if constexpr (kFast) {
+    const double id = rcp_nr(m.dLR[f]);
 #pragma unroll
-    for (int v = 0; v < 5; ++v) LR[v] = (s.prim[v * (size_t)m.ldc + icr] - s.prim[v * (size_t)m.ldc + icl]) / m.dLR[f];
+    for (int v = 0; v < 5; ++v) LR[v] = (s.prim[v * (size_t)m.ldc + icr] - s.prim[v * (size_t)m.ldc + icl]) * id;
   } else {
     const Divisor d = divisor(m.dLR[f]);
 #pragma unroll
