@@ -512,8 +512,10 @@ __device__ __forceinline__ void fetch_blocks(const void* mine, char* stage) {
 // ascending order.  Boundary faces multiply the (zero) ghost unknowns and are skipped.
 // F32: y = S A x with FP32 blocks and FP32 x, FP32 accumulation, FP64 result.  The FP64 fast mode
 // accumulates every product into the row's sum (25 multiply-adds a block instead of 30 operations).
-// GB300, us per product, own loads -> staged: 250,000 cells FP32 40.5 -> 35.6, 320,000 FP64
-// (fast) 108 -> 90.
+// A slot's list entries are read one list ahead of its fetch.  GB300, us per product, own loads ->
+// staged -> entries ahead: 250,000 cells FP32 40.5 -> 35.6 -> 32.4, 320,000 FP64 (fast) 108 -> 90 -> 79
+// (the floors: 23 us of HBM traffic, 28 with the 64-byte granules that 112-byte blocks touch; 65 us of
+// FP64 multiply-adds).
 constexpr int kMvThreads = 128;
 template <bool F32>
 __global__ void __launch_bounds__(kMvThreads) k_imp_matvec(DevMesh m, ImpState im, const void* __restrict__ xp,
@@ -534,11 +536,16 @@ __global__ void __launch_bounds__(kMvThreads) k_imp_matvec(DevMesh m, ImpState i
   const T* A = nullptr;
   int nb = c;
   bool more = on;
+  int ne = m.nslot > 0 ? im.cfo[c] : -1, nn = m.nslot > 0 ? im.cfon[c] : c;  // the next slot's, one list ahead
   auto entry = [&](int sl) {
-    const int e = more && sl < m.nslot ? im.cfo[sl * n + c] : -1;
+    const int e = more && sl < m.nslot ? ne : -1;
     more = e >= 0 && (e >> 1) < m.nfi;
     A = more ? ((e & 1) ? lo : up) + (size_t)(e >> 1) * kStride : nullptr;
-    nb = more ? im.cfon[sl * n + c] : c;
+    nb = more ? nn : c;
+    if (sl + 1 < m.nslot) {
+      ne = im.cfo[(sl + 1) * n + c];
+      nn = im.cfon[(sl + 1) * n + c];
+    }
   };
   fetch_blocks<PIECES>(on ? dg + (size_t)c * kStride : nullptr, mine);
   T xv[5], yv[5];
@@ -1297,7 +1304,7 @@ void mv_staged(const DevMesh& m, const ImpState& im, const void* x, const double
 
 // A row per thread up to 40,000 cells, a cell per thread above, where the row form's narrower
 // loads cost more than its shorter chains gain.  GB300, us per product, cell / row form: 24,565
-// tetrahedra (exact) 24 / 19, 320,000 (fast) 90 (108 before its blocks were staged) / 153.
+// tetrahedra (exact) 24 / 17, 320,000 (fast) 79 (108 before its blocks were staged) / 153.
 constexpr int kRowFormCells = 40000;
 inline void matvec_launch(const DevMesh& m, const ImpState& im, const double* x, const double* z, double* y,
                           cudaStream_t st) {
