@@ -232,16 +232,16 @@ def kernel_bytes(md, nslot_avg, mtab=False):
         "barth": cf + nf * (8 + 80) + nc * 40 + nci * 24,    # list, fc, cl/cr, prim, write ratio
         "face_flux_lim": nf * (8 + 4 + 4 + 80 + 24 + 8 + 40) + nc * (40 + 24),
         "face_flux": nf * (8 + 4 + 4 + 24 + 8 + 40 + 64) + nc * (40 + 120),
-        "rk_update": cf + nf * 40 + nci * (8 + 40 + 40 + 40 + 40 + 40 + 40),  # vol, flux, u0, acc r/w, cur, prim
+        "rk_update": cf + nf * 40 + nci * (8 + 40 + 40 + 40 + 40),  # vol, flux, u0, acc r/w, prim
         "gather": cf + nf * 40 + nci * (8 + 40),
         "timestep": nci * (8 + 8 + 40),
         "prim": nci * 80,
         # fused fast-mode kernels
-        # lists, A^-1 d, reconstruction weights, write cl/cr; prim; write grad + ratio; or, with the
-        # per-cell increment matrices (MUSCL/-UNS without limiter), lists, the matrix (nslot^2 per
-        # cell), write cl/cr; prim; write ratio
+        # lists, 11 weights a slot, write cl/cr; prim; write grad + ratio; or, with the per-cell
+        # increment matrices (MUSCL/-UNS without limiter), lists, the matrix (nslot^2 per cell),
+        # write cl/cr; prim; write ratio
         "cell_fast": (8 * nslot_avg * nci + 8 * nslot_avg ** 2 * nci + nf * 80 + nc * 40 + nci * 24) if mtab else
-                     (8 * nslot_avg * nci + nf * (48 + 64 + 80) + nc * 40 + nci * (120 + 24)),
+                     (8 * nslot_avg * nci + 88 * nslot_avg * nci + nf * 80 + nc * 40 + nci * (120 + 24)),
         "face_flux_fast": nf * (80 + 8 + 24 + 8 + 40),     # cl/cr, bc/partner, normal, surface, write flux
     }
 

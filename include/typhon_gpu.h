@@ -369,8 +369,8 @@ int ty_kdif_get_temperature(ty_mesh* mesh, double* T);         /* host [ncell_in
 int ty_kdif_residual(ty_mesh* mesh, double dt, double* R);
 typedef enum {
   TY_KSOLVE_CG = 0,          /* conjugate gradients + Jacobi, FP64 (new: Typhon has CGS/BiCG/GMRES):
-                                Chronopoulos-Gear single-reduction form, two launches per
-                                iteration, no host round trip between checks */
+                                Chronopoulos-Gear single-reduction form, up to 1,000
+                                iterations in one cooperative launch */
   TY_KSOLVE_CG32_REFINE = 1, /* FP32 conjugate gradients inside FP64 iterative refinement */
   TY_KSOLVE_CG_MIXED = 2     /* TY_KSOLVE_CG on the face conductances stored in FP32 (FP64
                                 vectors and arithmetic; the difference form keeps the matrix

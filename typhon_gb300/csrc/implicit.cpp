@@ -93,7 +93,7 @@ int build_lists(ty_mesh* h) {
       (rc = h->alloc(im.dtloc, (size_t)nci)) || (rc = h->alloc(im.jacL, (size_t)m.nf * kBlk)) ||
       (rc = h->alloc(im.jacR, (size_t)m.nf * kBlk)) || (rc = h->alloc(im.b, 5 * (size_t)nci)) ||
       (rc = h->alloc(im.x, 5 * (size_t)nci)) || (rc = h->alloc(im.r, basis_ld(5 * (size_t)nci))) ||
-      (rc = h->alloc(im.w, basis_ld(5 * (size_t)nci))) || (rc = h->alloc(im.part, (size_t)(2 * kMaxKrylov + 1) * kRedBlocks / 2 + kRedBlocks)) ||
+      (rc = h->alloc(im.w, basis_ld(5 * (size_t)nci))) || (rc = h->alloc(im.part, 2 * kMgsSlots + kRedBlocks)) ||
       (rc = h->alloc(im.scal, (size_t)kScalCount)) || (rc = h->alloc(im.done, 2)) ||
       (rc = h->alloc(im.mgs_L, (size_t)(kMaxKrylov + 1) * kMaxKrylov)))
     return rc;
@@ -162,6 +162,11 @@ Row5 row_scale(const ImpState& im) {
 int fetch(ty_mesh* h, int off, int k) {
   IMP_CU(cudaMemcpyAsync(h->imp.pinned + off, h->imp.scal + off, k * sizeof(double), cudaMemcpyDeviceToHost,
                          h->stream));
+  IMP_CU(cudaStreamSynchronize(h->stream));
+  return TY_OK;
+}
+// wait for kernels that wrote their results to the pinned buffer themselves
+int wait(ty_mesh* h) {
   IMP_CU(cudaStreamSynchronize(h->stream));
   return TY_OK;
 }
@@ -255,8 +260,8 @@ int gmres_typhon(ty_mesh* h, const ty_imp_params* p, ty_imp_stats* st) {
       IMP_CU(IMP_CALL(h, imp_matvec, m, im, V(jk - 1), nullptr, im.w, s, &h->prof));
       ++matvecs;
       // h(ik,jk) = (w, v_ik) after w -= h(ik-1,jk) v_(ik-1); h(jk+1,jk)^2 = (w, w); V(jk) = w / h(jk+1,jk)
-      IMP_CU(IMP_CALL(h, imp_mgs_column, im.w, im.V, n, jk, im.mgs_L, im.part, im.scal, im.done + 1, s));
-      if (int rc = fetch(h, 0, jk + 1)) return rc;
+      IMP_CU(IMP_CALL(h, imp_mgs_column, im.w, im.V, n, jk, im.mgs_L, im.part, P, im.done + 1, s));
+      if (int rc = wait(h)) return rc;
       for (int ik = 1; ik <= jk; ++ik) H(ik, jk) = P[ik - 1];
       H(jk + 1, jk) = std::sqrt(P[jk]);
       for (int ik = 1; ik <= jk - 1; ++ik) {
@@ -435,12 +440,12 @@ int fgmres(ty_mesh* h, Operator& op, const ty_imp_params* p, ty_imp_stats* st) {
       int j, nused = 0;
       for (j = 0; j < mk; ++j) {
         IMP_CU(IMP_CALL(h, imp_basis_pass, V64, V32, ldv, j, im.scal + kScalCoef, j == 0 ? src : im.w,
-                        im.scal + kScalCoef + j, 1, n, im.part, im.done, im.scal + kScalGram, s, &h->prof));
+                        im.scal + kScalCoef + j, 1, n, im.part, im.done, P + kScalGram, s, &h->prof));
         IMP_CU(IMP_CALL(h, imp_precond, m, im, Vd(j), Vf(j), Z(j), Z32(j), s, &h->prof));
         if (int rc = op.apply(Z(j), Z32(j), im.w, &matvecs)) return rc;
         IMP_CU(IMP_CALL(h, imp_basis_pass, V64, V32, ldv, j + 1, nullptr, im.w, nullptr, 0, n, im.part, im.done,
-                        im.scal + kScalProj, s, &h->prof));
-        if (int rc = fetch(h, 0, kScalProj + j + 2)) return rc;
+                        P + kScalProj, s, &h->prof));
+        if (int rc = wait(h)) return rc;
         // column j of the Cholesky factor of G
         double d = P[kScalGram + j];
         for (int i = 0; i < j; ++i) {

@@ -809,18 +809,20 @@ __global__ void k_bicg_shift(double* sc) {
 // form of modified Gram-Schmidt of Swirydowicz, Langou, Ananthan, Yang and Thomas, Numer. Linear
 // Algebra Appl. 28, 2021: two reductions a vector, the same loss of orthogonality).
 // The grid is resident and every thread keeps its K entries of w in registers (K = 0: in
-// memory).  No barrier: a block publishes its sums in slots of its own (prefilled with a NaN
-// pattern that no arithmetic produces) and every block reads all slots, waiting (bounded) for
+// memory).  No barrier: a block publishes its sums in slots of its own (prefilled by the column
+// before with a NaN pattern that no arithmetic produces) and every block reads all slots, waiting (bounded) for
 // those still empty; nothing else travels between blocks.  GB300, 122,825 unknowns, restart 30, us a
 // vector on average: 142 in 2 (jk + 1) launches, 105 with the reductions one after the other in one
-// launch, 35 so (60 with 128 threads a block, 37 with 512).
+// launch, 35 so (60 with 128 threads a block, 37 with 512).  The memset before and the copy after each
+// launch cost 8 us a vector more: the column before empties the slots (a later column has as many
+// blocks or fewer), and the sums go to pinned memory.
 constexpr int kMgsThreads = 256;
 constexpr unsigned long long kMgsEmpty = ~0ull;
 constexpr int kMgsSpins = 1 << 22;
 
 template <int K>
 __global__ void __launch_bounds__(kMgsThreads) k_mgs_column(double* w, double* V, size_t n, int jk, double* L,
-                                                            double* slots, double* out, unsigned* err) {
+                                                            double* slots, double* next, double* out, unsigned* err) {
   constexpr int KR = K > 0 ? K : 1, kWarps = kMgsThreads / 32;
   extern __shared__ double acc[];  // [jk + 1][kMgsThreads] per-thread sums
   __shared__ double h[kMaxKrylov + 1];
@@ -829,6 +831,10 @@ __global__ void __launch_bounds__(kMgsThreads) k_mgs_column(double* w, double* V
   const size_t first = blockIdx.x * (size_t)kMgsThreads + t, stride = g * (size_t)kMgsThreads;
   double W[KR];
   if (t == 0) bad = 0;
+  // this block's slots of the next column's exchanges (read by nobody until the next launch)
+  if (jk < kMaxKrylov)
+    for (int i = t; i < 2 * jk + 3; i += kMgsThreads)
+      reinterpret_cast<unsigned long long*>(next)[(size_t)i * g + blockIdx.x] = kMgsEmpty;
   if constexpr (K > 0) {
 #pragma unroll
     for (int k = 0; k < K; ++k) W[k] = first + k * stride < n ? w[first + k * stride] : 0.0;
@@ -1380,7 +1386,7 @@ cudaError_t imp_asum(const double* a, size_t n, double* part, double* out, cudaS
 }
 
 template <int K>
-cudaError_t mgs_launch(double* w, double* V, size_t n, int jk, double* L, double* slots, double* out, unsigned* err,
+cudaError_t mgs_launch(double* w, double* V, size_t n, int jk, double* L, double* part, double* out, unsigned* err,
                        int sms, cudaStream_t st) {
   const size_t lists = (size_t)(jk + 1) * kMgsThreads * sizeof(double);
   cudaError_t e = cudaFuncSetAttribute(k_mgs_column<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lists);
@@ -1394,15 +1400,16 @@ cudaError_t mgs_launch(double* w, double* V, size_t n, int jk, double* L, double
     if (e != cudaSuccess) return e;
     blocks = std::min(sms * std::max(per, 1), kRedBlocks / 2);
   }
-  if ((e = cudaMemsetAsync(slots, 0xff, (size_t)(2 * jk + 1) * blocks * sizeof(double), st)) != cudaSuccess) return e;
-  void* args[] = {&w, &V, &n, &jk, &L, &slots, &out, &err};
+  double *slots = part + (jk & 1 ? 0 : kMgsSlots), *next = part + (jk & 1 ? kMgsSlots : 0);
+  if (jk == 1 && (e = cudaMemsetAsync(slots, 0xff, (size_t)3 * blocks * sizeof(double), st)) != cudaSuccess) return e;
+  void* args[] = {&w, &V, &n, &jk, &L, &slots, &next, &out, &err};
   return cudaLaunchCooperativeKernel((const void*)k_mgs_column<K>, dim3((unsigned)blocks), dim3(kMgsThreads), args, lists,
                                      st);
 }
 
 // One block per SM with the fewest register entries per thread that cover the vector (152 x 256 x
 // 16 = 622,592 unknowns on GB300); beyond that w stays in memory.
-cudaError_t imp_mgs_column(double* w, double* V, size_t n, int jk, double* L, double* slots, double* out, unsigned* err,
+cudaError_t imp_mgs_column(double* w, double* V, size_t n, int jk, double* L, double* part, double* out, unsigned* err,
                            cudaStream_t st) {
   if (jk < 1 || jk > kMaxKrylov) return cudaErrorInvalidValue;
   int dev = 0, sms = 0;
@@ -1410,12 +1417,12 @@ cudaError_t imp_mgs_column(double* w, double* V, size_t n, int jk, double* L, do
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   sms = std::min(sms, kRedBlocks / 2);
   const size_t row = (size_t)sms * kMgsThreads;
-  if (n <= row) return mgs_launch<1>(w, V, n, jk, L, slots, out, err, sms, st);
-  if (n <= 2 * row) return mgs_launch<2>(w, V, n, jk, L, slots, out, err, sms, st);
-  if (n <= 4 * row) return mgs_launch<4>(w, V, n, jk, L, slots, out, err, sms, st);
-  if (n <= 8 * row) return mgs_launch<8>(w, V, n, jk, L, slots, out, err, sms, st);
-  if (n <= 16 * row) return mgs_launch<16>(w, V, n, jk, L, slots, out, err, sms, st);
-  return mgs_launch<0>(w, V, n, jk, L, slots, out, err, sms, st);
+  if (n <= row) return mgs_launch<1>(w, V, n, jk, L, part, out, err, sms, st);
+  if (n <= 2 * row) return mgs_launch<2>(w, V, n, jk, L, part, out, err, sms, st);
+  if (n <= 4 * row) return mgs_launch<4>(w, V, n, jk, L, part, out, err, sms, st);
+  if (n <= 8 * row) return mgs_launch<8>(w, V, n, jk, L, part, out, err, sms, st);
+  if (n <= 16 * row) return mgs_launch<16>(w, V, n, jk, L, part, out, err, sms, st);
+  return mgs_launch<0>(w, V, n, jk, L, part, out, err, sms, st);
 }
 
 // Blocks of a sweep: a fixed function of n and the device, so that sums repeat from run to run.

@@ -24,6 +24,7 @@ constexpr int kBlk32 = 28;       // FP32 block stride (25 entries + pad to 16 by
 constexpr int kMaxKrylov = 64;   // largest NKRYLOV of Typhon's GMRES
 constexpr int kMaxCgs = 32;      // largest restart length of the flexible GMRES (CGS2)
 constexpr int kRedBlocks = 1216; // blocks of a reduction (152 SMs x 8), fixed for determinism
+constexpr size_t kMgsSlots = (size_t)(2 * kMaxKrylov + 1) * (kRedBlocks / 2);  // block sums of a Krylov vector's exchanges
 constexpr int kRedThreads = 256;
 constexpr int kCgsThreads = 128;  // threads of a Krylov basis pass block (sums: (kMaxCgs + 1) x 128 doubles of shared memory)
 
@@ -52,7 +53,7 @@ struct ImpState {
   float* V32 = nullptr;       // [nk + 1][5 nci] Krylov basis of the mixed-precision flexible GMRES
   double* Z = nullptr;        // [nk][5 nci] preconditioned basis (flexible GMRES, FP64)
   float* Z32 = nullptr;       // [nk][5 nci] preconditioned basis (mixed precision)
-  double* part = nullptr;     // [kMaxKrylov + 1][kRedBlocks] partial sums
+  double* part = nullptr;     // [2 * kMgsSlots + kRedBlocks] partial sums; two sets of exchange slots in turn
   double* mgs_L = nullptr;    // [kMaxKrylov + 1][kMaxKrylov] products v_i . v_j, j < i (Typhon's GMRES)
   double* scal = nullptr;     // [4 * kMaxKrylov] device scalars (Hessenberg column, step sizes)
   unsigned* done = nullptr;   // [2] blocks finished in a one-launch reduction (zero between launches);
@@ -65,7 +66,7 @@ struct ImpState {
   // minimises |S (b - A x)| over physical updates x.  Ones (exact no-ops) outside that solve.
   double rs[5] = {1.0, 1.0, 1.0, 1.0, 1.0};
   double rsi[5] = {1.0, 1.0, 1.0, 1.0, 1.0};  // 1 / rs
-  double* pinned = nullptr;   // host mirror of scal (pinned)
+  double* pinned = nullptr;   // host mirror of scal (pinned; Krylov kernels write their results here)
   int last_local = 1;         // time step of the last step: per cell, or last_dt everywhere
   double last_dt = 0.0;
 };
@@ -103,7 +104,7 @@ struct ImpArgs {
                       cudaStream_t st);                                                                 \
   cudaError_t imp_asum(const double* a, size_t n, double* part, double* out, cudaStream_t st);           \
   cudaError_t res_l1(int nci, const double* acc, size_t ld, double* part, double* out, cudaStream_t st);  \
-  cudaError_t imp_mgs_column(double* w, double* V, size_t n, int jk, double* L, double* slots,           \
+  cudaError_t imp_mgs_column(double* w, double* V, size_t n, int jk, double* L, double* part,            \
                              double* out, unsigned* err, cudaStream_t st);                               \
   cudaError_t imp_basis_pass(double* V, float* V32, size_t ldv, int nv, const double* c,                \
                              const double* src, const double* sp, int extend, size_t n, double* part,   \

@@ -6,7 +6,7 @@
 // colour order (flux_to_res.f90); the diagonal of the symmetrised implicit matrix
 // diag(V/dt) A is V/dt - sum_f J_R S over the cell's faces in ascending face order, its
 // off-diagonal J_R S, as the oracle assembles them.  Conjugate gradients keep their scalars
-// on the device; the host reads the residual norm every few iterations.
+// on the device: the FP64 solve runs in launches of up to 1,000 iterations of one cooperative kernel.
 #pragma once
 #include "implicit.hpp"
 #include "kdif.hpp"
