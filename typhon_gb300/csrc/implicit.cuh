@@ -811,7 +811,7 @@ __global__ void k_bicg_shift(double* sc) {
 // The grid is resident and every thread keeps its K entries of w in registers (K = 0: in
 // memory).  No barrier: a block publishes its sums in slots of its own (prefilled by the column
 // before with a NaN pattern that no arithmetic produces) and every block reads all slots, waiting (bounded) for
-// those still empty; nothing else travels between blocks.  GB300, 122,825 unknowns, restart 30, us a
+// those still empty, five polls in flight per lane; nothing else travels between blocks.  GB300, 122,825 unknowns, restart 30, us a
 // vector on average: 142 in 2 (jk + 1) launches, 105 with the reductions one after the other in one
 // launch, 35 so (60 with 128 threads a block, 37 with 512).  The memset before and the copy after each
 // launch cost 8 us a vector more: the column before empties the slots (a later column has as many
@@ -896,14 +896,23 @@ __global__ void __launch_bounds__(kMgsThreads) k_mgs_column(double* w, double* V
     }
     for (int i = wid; i < count; i += kWarps) {
       double s = 0.0;
-      for (int q = lane; q < g; q += 32) {
+      auto poll = [&](int q) {
         unsigned long long b;
-        int spins = 0;
-        do {
-          asm volatile("ld.relaxed.gpu.u64 %0, [%1];" : "=l"(b) : "l"(sl + (size_t)i * g + q) : "memory");
-        } while (b == kMgsEmpty && ++spins < kMgsSpins);
-        if (b == kMgsEmpty) bad = 1;
-        s += __longlong_as_double((long long)b);
+        asm volatile("ld.relaxed.gpu.u64 %0, [%1];" : "=l"(b) : "l"(sl + (size_t)i * g + q) : "memory");
+        return b;
+      };
+      constexpr int kBatch = 5;  // polls in flight per lane: 160 blocks
+      for (int q = lane; q < g; q += 32 * kBatch) {
+        unsigned long long b[kBatch];
+#pragma unroll
+        for (int d = 0; d < kBatch; ++d) b[d] = q + 32 * d < g ? poll(q + 32 * d) : 0ull;
+#pragma unroll
+        for (int d = 0; d < kBatch; ++d) {
+          if (q + 32 * d >= g) break;
+          for (int spins = 0; b[d] == kMgsEmpty && spins < kMgsSpins; ++spins) b[d] = poll(q + 32 * d);
+          if (b[d] == kMgsEmpty) bad = 1;
+          s += __longlong_as_double((long long)b[d]);
+        }
       }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
