@@ -321,9 +321,9 @@ def run_ours(args, rank, world, local):
     ach = per[dom]["achieved_gbs"]
     # DRAM traffic and FP64 instructions per unit, from one ncu capture of the same kernels on
     # the 40^3x5 mesh (320,000 cells, 649,600 faces), scaled by the units of this mesh
-    per_unit = {"cell_fast": (nci, (65.42e6 + 11.33e6) / 320000, 198) if mtab else
-                (nci, (96.07e6 + 53.98e6) / 320000, 261),
-                "face_flux_fast": (md.nface, (72.21e6 + 4.60e6) / 649600, 127)}
+    per_unit = {"cell_fast": (nci, (65.10e6 + 12.46e6) / 320000, 145) if mtab else
+                (nci, (126.32e6 + 48.47e6) / 320000, 425),  # van Albada
+                "face_flux_fast": (md.nface, (72.22e6 + 1.64e6) / 649600, 105)}  # Roe
     traffic = None
     fp64_roof = None
     if dom in per_unit and args.mode == "fast":

@@ -813,7 +813,7 @@ __global__ void k_bicg_shift(double* sc) {
 // before with a NaN pattern that no arithmetic produces) and every block reads all slots, waiting (bounded) for
 // those still empty, five polls in flight per lane; nothing else travels between blocks.  GB300, 122,825 unknowns, restart 30, us a
 // vector on average: 142 in 2 (jk + 1) launches, 105 with the reductions one after the other in one
-// launch, 35 so (60 with 128 threads a block, 37 with 512).  The memset before and the copy after each
+// launch, 35 so (60 with 128 threads a block, 37 with 512), 33 with several polls in flight.  The memset before and the copy after each
 // launch cost 8 us a vector more: the column before empties the slots (a later column has as many
 // blocks or fewer), and the sums go to pinned memory.
 constexpr int kMgsThreads = 256;
