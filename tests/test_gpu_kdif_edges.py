@@ -1,0 +1,56 @@
+"""Conjugate gradients of heat conduction at the edges: data so small that r.D^-1 r is subnormal."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ty():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from typhon_gb300 import build
+    build.build()
+    import typhon_gb300
+    return typhon_gb300
+
+
+def setup(ty, n, sigma):
+    """n^3 x 6 tetrahedra, lognormal conductivity, zero temperature on the x faces, adiabatic elsewhere."""
+    from typhon_gb300 import umesh
+    md = ty.preprocess(umesh.gen_kuhn_box(n, 1.0), 3, [(f, umesh.BC_WALL, "", (0.0, 0.0, 0.0)) for f in
+                                                       ("IMIN", "IMAX", "JMIN", "JMAX", "KMIN", "KMAX")])
+    kind = np.zeros(md.nface, np.int32)
+    b = np.arange(md.nface_int, md.nface)
+    kind[b] = np.where(np.abs(md.face_centre[b, 0] - 0.5) > 0.4999, 1, 2)
+    g = ty.Grid(md)
+    g.set_spat("HLLC", mode="fast")
+    kc = np.exp(sigma * np.random.default_rng(n).standard_normal(md.ncell_int))
+    g.kdif_setup(kc, kind, np.zeros(md.nface), flux="FULL", heat_capacity=1.0)
+    return md, g
+
+
+def residual(md, g, x, b):
+    """|b - S x| / |b| on the assembled symmetrised matrix."""
+    a, c1, c2 = g.kdif_get("jac")[:md.nface_int], md.fc1[:md.nface_int], md.fc2[:md.nface_int]
+    n = len(x)
+    y = g.kdif_get("diag") * x + np.bincount(c1, a * x[c2], n) + np.bincount(c2, a * x[c1], n)
+    return np.linalg.norm(b - y) / np.linalg.norm(b)
+
+
+# |b|^2 is about 1e-299; where |r| / |b| has fallen to 1e-5, gamma = r.D^-1 r is below 2^-1022 and still
+# has 2^-1074 / 1e-310 = 5e-14 relative precision.  Tolerance: the requested 1e-5, and as much again
+# for the recurrence's drift from the true residual.
+@pytest.mark.parametrize("solver", ["CG"])
+def test_subnormal_gamma(ty, solver):
+    md, g = setup(ty, 8, 2.0)
+    scale = 1e-150
+    g.kdif_set_temperature(scale * np.random.default_rng(1).uniform(0.0, 1.0, md.ncell_int))
+    T0 = g.kdif_temperature()
+    st = g.kdif_implicit_step(0.05, solver, tol=1e-5, max_it=2000)
+    assert st["iterations"] < 2000 and st["rel_res"] < 1e-5
+    x = (g.kdif_temperature() - T0) / scale
+    assert np.isfinite(x).all() and np.abs(x).max() > 0
+    assert residual(md, g, x, g.kdif_get("balance") / scale) < 2e-5
+    g.close()

@@ -270,7 +270,7 @@ __global__ void k_kdif_update_T(DevMesh m, KdifState k) {
 // delta = w.u (and r.r when the residual is checked), come from the same iterate:
 //   p = u + beta p, s = w + beta s, x += alpha p, r -= alpha s, u = r / diag;  barrier
 //   w = S u; gamma, delta;  barrier;  beta = gamma / gamma_old,
-//   alpha = gamma / (delta - beta gamma / alpha_old)
+//   alpha = gamma / (delta - beta (gamma / alpha_old))
 // One cooperative launch runs up to kPcgChunk iterations: the grid is resident, every thread
 // owns up to K cells whose r, p, s and w stay in registers, only u travels through L2 (z), and
 // the scalars are recomputed by every block from the blocks' partial sums, in block order
@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(kPcgThreads, K > 0 ? 1 : 2) k_kdif_pcg(int n, 
   unsigned goal = 0;
   bool a32 = a.a32 != 0;
   int it = a.it0, done = 0, switched = 0;
-  double alpha, beta, gamma, b2, rr = 0.0;
+  double alpha = 0.0, beta = 0.0, gamma = 0.0, b2, rr = 0.0;
   // neighbour lists of this thread's cells, [j][slot][thread]: read every iteration, and the
   // address of the gather that the FP64 chain waits for
   extern __shared__ int nbs[];
@@ -419,17 +419,18 @@ __global__ void __launch_bounds__(kPcgThreads, K > 0 ? 1 : 2) k_kdif_pcg(int n, 
     else product_of(k.ell_a, v, want_rr);
   };
   double v[kPcgPart];
-  // scalars of the next step, by one thread: sh[0..2] the sums, sh[3] alpha, sh[4] beta, with
-  // 1/alpha = delta/gamma - beta/alpha_old
+  // Scalars of the next step: sh[0..2] the sums, sh[3] alpha, sh[4] beta.  IEEE divisions (a
+  // reciprocal's seed flushes the subnormal numbers that gamma may fall to), two of the three
+  // side by side in one warp: gamma / gamma_old and gamma / alpha_old.
   __shared__ double sh[5];
-  double ialpha = 0.0, igamma = 0.0;  // thread 0's: 1/alpha, 1/gamma
   auto scalars = [&](bool first_step) {
-    if (threadIdx.x == 0) {
-      const double ig = rcp_nr(sh[0]), be = first_step ? 0.0 : sh[0] * igamma;
-      ialpha = fma(sh[1], ig, -(be * ialpha));
-      igamma = ig;
-      sh[3] = rcp_nr(ialpha);
-      sh[4] = be;
+    if (threadIdx.x < 32) {
+      const double g = sh[0], q = first_step ? 0.0 : g / (threadIdx.x == 0 ? gamma : alpha);
+      const double ga = __shfl_sync(0xffffffffu, q, 1);
+      if (threadIdx.x == 0) {
+        sh[3] = g / (sh[1] - q * ga);
+        sh[4] = q;
+      }
     }
     __syncthreads();
     gamma = sh[0];
@@ -466,8 +467,6 @@ __global__ void __launch_bounds__(kPcgThreads, K > 0 ? 1 : 2) k_kdif_pcg(int n, 
     if (!(b2 > 0.0)) done = 1;  // zero right-hand side
   } else {
     alpha = k.scal[kPcgAlpha]; beta = k.scal[kPcgBeta]; gamma = k.scal[kPcgGamma]; b2 = k.scal[kPcgB2];
-    ialpha = 1.0 / alpha;
-    igamma = 1.0 / gamma;
     if (K > 0) {
       TY_EACH_CELL
         R[q] = gr[i]; P[q] = gp[i]; Q[q] = gs[i]; W[q] = gw[i];
