@@ -1,4 +1,5 @@
-"""Conjugate gradients of heat conduction at the edges: data so small that r.D^-1 r is subnormal."""
+"""Conjugate gradients of heat conduction at the edges: data so small that r.D^-1 r is subnormal,
+and few cells, where the residual becomes exactly zero between two checks of it."""
 import numpy as np
 import pytest
 
@@ -53,4 +54,34 @@ def test_subnormal_gamma(ty, solver):
     x = (g.kdif_temperature() - T0) / scale
     assert np.isfinite(x).all() and np.abs(x).max() > 0
     assert residual(md, g, x, g.kdif_get("balance") / scale) < 2e-5
+    g.close()
+
+
+# One cell: one step solves the system and leaves r = 0 or rounding.  A strip of equal cells, heated
+# alike along both sides: equal rows, the same.  Checked every ten iterations, the solve must end at
+# the next check and not carry 0 / 0 into x.  Tolerance: 1e-12 is requested; the true residual of a
+# well-conditioned system of a few cells is within a few ulp of the recurrence's.
+@pytest.mark.parametrize("solver", ["CG", "CG-MIXED"])
+@pytest.mark.parametrize("cells", ["one", "strip"])
+@pytest.mark.parametrize("seed", range(8))
+def test_exact_convergence(ty, cells, solver, seed):
+    from typhon_gb300 import umesh
+    rng = np.random.default_rng(seed)
+    ni = 1 if cells == "one" else 6
+    md = ty.preprocess(umesh.gen_grid2d(ni, 1, 1.0, rng.uniform(0.5, 2.0), "quad"), 2,
+                       [(f, umesh.BC_WALL, "", (0.0, 0.0, 0.0)) for f in ("IMIN", "IMAX", "JMIN", "JMAX")])
+    kind, val = np.zeros(md.nface, np.int32), np.zeros(md.nface)
+    b = np.arange(md.nface_int, md.nface)
+    y = np.abs(md.face_normal[b, 1]) > 0.5  # the long sides: isothermal; the ends: adiabatic
+    kind[b], val[b] = np.where(y, 1, 2), np.where(y, rng.uniform(0.5, 2.0), 0.0)
+    g = ty.Grid(md)
+    g.set_spat("HLLC", mode="fast")
+    g.kdif_setup(np.full(ni, rng.uniform(0.1, 10.0)), kind, val, flux="COMPACT", heat_capacity=rng.uniform(0.5, 2.0))
+    cp = g._kdif_cp
+    g.kdif_set_temperature(np.full(ni, rng.uniform(0.0, 1.0)))
+    T0 = g.kdif_temperature()
+    st = g.kdif_implicit_step(rng.uniform(0.1, 1.0), solver, tol=1e-12, max_it=2000)
+    T = g.kdif_temperature()
+    assert np.isfinite(T).all() and np.isfinite(st["rel_res"]) and st["rel_res"] < 1e-12 and st["iterations"] <= 30
+    assert residual(md, g, (T - T0) * cp, g.kdif_get("balance")) < 1e-10
     g.close()

@@ -421,14 +421,17 @@ __global__ void __launch_bounds__(kPcgThreads, K > 0 ? 1 : 2) k_kdif_pcg(int n, 
   double v[kPcgPart];
   // Scalars of the next step: sh[0..2] the sums, sh[3] alpha, sh[4] beta.  IEEE divisions (a
   // reciprocal's seed flushes the subnormal numbers that gamma may fall to), two of the three
-  // side by side in one warp: gamma / gamma_old and gamma / alpha_old.
+  // side by side in one warp: gamma / gamma_old and gamma / alpha_old.  gamma = 0: r = 0, reached
+  // exactly by a few cells before the residual is due for a check; every block sees it and stops.
   __shared__ double sh[5];
   auto scalars = [&](bool first_step) {
     if (threadIdx.x < 32) {
       const double g = sh[0], q = first_step ? 0.0 : g / (threadIdx.x == 0 ? gamma : alpha);
       const double ga = __shfl_sync(0xffffffffu, q, 1);
       if (threadIdx.x == 0) {
-        sh[3] = g / (sh[1] - q * ga);
+        const double den = sh[1] - q * ga;
+        if (den == 0.0 && fabs(g) < 0x1p-1022) sh[0] = 0.0;  // both underflowed
+        sh[3] = g / den;
         sh[4] = q;
       }
     }
@@ -464,7 +467,7 @@ __global__ void __launch_bounds__(kPcgThreads, K > 0 ? 1 : 2) k_kdif_pcg(int n, 
     TY_END_CELL
     if (!restart()) { if (threadIdx.x == 0) k.count[1] = 1u; return; }
     b2 = rr = sh[2];
-    if (!(b2 > 0.0)) done = 1;  // zero right-hand side
+    if (!(b2 > 0.0) || gamma == 0.0) done = 1;  // zero right-hand side
   } else {
     alpha = k.scal[kPcgAlpha]; beta = k.scal[kPcgBeta]; gamma = k.scal[kPcgGamma]; b2 = k.scal[kPcgB2];
     if (K > 0) {
@@ -489,8 +492,8 @@ __global__ void __launch_bounds__(kPcgThreads, K > 0 ? 1 : 2) k_kdif_pcg(int n, 
     product(v, check);
     if (!grid_sum(v, sh, k.part, k.count, goal += gridDim.x)) { if (threadIdx.x == 0) k.count[1] = 1u; return; }
     scalars(false);
-    if (check) {
-      rr = sh[2];
+    if (check || gamma == 0.0) {
+      rr = sh[2];  // 0 where it was not summed: r = 0
       const double rel = sqrt(rr / b2);
       if (a32 && rel < a.sw) {
         // restart on the FP64 conductances from the true residual r = b - S x (continuing the
@@ -513,7 +516,9 @@ __global__ void __launch_bounds__(kPcgThreads, K > 0 ? 1 : 2) k_kdif_pcg(int n, 
           ok = grid_barrier(k.count, goal += gridDim.x) && restart();
         }
         if (!ok) { if (threadIdx.x == 0) k.count[1] = 1u; return; }
-      } else if (!a32 && rel < a.tol) {
+        rr = sh[2];
+        done = gamma == 0.0;
+      } else if (!a32 && (rel < a.tol || gamma == 0.0)) {
         done = 1;
       }
     }
