@@ -61,3 +61,28 @@ def test_barth_subnormal_velocity(ty, highres, limiter, postlim, size):
     s.rhs(dt)
     close(R, s.get("residu")[:, :md.ncell_int])
     g.close()
+
+
+# Cells of zero pressure (an evacuated region): T = 0 at the faces between them, where Sutherland's
+# viscosity is 0.  The inviscid flux is Rusanov's, regular there.
+@pytest.mark.parametrize("flux", ["CELL-AVERAGE", "FULL"])
+def test_sutherland_zero_temperature(ty, flux):
+    raw, bcs, md = tet_box(ty)
+    rng = np.random.default_rng(4)
+    x = md.cell_centre
+    q = np.stack([1.2 + 0.1 * rng.random(len(x)), 1e5 * (1.0 + 0.1 * rng.random(len(x))), 30.0 * rng.standard_normal(len(x)),
+                  20.0 * rng.standard_normal(len(x)), 10.0 * rng.standard_normal(len(x))])
+    q[1:, np.linalg.norm(x - 0.5, axis=1) < 0.35] = 0.0  # at rest: p = 0 exactly from the conserved state
+    visc = dict(rgas=287.0, prandtl=0.72)
+    g = ty.Grid(md)
+    g.set_spat("RUSANOV", mode="fast", dissipative_flux=flux, viscosity="SUTHERLAND", **visc)
+    om = op.Mesh.from_raw(raw).build(3, [tuple(b) for b in bcs])
+    s = op.Solver(om, op.SCH_RUSANOV, gradmeth=op.GRAD_LSQ, viscous={"CELL-AVERAGE": op.VISC_CELLAVG, "FULL": op.VISC_CELLFULL}[flux],
+                  visc_law=1, **visc)
+    s.set_prim(q)
+    g.set_prim(q)
+    s.rhs(1e-6)
+    b = s.get("residu")[:, :md.ncell_int]
+    assert np.isfinite(b).all()
+    close(g.integration_grid(1e-6), b)
+    g.close()

@@ -179,13 +179,21 @@ __global__ void k_prim(DevMesh m, const double* __restrict__ cons, double* __res
   for (int v = 0; v < 5; ++v) prim[v * (size_t)m.ldc + c] = q[v];
 }
 
+// x^1.5: 0 for x = 0 (and below the normal numbers, whose result underflows), where the root's
+// reciprocal is infinite; NaN for x < 0
+template <class T>
+__device__ __forceinline__ T pow15_nr(T x) {
+  const T r = x * x * rsqrt_nr(x);
+  return ((unsigned)__double2hiint(value(x)) << 1) < (2u << 20) ? T(0.0) : r;
+}
+
 // calc_viscosity (SOURCE/EQNS/EQNS.f90:225-265): nu rho, or Sutherland with AIR's constants
 __device__ __forceinline__ double viscosity(const SpatOpts& o, double rho, double T) {
   if (o.visc_law == TY_VISC_KINEMATIC) return o.visc_kin * rho;
   const double mu0 = 0.0000168, T0 = 273.00, S = 110.50;
   if constexpr (kFast) {
     const double x = T * (1.0 / T0);
-    return mu0 * (T0 + S) * (x * sqrt_nr(x)) * rcp_nr(T + S);
+    return mu0 * (T0 + S) * pow15_nr(x) * rcp_nr(T + S);
   }
   return mu0 * pow(T / T0, 1.5) * (T0 + S) / (T + S);
 }
@@ -1104,7 +1112,7 @@ __device__ void add_viscous_fast(const DevMesh& m, const DevState& s, const Spat
   } else {  // mu0 (T/T0)^1.5 (T0 + S) / (T + S), T = tH / r
     const double T0 = 273.00, S0 = 110.50;
     const F64 T = tH * F64(o.irgas), x = T * F64(1.0 / T0);
-    mu = F64(0.0000168 * (T0 + S0)) * (x * x * rsqrt_nr(x)) * rcp_nr(T + F64(S0));
+    mu = F64(0.0000168 * (T0 + S0)) * pow15_nr(x) * rcp_nr(T + F64(S0));
   }
   // velocity gradient at the face (CELL-AVERAGE), G n and G^T n and the divergence
   F64 vL[3], vR[3], G[3][3];
