@@ -86,3 +86,25 @@ def test_sutherland_zero_temperature(ty, flux):
     assert np.isfinite(b).all()
     close(g.integration_grid(1e-6), b)
     g.close()
+
+
+# Cells of negative pressure, single and side by side: Rusanov's wave speed is the ordinary neighbour's
+# beside a single one and NaN between two, in both modes.  Finite entries: the fast mode's envelope.
+def test_rusanov_negative_pressure(ty):
+    raw, bcs, md = tet_box(ty)
+    rng = np.random.default_rng(6)
+    nci = md.ncell_int
+    q = np.stack([1.0 + 0.1 * rng.random(nci), 2.0 + 0.2 * rng.random(nci), *(2.5 * rng.standard_normal((3, nci)))])
+    q[1, rng.random(nci) < 0.08] *= -1.0
+    R = {}
+    for mode in ("exact", "fast"):
+        g = ty.Grid(md)
+        g.set_spat("RUSANOV", mode=mode)
+        g.set_prim(q)
+        R[mode] = g.integration_grid(1e-3)
+        g.close()
+    e, f = R["exact"], R["fast"]
+    nan = ~np.isfinite(e)
+    assert nan.any() and not nan.all()
+    assert np.array_equal(nan, ~np.isfinite(f))
+    close(np.where(nan, 0.0, f), np.where(nan, 0.0, e))

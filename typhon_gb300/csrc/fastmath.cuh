@@ -99,4 +99,15 @@ __device__ __forceinline__ F64 sqrt_nr(F64 a) {
   return __double2hiint(a.v) > 0 ? r.v : 0.0;
 }
 
+// sqrt(a) as the library's for normal numbers: 0 for a == 0 (and subnormal a), NaN for a < 0.  For places
+// where the root of a negative number has to show.
+__device__ __forceinline__ F64 root_nr(F64 a) {
+  const F64 r = a * rsqrt_nr(a);
+  return ((unsigned)__double2hiint(a.v) << 1) < (2u << 20) ? 0.0 : r.v;
+}
+__device__ __forceinline__ double root_nr(double a) {
+  const double r = a * rsqrt_nr(a);
+  return ((unsigned)__double2hiint(a) << 1) < (2u << 20) ? 0.0 : r;
+}
+
 }  // namespace tyk

@@ -29,7 +29,7 @@ __device__ __forceinline__ double jac_div(double a, double b) {
   return a / b;
 }
 __device__ __forceinline__ double jac_sqrt(double a) {
-  if constexpr (kFast) return sqrt_nr(a);
+  if constexpr (kFast) return root_nr(a);
   return sqrt(a);
 }
 

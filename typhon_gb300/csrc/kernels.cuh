@@ -338,6 +338,9 @@ __device__ __forceinline__ long long order_key(double x) {  // orders like x
 }
 __device__ __forceinline__ double min_bits(double a, double b) { return order_key(a) < order_key(b) ? a : b; }
 __device__ __forceinline__ double max_bits(double a, double b) { return order_key(a) < order_key(b) ? b : a; }
+__device__ __forceinline__ bool is_nan(double x) {  // of the quiet NaNs that arithmetic makes
+  return ((unsigned)__double2hiint(x) << 1) > (0x7ffu << 21);
+}
 __device__ __forceinline__ bool is_neg(double x) { return __double2hiint(x) < 0; }  // sign bit
 // x without the sign (fabs of a stored value is an FP64 instruction)
 __device__ __forceinline__ double abs_bits(double x) {
@@ -984,13 +987,21 @@ __device__ void flux_hllc_fast(const SpatOpts& o, const F64* L, const F64* R, F6
   F[4] = fma(m0, qz, c * nz);
 }
 
-// Rusanov times S (calc_flux_rusanov.f90:57-83) without divisions
+// fmax of numbers that are not negative, on their bit patterns; a NaN of either sign loses
+__device__ __forceinline__ double fmax_bits(double a, double b) {
+  const long long ka = is_nan(a) ? -1ll : dbits(a), kb = is_nan(b) ? -1ll : dbits(b);
+  return ka < kb ? b : a;
+}
+
+// Rusanov times S (calc_flux_rusanov.f90:57-83) without divisions.  The root of a negative pressure is
+// NaN, and a face of two such states too; beside an ordinary state it has no say (fmax), as in the
+// exact mode.
 __device__ void flux_rusanov_fast(const SpatOpts& o, const F64* L, const F64* R, F64 nx, F64 ny, F64 nz,
                                   F64 S, F64* F) {
   const F64 TL = L[1] * rcp_nr(L[0]), TR = R[1] * rcp_nr(R[0]);
   const F64 vnl = fma(L[2], nx, fma(L[3], ny, L[4] * nz)), vnr = fma(R[2], nx, fma(R[3], ny, R[4] * nz));
-  const F64 cl = F64(abs_bits(vnl.v)) + sqrt_nr(F64(o.gamma) * TL), cr = F64(abs_bits(vnr.v)) + sqrt_nr(F64(o.gamma) * TR);
-  const F64 ray = max_bits(cl.v, cr.v), hs = F64(0.5) * S;
+  const F64 cl = F64(abs_bits(vnl.v)) + root_nr(F64(o.gamma) * TL), cr = F64(abs_bits(vnr.v)) + root_nr(F64(o.gamma) * TR);
+  const F64 ray = fmax_bits(cl.v, cr.v), hs = F64(0.5) * S;
   const F64 el = fma(F64(o.ig1), TL, F64(0.5) * fma(L[2], L[2], fma(L[3], L[3], L[4] * L[4])));
   const F64 er = fma(F64(o.ig1), TR, F64(0.5) * fma(R[2], R[2], fma(R[3], R[3], R[4] * R[4])));
   const F64 A = hs * ((vnl + ray) * L[0]), B = hs * ((vnr - ray) * R[0]), pp = hs * (L[1] + R[1]);
