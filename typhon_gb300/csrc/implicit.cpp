@@ -58,6 +58,9 @@ constexpr int kScalCount = 3 * kMaxKrylov + 20;
 // vectors they read beside the basis are allocated as long)
 size_t basis_ld(size_t n) { return (n + 1) / 2 * 2; }
 
+// error word of the Krylov kernels' bounded waits: pinned, behind the scalars
+unsigned* late_word(ty_mesh* h) { return reinterpret_cast<unsigned*>(h->imp.pinned + kScalCount); }
+
 template <class T>
 int grow(ty_mesh* h, T*& p, size_t n) {
   if (p) {
@@ -94,14 +97,15 @@ int build_lists(ty_mesh* h) {
       (rc = h->alloc(im.jacR, (size_t)m.nf * kBlk)) || (rc = h->alloc(im.b, 5 * (size_t)nci)) ||
       (rc = h->alloc(im.x, 5 * (size_t)nci)) || (rc = h->alloc(im.r, basis_ld(5 * (size_t)nci))) ||
       (rc = h->alloc(im.w, basis_ld(5 * (size_t)nci))) || (rc = h->alloc(im.part, 2 * kMgsSlots + kRedBlocks)) ||
-      (rc = h->alloc(im.scal, (size_t)kScalCount)) || (rc = h->alloc(im.done, 2)) ||
+      (rc = h->alloc(im.scal, (size_t)kScalCount)) || (rc = h->alloc(im.done, 1)) ||
       (rc = h->alloc(im.mgs_L, (size_t)(kMaxKrylov + 1) * kMaxKrylov)))
     return rc;
-  IMP_CU(cudaMemset(im.done, 0, 2 * sizeof(unsigned)));
+  IMP_CU(cudaMemset(im.done, 0, sizeof(unsigned)));
   IMP_CU(cudaMemcpy(im.cfo, cfo.data(), cfo.size() * sizeof(int), cudaMemcpyHostToDevice));
   IMP_CU(cudaMemcpy(im.cfon, cfon.data(), cfon.size() * sizeof(int), cudaMemcpyHostToDevice));
-  if (!im.pinned && cudaMallocHost((void**)&im.pinned, kScalCount * sizeof(double)) != cudaSuccess)
+  if (!im.pinned && cudaMallocHost((void**)&im.pinned, (kScalCount + 1) * sizeof(double)) != cudaSuccess)
     return TY_ERR_NOMEM;
+  *late_word(h) = 0u;
   im.lists = true;
   return TY_OK;
 }
@@ -165,26 +169,20 @@ int fetch(ty_mesh* h, int off, int k) {
   IMP_CU(cudaStreamSynchronize(h->stream));
   return TY_OK;
 }
-// wait for kernels that wrote their results to the pinned buffer themselves
+// wait for kernels that wrote their results, and that word, to the pinned buffer themselves
 int wait(ty_mesh* h) {
   IMP_CU(cudaStreamSynchronize(h->stream));
-  return TY_OK;
+  volatile unsigned* late = late_word(h);
+  if (!*late) return TY_OK;
+  *late = 0u;
+  tyi::set_error("ty_implicit_step: a wait inside a Krylov kernel timed out");
+  return TY_ERR_CUDA;
 }
 int put(ty_mesh* h, int off, const double* v, int k) {
   std::memcpy(h->imp.pinned + off, v, k * sizeof(double));
   IMP_CU(cudaMemcpyAsync(h->imp.scal + off, h->imp.pinned + off, k * sizeof(double), cudaMemcpyHostToDevice,
                          h->stream));
   return TY_OK;
-}
-
-// the error word of the kernels' bounded waits (stream idle)
-int check_waits(ty_mesh* h) {
-  unsigned timed_out = 0;
-  IMP_CU(cudaMemcpy(&timed_out, h->imp.done + 1, sizeof(unsigned), cudaMemcpyDeviceToHost));
-  if (!timed_out) return TY_OK;
-  IMP_CU(cudaMemset(h->imp.done + 1, 0, sizeof(unsigned)));
-  tyi::set_error("ty_implicit_step: a wait inside a Krylov kernel timed out");
-  return TY_ERR_CUDA;
 }
 
 // ---- Typhon's bdlu_bicgstab on the device (bdlu_bicgstab.f90:40-80) ----
@@ -260,7 +258,7 @@ int gmres_typhon(ty_mesh* h, const ty_imp_params* p, ty_imp_stats* st) {
       IMP_CU(IMP_CALL(h, imp_matvec, m, im, V(jk - 1), nullptr, im.w, s, &h->prof));
       ++matvecs;
       // h(ik,jk) = (w, v_ik) after w -= h(ik-1,jk) v_(ik-1); h(jk+1,jk)^2 = (w, w); V(jk) = w / h(jk+1,jk)
-      IMP_CU(IMP_CALL(h, imp_mgs_column, im.w, im.V, n, jk, im.mgs_L, im.part, P, im.done + 1, s));
+      IMP_CU(IMP_CALL(h, imp_mgs_column, im.w, im.V, n, jk, im.mgs_L, im.part, P, late_word(h), s));
       if (int rc = wait(h)) return rc;
       for (int ik = 1; ik <= jk; ++ik) H(ik, jk) = P[ik - 1];
       H(jk + 1, jk) = std::sqrt(P[jk]);
@@ -299,7 +297,6 @@ int gmres_typhon(ty_mesh* h, const ty_imp_params* p, ty_imp_stats* st) {
     errgmres = ss[nkk + 1] / normp1;
     nit = nit + 1;
   }
-  if (int rc = check_waits(h)) return rc;
   st->restarts = nit;
   st->matvecs = matvecs;
   st->lin_res = errgmres;
@@ -440,11 +437,12 @@ int fgmres(ty_mesh* h, Operator& op, const ty_imp_params* p, ty_imp_stats* st) {
       int j, nused = 0;
       for (j = 0; j < mk; ++j) {
         IMP_CU(IMP_CALL(h, imp_basis_pass, V64, V32, ldv, j, im.scal + kScalCoef, j == 0 ? src : im.w,
-                        im.scal + kScalCoef + j, 1, n, im.part, im.done, P + kScalGram, s, &h->prof));
+                        im.scal + kScalCoef + j, 1, n, im.part, im.done, P + kScalGram, late_word(h),
+                        s, &h->prof));
         IMP_CU(IMP_CALL(h, imp_precond, m, im, Vd(j), Vf(j), Z(j), Z32(j), s, &h->prof));
         if (int rc = op.apply(Z(j), Z32(j), im.w, &matvecs)) return rc;
         IMP_CU(IMP_CALL(h, imp_basis_pass, V64, V32, ldv, j + 1, nullptr, im.w, nullptr, 0, n, im.part, im.done,
-                        P + kScalProj, s, &h->prof));
+                        P + kScalProj, late_word(h), s, &h->prof));
         if (int rc = wait(h)) return rc;
         // column j of the Cholesky factor of G
         double d = P[kScalGram + j];
@@ -500,7 +498,6 @@ int fgmres(ty_mesh* h, Operator& op, const ty_imp_params* p, ty_imp_stats* st) {
       if (std::fabs(a[nused]) <= tol) { ++cycles; break; }
     }
   }
-  if (int rc = check_waits(h)) return rc;
   st->restarts = cycles;
   st->matvecs = matvecs;
   st->lin_res = rel;

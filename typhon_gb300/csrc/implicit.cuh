@@ -1065,7 +1065,7 @@ __global__ void __launch_bounds__(kSweepThreads + 32) k_basis_pass(double* V, si
                                                                const double* __restrict__ src,
                                                                const double* __restrict__ sp, size_t n,
                                                                double* __restrict__ part, unsigned* __restrict__ done,
-                                                               double* __restrict__ out) {
+                                                               double* __restrict__ out, unsigned* err) {
   constexpr int T = kSweepThreads, S = kSweepStages<J>;
   extern __shared__ __align__(16) double buf[];  // [S][J + 1][T]: the vectors 0 .. nv-1, then src
   __shared__ __align__(8) unsigned long long full[S], empty[S];
@@ -1132,7 +1132,7 @@ __global__ void __launch_bounds__(kSweepThreads + 32) k_basis_pass(double* V, si
     __syncwarp();
     if ((t & 31) == 0) mbar_arrive(&empty[st]);
   }
-  if (!ok) done[1] = 1u;
+  if (!ok) *err = 1u;
   __syncthreads();  // every copy has been waited for: the stages become the per-thread sums
   if (t < T) {
 #pragma unroll
@@ -1444,24 +1444,25 @@ inline unsigned sm_count() {
 
 template <int J>
 cudaError_t basis_launch_j(double* V, size_t ldv, int nv, const double* c, const double* src, const double* sp,
-                           int extend, size_t n, double* part, unsigned* done, double* out, cudaStream_t st) {
+                           int extend, size_t n, double* part, unsigned* done, double* out, unsigned* err,
+                           cudaStream_t st) {
   const unsigned g = (unsigned)std::max<size_t>(1, std::min<size_t>((n + kSweepThreads - 1) / kSweepThreads, sm_count()));
   const size_t sums = (size_t)kSweepStages<J> * (J + 1) * kSweepThreads * sizeof(double);
   auto* k = extend ? k_basis_pass<J, true> : k_basis_pass<J, false>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sums);
   if (e != cudaSuccess) return e;
-  k<<<g, kSweepThreads + 32, sums, st>>>(V, ldv, nv, c, src, sp, n, part, done, out);
+  k<<<g, kSweepThreads + 32, sums, st>>>(V, ldv, nv, c, src, sp, n, part, done, out, err);
   return cudaGetLastError();
 }
 
 // the smallest even J >= nv
 template <int J = 2>
 cudaError_t basis_launch(double* V, size_t ldv, int nv, const double* c, const double* src, const double* sp, int extend,
-                         size_t n, double* part, unsigned* done, double* out, cudaStream_t st) {
+                         size_t n, double* part, unsigned* done, double* out, unsigned* err, cudaStream_t st) {
   if constexpr (J < kMaxCgs) {
-    if (nv > J) return basis_launch<J + 2>(V, ldv, nv, c, src, sp, extend, n, part, done, out, st);
+    if (nv > J) return basis_launch<J + 2>(V, ldv, nv, c, src, sp, extend, n, part, done, out, err, st);
   }
-  return basis_launch_j<J>(V, ldv, nv, c, src, sp, extend, n, part, done, out, st);
+  return basis_launch_j<J>(V, ldv, nv, c, src, sp, extend, n, part, done, out, err, st);
 }
 
 // an FP32 sweep, bound by HBM, takes 8, 16 or 32 slots and every resident block
@@ -1486,12 +1487,12 @@ inline cudaError_t basis_launch32(float* V, size_t ldv, int nv, const double* c,
 
 cudaError_t imp_basis_pass(double* V, float* V32, size_t ldv, int nv, const double* c, const double* src,
                            const double* sp, int extend, size_t n, double* part, unsigned* done, double* out,
-                           cudaStream_t st, Prof* pr) {
+                           unsigned* err, cudaStream_t st, Prof* pr) {
   if (nv < 0 || nv > kMaxCgs) return cudaErrorInvalidValue;
   cudaError_t e = cudaSuccess;
   pr->launch(K_IMP_ORTHO, st, [&] {
     e = V32 ? basis_launch32(V32, ldv, nv, c, src, sp, extend, n, part, done, out, st)
-            : basis_launch(V, ldv, nv, c, src, sp, extend, n, part, done, out, st);
+            : basis_launch(V, ldv, nv, c, src, sp, extend, n, part, done, out, err, st);
   });
   return e;
 }

@@ -56,8 +56,7 @@ struct ImpState {
   double* part = nullptr;     // [2 * kMgsSlots + kRedBlocks] partial sums; two sets of exchange slots in turn
   double* mgs_L = nullptr;    // [kMaxKrylov + 1][kMaxKrylov] products v_i . v_j, j < i (Typhon's GMRES)
   double* scal = nullptr;     // [4 * kMaxKrylov] device scalars (Hessenberg column, step sizes)
-  unsigned* done = nullptr;   // [2] blocks finished in a one-launch reduction (zero between launches);
-                              // error word of the bounded waits inside the Krylov kernels
+  unsigned* done = nullptr;   // [1] blocks finished in a one-launch reduction (zero between launches)
   double* upert = nullptr;    // [5][ldc] perturbed state (Jacobian-free products)
   double* r0 = nullptr;       // [5 nci] residual at the unperturbed state (Jacobian-free)
   double* bs = nullptr;       // [5 nci] right-hand side of the flexible GMRES with its rows scaled
@@ -66,7 +65,8 @@ struct ImpState {
   // minimises |S (b - A x)| over physical updates x.  Ones (exact no-ops) outside that solve.
   double rs[5] = {1.0, 1.0, 1.0, 1.0, 1.0};
   double rsi[5] = {1.0, 1.0, 1.0, 1.0, 1.0};  // 1 / rs
-  double* pinned = nullptr;   // host mirror of scal (pinned; Krylov kernels write their results here)
+  double* pinned = nullptr;   // host mirror of scal (pinned; Krylov kernels write their results here), and
+                              // behind it the error word of their bounded waits
   int last_local = 1;         // time step of the last step: per cell, or last_dt everywhere
   double last_dt = 0.0;
 };
@@ -108,7 +108,7 @@ struct ImpArgs {
                              double* out, unsigned* err, cudaStream_t st);                               \
   cudaError_t imp_basis_pass(double* V, float* V32, size_t ldv, int nv, const double* c,                \
                              const double* src, const double* sp, int extend, size_t n, double* part,   \
-                             unsigned* done, double* out, cudaStream_t st, Prof* pr);                   \
+                             unsigned* done, double* out, unsigned* err, cudaStream_t st, Prof* pr);    \
   cudaError_t imp_scale(const double* w, double s, double* v, size_t n, cudaStream_t st);                \
   cudaError_t imp_bicgstab_iter(const DevMesh& m, const ImpState& im, double* x, double* r1,             \
                                 const double* r2, double* p, double* v, double* s, double* t, int first,  \
