@@ -1398,7 +1398,10 @@ template <int K>
 cudaError_t mgs_launch(double* w, double* V, size_t n, int jk, double* L, double* part, double* out, unsigned* err,
                        int sms, cudaStream_t st) {
   const size_t lists = (size_t)(jk + 1) * kMgsThreads * sizeof(double);
-  cudaError_t e = cudaFuncSetAttribute(k_mgs_column<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lists);
+  // the limit of the longest column, whatever this one needs: the attribute is the function's, and
+  // another thread's launch may stand between this call and the launch below
+  cudaError_t e = cudaFuncSetAttribute(k_mgs_column<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (kMaxKrylov + 1) * kMgsThreads * (int)sizeof(double));
   if (e != cudaSuccess) return e;
   int blocks = sms;
   if (K > 0) {

@@ -572,7 +572,10 @@ cudaError_t pcg_launch(int n, int ns, const KdifState& k, const PcgArgs& a, int 
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const size_t lists = (size_t)K * ns * threads * sizeof(int);
-  cudaError_t e = cudaFuncSetAttribute(k_kdif_pcg<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lists);
+  // the limit of the largest lists, whatever these need: the attribute is the function's, and another
+  // thread's launch on another mesh may stand between this call and the launch below
+  cudaError_t e = cudaFuncSetAttribute(k_kdif_pcg<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       K * kMaxSlot * kPcgThreads * (int)sizeof(int));
   if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_kdif_pcg<K>, threads, lists);
   if (e != cudaSuccess) return e;
   if (per < 1) return cudaErrorCooperativeLaunchTooLarge;
