@@ -43,7 +43,8 @@ constexpr int kBlock = 256;
 // on the stream drains, and may start before it has finished; pdl_wait() returns when it has,
 // and its writes are visible (at once in a kernel launched normally).  Every kernel so launched
 // calls it before it touches anything that a kernel writes (mesh tables copied at creation may
-// be read earlier), so completion is transitive along the stream.  The gap between the short
+// be read earlier), so completion is transitive along the stream.  Their parameters carry no
+// __restrict__: a compiler may take such data as constant and read it ahead of the wait.  The gap between the short
 // kernels of a Runge-Kutta stage shrinks from 2.7 to 0.2 us.  No kernel calls
 // launch_dependents: blocks of the next kernel then fill the SMs that have room first and stay
 // there, which doubled the 8,192-cell vortex's step (75 -> 150 us).
@@ -167,7 +168,7 @@ __device__ __forceinline__ void cons_to_prim(double gamma, const double c[5], do
   q[2] = vx; q[3] = vy; q[4] = vz;
 }
 
-__global__ void k_prim(DevMesh m, const double* __restrict__ cons, double* __restrict__ prim, double gamma) {
+__global__ void k_prim(DevMesh m, const double* cons, double* prim, double gamma) {
   pdl_wait();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= m.nci) return;
@@ -270,7 +271,7 @@ __device__ void inout_state(const DevMesh& m, const SpatOpts& o, int f, int kind
 // ghost states: periodic copy, symmetry mirror (velocity reflected across the face),
 // adiabatic moving wall (setboco_ns_flux.f90, cell-state mode: pressure copied, temperature
 // of the cell minus lflux d / conduct with lflux = 0, velocity reflected about the wall's)
-__global__ void k_ghost_prim(DevMesh m, double* __restrict__ prim, SpatOpts o) {
+__global__ void k_ghost_prim(DevMesh m, double* prim, SpatOpts o) {
   pdl_wait();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= m.ng) return;
@@ -478,7 +479,7 @@ __global__ void __launch_bounds__(kBlock) k_grad(DevMesh m, DevState s) {
   }
 }
 
-__global__ void k_ghost_grad(DevMesh m, double* __restrict__ grad) {
+__global__ void k_ghost_grad(DevMesh m, double* grad) {
   pdl_wait();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= m.ng) return;
@@ -1714,7 +1715,7 @@ __device__ __forceinline__ double load_dt(double dt, const unsigned long long* d
 }
 
 __global__ void __launch_bounds__(kBlock) k_gather(DevMesh m, DevState s, double dt, const unsigned long long* dtbits,
-                                                   double* __restrict__ out, int ld) {
+                                                   double* out, int ld) {
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= m.nci) return;
   using T = typename std::conditional<kFast, F64, double>::type;
@@ -1779,7 +1780,7 @@ __device__ __forceinline__ void flag_error(int* err, int code, int cell) {
   if (atomicCAS(err, 0, code) == 0) err[1] = cell;
 }
 
-__global__ void __launch_bounds__(kBlock) k_timestep(DevMesh m, const double* __restrict__ cons, double gamma,
+__global__ void __launch_bounds__(kBlock) k_timestep(DevMesh m, const double* cons, double gamma,
                                                       double cfl, unsigned long long* dtbits, int* err) {
   pdl_wait();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
