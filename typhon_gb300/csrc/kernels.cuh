@@ -1362,13 +1362,18 @@ __global__ void __launch_bounds__(kBlock) k_face_flux_lim(DevMesh m, DevState s,
 
 
 #if TY_FAST
-// |a| b < |c| d of positive products, as bit patterns, scaled where c or b is so small that a product
-// could be subnormal.  A call, so that the multiplications are not if-converted into the callers (a
-// predicated-off FP64 instruction occupies the pipe as well), and a short one: the registers of a
-// division, with its own call, or of two scale factors are the callers' too (FORM 0 of the kernel
-// below: 51 -> 69 and 54, its launch 10 % slower with the first).
-constexpr int kTiny = (1023 - 400) << 20;  // upper word of 2^-400
+// |a| b < |c| d of positive products, as bit patterns.  A call, so that the multiplications are not
+// if-converted into the callers (a predicated-off FP64 instruction occupies the pipe as well), and a
+// short one: the registers of a division, with its own call, are the callers' too (FORM 0 of the
+// kernel below: 51 -> 69, its launch 10 % slower).
 __device__ __noinline__ bool product_less(double a, double b, double c, double d) {
+  return dbits(fabs(a) * b) < dbits(d * fabs(c));
+}
+
+// The same where a, b, c or d is out of the FP32 comparison's range: scaled where c or b is so small that
+// a product could be subnormal.
+constexpr int kTiny = (1023 - 400) << 20;  // upper word of 2^-400
+__device__ __noinline__ bool product_less_far(double a, double b, double c, double d) {
   a = fabs(a);
   c = fabs(c);
   if (__double2hiint(c) < kTiny || __double2hiint(b) < kTiny) {
@@ -1380,13 +1385,9 @@ __device__ __noinline__ bool product_less(double a, double b, double c, double d
   return dbits(a * b) < dbits(d * c);
 }
 
-// klim n / d where d may have no normal reciprocal (a call for the same reasons)
+// klim n / d where d is below 2^-400 and may have no normal reciprocal (a call for the same reasons)
 __device__ __noinline__ double barth_ratio(double klim, double n, double d) {
-  if (__double2hiint(d) < kTiny) {
-    n *= 0x1p600;
-    d *= 0x1p600;
-  }
-  return klim * n * rcp_nr(d);
+  return klim * (n * 0x1p600) * rcp_nr(d * 0x1p600);
 }
 
 // van Albada's phi(a, b) = a b (a + b) / (a^2 + b^2) where a b > 0, else 0, sum = a + b given.
@@ -1528,7 +1529,8 @@ __global__ void __launch_bounds__(32 * kCellVars) k_cell_fast(DevMesh m, DevStat
       const float fq = trunc32(dq[i], ok), fD = trunc32(D[i], ok);
       const float x = fq * fd, y = fn * fD;
       bool less = x < y;
-      if (!ok || fabsf(x - y) <= 9.6e-7f * y) less = product_less(dq[i], bd, D[i], bn);
+      if (!ok) less = product_less_far(dq[i], bd, D[i], bn);
+      else if (fabsf(x - y) <= 9.6e-7f * y) less = product_less(dq[i], bd, D[i], bn);
       if (less) {
         bn = abs_bits(dq[i]);
         bd = abs_bits(D[i]);
@@ -1540,7 +1542,7 @@ __global__ void __launch_bounds__(32 * kCellVars) k_cell_fast(DevMesh m, DevStat
     // the fraction starts at 1: min(1, klim n/d), as bit patterns (positive doubles order alike; a NaN
     // of either sign orders above 1 when unsigned).  The reciprocal's seed flushes subnormal numbers.
     r = klim * bn * rcp_nr(bd);
-    if (far) r = barth_ratio(klim, bn, bd);
+    if (__double2hiint(bd) < kTiny) r = barth_ratio(klim, bn, bd);
     if ((unsigned long long)dbits(r) > (unsigned long long)dbits(1.0)) r = 1.0;
     if (zero) r = 0.0;
     if (v >= 2) sr[v - 2][threadIdx.x] = r;
