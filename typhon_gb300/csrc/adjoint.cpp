@@ -55,7 +55,7 @@ int ty_adjoint_vjp(ty_mesh* h, double dt, const double* lamR, double* lamU) {
   int rc;
   if (second && h->o.mode == TY_MODE_FAST) {
     // array-of-structures records, lambda read and written in the caller's layout
-    if (h->o.postlim != TY_POSTLIM_NONE && (rc = ensure_stab(h))) return rc;
+    if (h->o.postlim != TY_POSTLIM_NONE && (rc = ensure_stab(h, h->o.limiter))) return rc;
     if (!h->adj_cell &&
         ((rc = h->alloc(h->adj_cell, 32 * (size_t)m.ldc)) || (rc = h->alloc(h->adj_rec, 44 * (size_t)m.ldf)) ||
          (rc = h->alloc(h->adj_qg, 5 * (size_t)m.ldc)) || (rc = h->alloc(h->adj_ctb, 10 * (size_t)m.ldf)) ||

@@ -326,13 +326,14 @@ int stage_faces(ty_mesh* h) {
   return TY_OK;
 }
 
-// the slot tables of the fast cell kernel for the selected gradient method and MUSCL variant
-int ensure_stab(ty_mesh* h) {
-  const int key = h->geo_highres * 16 + h->lsq_gradmeth;
+// the slot tables of the fast cell kernel for the selected gradient method, MUSCL variant and limiter
+int ensure_stab(ty_mesh* h, int limiter) {
+  const bool lim03 = limiter == TY_LIM_LIM03;
+  const int key = (h->geo_highres * 16 + h->lsq_gradmeth) * 2 + (lim03 ? 1 : 0);
   if (h->m.stab && h->stab_key == key) return TY_OK;
   int rc;
   if (!h->stab_buf && (rc = h->alloc(h->stab_buf, (size_t)tyk::kSlotTab * h->m.nslot * (size_t)h->m.nci))) return rc;
-  cudaError_t e = tyk::kfast::build_stab(h->m, h->geo_highres, h->stab_buf, h->stream);
+  cudaError_t e = tyk::kfast::build_stab(h->m, h->geo_highres, lim03, h->stab_buf, h->stream);
   if (e != cudaSuccess) return cuda_fail(e, "slot tables");
   h->m.stab = h->stab_buf;
   h->stab_key = key;
@@ -681,7 +682,7 @@ int ty_set_params(ty_mesh* h, const ty_spat_params* p) {
     h->m.mtab = h->mtab_buf;
   }
   if (p->mode == TY_MODE_FAST && p->highres != TY_HRES_NONE && (!h->m.mtab || p->viscous != TY_VISC_NONE))
-    if ((rc = ensure_stab(h))) return rc;
+    if ((rc = ensure_stab(h, p->limiter))) return rc;
   h->o.scheme = p->scheme; h->o.highres = p->highres; h->o.limiter = p->limiter; h->o.postlim = p->postlim;
   h->o.gradmeth = p->gradmeth; h->o.mode = p->mode; h->o.gamma = p->gamma; h->o.entropy_fix = p->entropy_fix;
   h->o.inv_entropy_fix = p->entropy_fix > 0.0 ? 1.0 / p->entropy_fix : 0.0;

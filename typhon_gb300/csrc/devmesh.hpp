@@ -195,8 +195,9 @@ TY_DECLARE_MODE(kfast)
 namespace kfast {
 // the per-cell increment matrices of DevMesh::mtab, from lsqw, recw and the gather lists
 cudaError_t build_mtab(const DevMesh& m, double* mtab, cudaStream_t st);
-// DevMesh::stab for a MUSCL variant, from lsqw, uLR, dLR, kLF, kRF and recw
-cudaError_t build_stab(const DevMesh& m, int highres, double* stab, cudaStream_t st);
+// DevMesh::stab for a MUSCL variant (lim03: for LIM03's unscaled slopes), from lsqw, uLR, dLR, kLF, kRF
+// and recw
+cudaError_t build_stab(const DevMesh& m, int highres, bool lim03, double* stab, cudaStream_t st);
 }
 
 }  // namespace tyk

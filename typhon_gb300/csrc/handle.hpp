@@ -76,7 +76,7 @@ struct ty_mesh {
   // stage rows [kMaxStage][5][ng], primitive variables of the last stage's state [5][ng]
   double* mtab_buf = nullptr;  // [nslot][nslot][nci] increment matrices (DevMesh::mtab)
   double* stab_buf = nullptr;  // [nslot][kSlotTab][nci] slot tables (DevMesh::stab)
-  int stab_key = -1;           // MUSCL variant and gradient method they were built for
+  int stab_key = -1;           // MUSCL variant, gradient method and limiter kind they were built for
   double* gcons = nullptr;
   double* gres = nullptr;
   double* gprim = nullptr;
@@ -116,6 +116,6 @@ int reset_dt_slots(ty_mesh* h, int slot, int count);  // slots = largest finite 
 int ensure_prim(ty_mesh* h);                     // primitive variables of the resident state
 int ready(ty_mesh* h);                           // parameters and state present; device set
 int stage_faces(ty_mesh* h);                     // ghost states .. face fluxes of s.prim
-int ensure_stab(ty_mesh* h);                     // slot tables of the fast cell kernel
+int ensure_stab(ty_mesh* h, int limiter);        // slot tables of the fast cell kernel
 int ensure_lsq(ty_mesh* h);                      // least-squares factors (LSQ) on the device
 }  // namespace tyi
