@@ -516,10 +516,12 @@ __device__ __forceinline__ void fetch_blocks(const void* mine, char* stage) {
 // staged -> entries ahead: 250,000 cells FP32 40.5 -> 35.6 -> 32.4, 320,000 FP64 (fast) 108 -> 90 -> 79
 // (the floors: 23 us of HBM traffic, 28 with the 64-byte granules that 112-byte blocks touch; 65 us of
 // FP64 multiply-adds).
+// FP64 in the fast mode only: the exact mode's rounded products are k_imp_matvec_row's.
 constexpr int kMvThreads = 128;
 template <bool F32>
 __global__ void __launch_bounds__(kMvThreads) k_imp_matvec(DevMesh m, ImpState im, const void* __restrict__ xp,
                                                             const double* __restrict__ z, double* __restrict__ y) {
+  static_assert(F32 || kFast, "sums of fused products");
   using T = typename std::conditional<F32, float, double>::type;
   constexpr int PIECES = F32 ? 7 : 13, kBytes = 32 * PIECES * 16, kStride = F32 ? kBlk32 : kBlk;
   extern __shared__ __align__(16) char stages[];  // [warps][2][32 blocks]
@@ -583,27 +585,16 @@ __global__ void __launch_bounds__(kMvThreads) k_imp_matvec(DevMesh m, ImpState i
           a[2 * k] = t.x; a[2 * k + 1] = t.y;
         }
       }
-      if constexpr (F32 || kFast) {
 #pragma unroll
-        for (int i = 0; i < 5; ++i) {
-          T q = s == 0 ? T(0) : yv[i];
-          if (!F32 && s == 0 && z) q = (T)z[5 * (size_t)c + i];
+      for (int i = 0; i < 5; ++i) {
+        T q = s == 0 ? T(0) : yv[i];
+        if (!F32 && s == 0 && z) q = (T)z[5 * (size_t)c + i];
 #pragma unroll
-          for (int j = 0; j < 5; ++j) {
-            if constexpr (F32) q = fmaf(a[i * 5 + j], xv[j], q);
-            else q = fma(a[i * 5 + j], z ? -xv[j] : xv[j], q);
-          }
-          yv[i] = q;
+        for (int j = 0; j < 5; ++j) {
+          if constexpr (F32) q = fmaf(a[i * 5 + j], xv[j], q);
+          else q = fma(a[i * 5 + j], z ? -xv[j] : xv[j], q);
         }
-      } else {
-#pragma unroll
-        for (int i = 0; i < 5; ++i) {
-          T q = T(0);
-#pragma unroll
-          for (int j = 0; j < 5; ++j) q = q + a[i * 5 + j] * xv[j];
-          if (s == 0) yv[i] = z ? z[5 * (size_t)c + i] - q : q;
-          else yv[i] = z ? yv[i] - q : yv[i] + q;
-        }
+        yv[i] = q;
       }
     }
     if (!any) break;
@@ -1317,14 +1308,19 @@ void mv_staged(const DevMesh& m, const ImpState& im, const void* x, const double
   k_imp_matvec<F32><<<grid_of(m.nci, kMvThreads), kMvThreads, bytes, st>>>(m, im, x, z, y);
 }
 
-// A row per thread up to 40,000 cells, a cell per thread above, where the row form's narrower
-// loads cost more than its shorter chains gain.  GB300, us per product, cell / row form: 24,565
-// tetrahedra (exact) 24 / 17, 320,000 (fast) 79 (108 before its blocks were staged) / 153.
+// FP64: a row per thread in the exact mode, whose longer chains it shortens at every size, and up to
+// 40,000 cells in the fast mode, where above that its narrower loads cost more than its shorter chains
+// gain.  GB300, us per product, cell (staged) / row form, tetrahedra:
+//   cells     1,080       5,000       13,720      24,565      40,000      69,120      135,000     320,000    1,080,000
+//   fast   12.2 /  9.1 12.2 / 10.1 12.3 / 10.6 16.3 / 16.3 20.4 / 20.5 26.8 / 32.7 41.1 / 51.1 83.8 / 110  252 / 346
+//   exact  18.3 / 10.1 18.3 / 11.4 18.3 / 14.1 28.6 / 20.4 38.8 / 28.6 49.8 / 43.5 81.2 / 74.3  182 / 167  582 / 539
 constexpr int kRowFormCells = 40000;
 inline void matvec_launch(const DevMesh& m, const ImpState& im, const double* x, const double* z, double* y,
                           cudaStream_t st) {
-  if (m.nci <= kRowFormCells) k_imp_matvec_row<<<grid_of(m.nci, kRowCells), 5 * kRowCells, 0, st>>>(m, im, x, z, y);
-  else mv_staged<false>(m, im, x, z, y, st);
+  if constexpr (kFast) {
+    if (m.nci > kRowFormCells) return mv_staged<false>(m, im, x, z, y, st);
+  }
+  k_imp_matvec_row<<<grid_of(m.nci, kRowCells), 5 * kRowCells, 0, st>>>(m, im, x, z, y);
 }
 
 cudaError_t imp_matvec(const DevMesh& m, const ImpState& im, const double* x, const double* z, double* y,
