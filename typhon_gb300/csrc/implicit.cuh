@@ -817,11 +817,11 @@ __global__ void __launch_bounds__(kMgsThreads) k_mgs_column(double* w, double* V
   constexpr int KR = K > 0 ? K : 1, kWarps = kMgsThreads / 32;
   extern __shared__ double acc[];  // [jk + 1][kMgsThreads] per-thread sums
   __shared__ double h[kMaxKrylov + 1];
-  __shared__ int bad;
+  __shared__ volatile int late;  // a wait of this block ran out (about three seconds): its others end too
   const int t = threadIdx.x, lane = t & 31, wid = t >> 5, g = gridDim.x;
   const size_t first = blockIdx.x * (size_t)kMgsThreads + t, stride = g * (size_t)kMgsThreads;
   double W[KR];
-  if (t == 0) bad = 0;
+  if (t == 0) late = 0;
   // this block's slots of the next column's exchanges (read by nobody until the next launch)
   if (jk < kMaxKrylov)
     for (int i = t; i < 2 * jk + 3; i += kMgsThreads)
@@ -900,8 +900,8 @@ __global__ void __launch_bounds__(kMgsThreads) k_mgs_column(double* w, double* V
 #pragma unroll
         for (int d = 0; d < kBatch; ++d) {
           if (q + 32 * d >= g) break;
-          for (int spins = 0; b[d] == kMgsEmpty && spins < kMgsSpins; ++spins) b[d] = poll(q + 32 * d);
-          if (b[d] == kMgsEmpty) bad = 1;
+          for (int spins = 0; b[d] == kMgsEmpty && spins < kMgsSpins && !late; ++spins) b[d] = poll(q + 32 * d);
+          if (b[d] == kMgsEmpty) late = 1;
           s += __longlong_as_double((long long)b[d]);
         }
       }
@@ -910,7 +910,7 @@ __global__ void __launch_bounds__(kMgsThreads) k_mgs_column(double* w, double* V
       if (lane == 0) h[i] = s;
     }
     __syncthreads();
-    return bad == 0;  // set at most once: nothing resets it
+    return late == 0;  // set at most once: nothing resets it
   };
   products(false);
   if (!exchange(jk, slots)) {
@@ -1026,15 +1026,22 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned b
                "l"(src), "r"(bytes), "r"(smem_addr(b))
                : "memory");
 }
-// waits (bounded) for the phase of the given parity; false after the limit
-__device__ __forceinline__ bool mbar_wait(unsigned long long* b, unsigned parity) {
-  unsigned ok = 0;
-  for (int i = 0; i < (1 << 20) && !ok; ++i)
-    asm volatile("{.reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p;}"
-                 : "=r"(ok)
-                 : "r"(smem_addr(b)), "r"(parity)
-                 : "memory");
+// waits for the phase of the given parity; false after the limit, about two seconds
+constexpr long long kWaitClocks = 4000000000ll;
+__device__ __forceinline__ bool mbar_try(unsigned long long* b, unsigned parity) {
+  unsigned ok;
+  asm volatile("{.reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p;}"
+               : "=r"(ok)
+               : "r"(smem_addr(b)), "r"(parity)
+               : "memory");
   return ok != 0;
+}
+__device__ __forceinline__ bool mbar_wait(unsigned long long* b, unsigned parity) {
+  if (mbar_try(b, parity)) return true;
+  const long long t0 = clock64();
+  while (!mbar_try(b, parity))
+    if (clock64() - t0 > kWaitClocks) return false;
+  return true;
 }
 
 // The FP64 sweep.  Bound by the FP64 pipe (nv + 1 multiply-adds a row, 2 nv + 2 when it extends):
@@ -1089,10 +1096,14 @@ __global__ void __launch_bounds__(kSweepThreads + 32) k_basis_pass(double* V, si
   }
   __syncthreads();
   bool ok = true;
+  int issued = 0;
   if (t == T)  // the producer: one thread of the ninth warp
-    for (int i = 0; i < mine; ++i) {
-      if (i >= S) ok = mbar_wait(&empty[i % S], (i / S - 1) & 1) && ok;
-      load(i);
+    for (; issued < mine; ++issued) {
+      if (issued >= S && !mbar_wait(&empty[issued % S], (issued / S - 1) & 1)) {
+        ok = false;
+        break;
+      }
+      load(issued);
     }
   double* vout = V + (size_t)nv * ldv;
   double ad[J], cr[EXTEND && J <= 20 ? J : 1], xx = 0.0;
@@ -1103,7 +1114,10 @@ __global__ void __launch_bounds__(kSweepThreads + 32) k_basis_pass(double* V, si
   }
   for (int i = 0; i < (t < T ? mine : 0); ++i) {
     const int st = i % S;
-    ok = mbar_wait(&full[st], (i / S) & 1) && ok;
+    if (!__all_sync(0xffffffffu, mbar_wait(&full[st], (i / S) & 1))) {
+      ok = false;
+      break;
+    }
     const double* d = buf + (size_t)st * (J + 1) * T + t;
     const size_t k = (size_t)(blockIdx.x + i * gridDim.x) * T + t;
     if (k < n) {
@@ -1123,8 +1137,13 @@ __global__ void __launch_bounds__(kSweepThreads + 32) k_basis_pass(double* V, si
     __syncwarp();
     if ((t & 31) == 0) mbar_arrive(&empty[st]);
   }
-  if (!ok) *err = 1u;
-  __syncthreads();  // every copy has been waited for: the stages become the per-thread sums
+  // every copy has been waited for: the stages become the per-thread sums
+  if (__syncthreads_or(!ok)) {  // or a wait ran out: the copies still on their way first
+    if (t == T)
+      for (int i = issued > S ? issued - S : 0; i < issued; ++i) mbar_wait(&full[i % S], (i / S) & 1);
+    if (t == 0) *err = 1u;
+    __syncthreads();
+  }
   if (t < T) {
 #pragma unroll
     for (int i = 0; i < J; ++i) buf[i * T + t] = ad[i];
