@@ -1045,26 +1045,31 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* b, unsigned parity
 }
 
 // The FP64 sweep.  Bound by the FP64 pipe (nv + 1 multiply-adds a row, 2 nv + 2 when it extends):
-// compiled per form and per even J >= nv (predicated-off slots occupy the pipe), one block of
-// two warps per SM quarter, its tiles of 256 rows of the nv + 1 vectors brought to shared memory
-// by a ninth warp's bulk copies several tiles ahead, so that neither registers nor occupancy
-// limit the loads in flight.  One block per SM also because a block's reduction costs (nv + 1) (T/32 + 5) additions
+// compiled per form and per even J >= nv (predicated-off slots occupy the pipe), one block per SM whose
+// tiles of T rows of the nv + 1 vectors are brought to shared memory by a last warp's bulk copies
+// several tiles ahead, so that neither registers nor occupancy limit the loads in flight.  T: 15 warps
+// compute up to J = 16, so that with the producer every SM quarter has four (a row's sum of nv
+// dependent multiply-adds leaves two warps a quarter short of the pipe; 16 + 1 warps leave 96 registers
+// a thread, too few at J = 14 and 16); 8 beyond, whose rows take more shared memory.
+// One block per SM also because a block's reduction costs (nv + 1) (T/32 + 5) additions
 // and the last block adds a partial per block: 15 us of a 66 us sweep when eight blocks per SM did.
-// The vectors are padded to 16 bytes (ldv a multiple of 2, src at least ldv long).  GB300, project /
-// extend: 1,250,000 rows, J = 14, 53 / 77 us with loads to registers, 46 / 81 us so; 1,600,000
-// rows, 24 vectors, 427 / 159 (the compiler spread the loads out) -> 88 / 169.
-constexpr int kSweepThreads = 256;
+// The vectors are padded to 16 bytes (ldv a multiple of 2, src at least ldv long).  GB300, us, project
+// on 15 / extend from 14 vectors: loads to registers 21 / 27 at 200,000 rows, 56 / 81 at 1,250,000,
+// 159 / 263 at 5,000,000; 8 warps 16 / 21, 52 / 78, 174 / 278; 15 warps 17 / 20, 49 / 76, 152 / 261.  24 vectors
+// of 1,412,500 rows 121 / 317 (the compiler spread the loads out) -> 79 / 146.
 template <int J>
-constexpr int kSweepStages = J <= 8 ? 8 : (J <= 16 ? 4 : 3);
+constexpr int kSweepThreads = J <= 16 ? 480 : 256;
+template <int J>
+constexpr int kSweepStages = std::min(8, 212000 / ((J + 1) * kSweepThreads<J> * (int)sizeof(double)));
 
 template <int J, bool EXTEND>
-__global__ void __launch_bounds__(kSweepThreads + 32) k_basis_pass(double* V, size_t ldv, int nv,
+__global__ void __launch_bounds__(kSweepThreads<J> + 32) k_basis_pass(double* V, size_t ldv, int nv,
                                                                const double* __restrict__ c,
                                                                const double* __restrict__ src,
                                                                const double* __restrict__ sp, size_t n,
                                                                double* __restrict__ part, unsigned* __restrict__ done,
                                                                double* __restrict__ out, unsigned* err) {
-  constexpr int T = kSweepThreads, S = kSweepStages<J>;
+  constexpr int T = kSweepThreads<J>, S = kSweepStages<J>;
   extern __shared__ __align__(16) double buf[];  // [S][J + 1][T]: the vectors 0 .. nv-1, then src
   __shared__ __align__(8) unsigned long long full[S], empty[S];
   __shared__ double cl[J];
@@ -1097,7 +1102,7 @@ __global__ void __launch_bounds__(kSweepThreads + 32) k_basis_pass(double* V, si
   __syncthreads();
   bool ok = true;
   int issued = 0;
-  if (t == T)  // the producer: one thread of the ninth warp
+  if (t == T)  // the producer: one thread of the last warp
     for (; issued < mine; ++issued) {
       if (issued >= S && !mbar_wait(&empty[issued % S], (issued / S - 1) & 1)) {
         ok = false;
@@ -1464,12 +1469,12 @@ template <int J>
 cudaError_t basis_launch_j(double* V, size_t ldv, int nv, const double* c, const double* src, const double* sp,
                            int extend, size_t n, double* part, unsigned* done, double* out, unsigned* err,
                            cudaStream_t st) {
-  const unsigned g = (unsigned)std::max<size_t>(1, std::min<size_t>((n + kSweepThreads - 1) / kSweepThreads, sm_count()));
-  const size_t sums = (size_t)kSweepStages<J> * (J + 1) * kSweepThreads * sizeof(double);
+  const unsigned g = (unsigned)std::max<size_t>(1, std::min<size_t>((n + kSweepThreads<J> - 1) / kSweepThreads<J>, sm_count()));
+  const size_t sums = (size_t)kSweepStages<J> * (J + 1) * kSweepThreads<J> * sizeof(double);
   auto* k = extend ? k_basis_pass<J, true> : k_basis_pass<J, false>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sums);
   if (e != cudaSuccess) return e;
-  k<<<g, kSweepThreads + 32, sums, st>>>(V, ldv, nv, c, src, sp, n, part, done, out, err);
+  k<<<g, kSweepThreads<J> + 32, sums, st>>>(V, ldv, nv, c, src, sp, n, part, done, out, err);
   return cudaGetLastError();
 }
 
