@@ -213,7 +213,7 @@ int ty_kdif_implicit_step(ty_mesh* h, double dt, const ty_kdif_solve* s, ty_kdif
     int it = 0;
     for (;;) {
       a.it0 = it;
-      a.it1 = std::min(s->max_it, it + kPcgChunk);
+      a.it1 = std::min(s->max_it, it + pcg_chunk(m.nci, check));
       TY_CU(KD_CALL(h, kdif_pcg, m, k, a, q));
       unsigned timed_out[2] = {0, 0};
       TY_CU(cudaMemcpyAsync(timed_out, k.count, sizeof(timed_out), cudaMemcpyDeviceToHost, q));

@@ -271,7 +271,7 @@ __global__ void k_kdif_update_T(DevMesh m, KdifState k) {
 //   p = u + beta p, s = w + beta s, x += alpha p, r -= alpha s, u = r / diag;  barrier
 //   w = S u; gamma, delta;  barrier;  beta = gamma / gamma_old,
 //   alpha = gamma / (delta - beta (gamma / alpha_old))
-// One cooperative launch runs up to kPcgChunk iterations: the grid is resident, every thread
+// One cooperative launch runs up to pcg_chunk() iterations: the grid is resident, every thread
 // owns up to K cells whose r, p, s and w stay in registers, only u travels through L2 (z), and
 // the scalars are recomputed by every block from the blocks' partial sums, in block order
 // (deterministic).  Separate launches cost 9 us of reduction tails and gaps each, whatever the
