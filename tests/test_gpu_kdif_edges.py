@@ -1,5 +1,6 @@
 """Conjugate gradients of heat conduction at the edges: data so small that r.D^-1 r is subnormal,
-and few cells, where the residual becomes exactly zero between two checks of it."""
+few cells, where the residual becomes exactly zero between two checks of it, and the continuation and
+the mixed form's change of matrix in every storage form of the vectors."""
 import numpy as np
 import pytest
 
@@ -84,4 +85,20 @@ def test_exact_convergence(ty, cells, solver, seed):
     T = g.kdif_temperature()
     assert np.isfinite(T).all() and np.isfinite(st["rel_res"]) and st["rel_res"] < 1e-12 and st["iterations"] <= 30
     assert residual(md, g, (T - T0) * cp, g.kdif_get("balance")) < 1e-10
+    g.close()
+
+
+# Two and six cells per thread in registers, and vectors in memory (n = 56): more iterations than a
+# launch runs, and the mixed form's restart on the FP64 conductances from the true residual.  Tolerance: the recurrence's
+# residual drifts from the true one by rounding times the iterations (1e-16 x 1e4 x a growth of 1e4).
+@pytest.mark.parametrize("solver", ["CG", "CG-MIXED"])
+@pytest.mark.parametrize("n", [24, 42, 56])
+def test_continuation(ty, n, solver):
+    md, g = setup(ty, n, 3.0)
+    T0 = np.random.default_rng(n).uniform(0.0, 1.0, md.ncell_int)
+    g.kdif_set_temperature(T0)
+    st = g.kdif_implicit_step(1e3, solver, tol=1e-9, max_it=20000)
+    assert st["iterations"] > 1000 and st["rel_res"] < 1e-9
+    assert st["refinements"] == (1 if solver == "CG-MIXED" else 0)
+    assert residual(md, g, g.kdif_temperature() - T0, g.kdif_get("balance")) < 1e-7
     g.close()
