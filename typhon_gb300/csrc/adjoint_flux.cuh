@@ -3,7 +3,7 @@
 // device code: the dual-number forms are the cross-check of the hand-written ones.
 //
 // Operation order follows the exact-mode residual kernels (calc_varprim_ns.f90 for cons ->
-// prim; SOURCE/VALE/calc_flux_rusanov.f90, calc_flux_hllc.f90, calc_flux_roe.f90 for the
+// prim; SOURCE/VALE/calc_flux_rusanov.f90, calc_flux_hllc.f90 and, new, the Roe flux for the
 // fluxes), so that the primal recomputed here equals the residual's.  The reverse forms take
 // Fb = lambda_F and add (dF/dL)^T Fb and (dF/dR)^T Fb to Lb and Rb (L, R primitive states
 // rho, p, u, v, w; n the unit face normal).

@@ -10,8 +10,9 @@
 //   3. linear solve (implicit_solve.f90:39-86), then U += dU.
 // Solvers of step 3:
 //   TY_KRYLOV_GMRES   Typhon's bdlu_gmres (SOURCE/MATH/bdlu_gmres.f90:50-217): restarted
-//                     GMRES(NKRYLOV), modified Gram-Schmidt (two reductions a vector), Givens rotations, x0 = b/diag,
-//                     its stopping test and restart limit, no preconditioner, FP64.
+//                     GMRES(NKRYLOV), modified Gram-Schmidt (two reductions a vector), Givens
+//                     rotations, x0 = b/diag, its stopping test and restart limit, no
+//                     preconditioner, FP64.
 //   TY_KRYLOV_FGMRES  flexible GMRES(m) with right block-Jacobi preconditioning on the
 //                     assembled BDLU matrix (new), its basis orthogonalised through a measured
 //                     Gram matrix; FP64, or mixed: FP32 blocks, FP32 mat-vec and preconditioner,
@@ -22,7 +23,7 @@
 //                     block-Jacobi preconditioned with the assembled diagonal blocks (new;
 //                     Typhon's gmres_free.f90 is not called by its drivers).
 // The Hessenberg matrix, the Givens rotations and the small triangular solve run on the host
-// from the device dot products (one device-to-host copy of a column per Krylov vector).
+// from the device dot products, which the Krylov kernels write to pinned memory (one wait per vector).
 #include <algorithm>
 #include <cfloat>
 #include <cmath>

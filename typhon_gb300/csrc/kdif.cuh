@@ -275,8 +275,8 @@ __global__ void k_kdif_update_T(DevMesh m, KdifState k) {
 // owns up to K cells whose r, p, s and w stay in registers, only u travels through L2 (z), and
 // the scalars are recomputed by every block from the blocks' partial sums, in block order
 // (deterministic).  Separate launches cost 9 us of reduction tails and gaps each, whatever the
-// mesh.  On GB300, us per iteration: 13,182 cells 25 -> 7.1, 750,000 cells 54 -> 29 (FP64 pipe:
-// 17 operations per cell, 20 us), 2,058,000 cells (vectors in memory, K = 0) 105 -> 80.
+// mesh.  On GB300, us per iteration: 13,182 cells 26.5 -> 8.0, 750,000 cells 51 -> 30 (FP64 pipe:
+// 17 operations per cell, 20 us), 2,058,000 cells (vectors in memory, K = 0) 104 -> 79.
 constexpr int kPcgThreads = 512;
 constexpr int kPcgPart = 3;  // partial sums per block: gamma, delta, r.r
 constexpr int kPcgBlocks = 4 * 160;

@@ -372,8 +372,9 @@ using X64 = typename std::conditional<kFast, double, F64>::type;
 // corrected once by its residual is within an ulp of a/b, and corrected again it is the
 // correctly rounded quotient (P. Markstein, "Computation of elementary functions on the IBM
 // RISC System/6000 processor", IBM J. Res. Dev. 34 (1990): q + (a - b q) y with exact residual).
-// Five fused multiply-adds where an IEEE division issues about ten FP64 instructions.  Exponents are limited so that no residual leaves the normal range; zeros
-// keep their sign (q0); anything else sets `bad` and is divided by div_ieee.
+// Five fused multiply-adds where an IEEE division issues about ten FP64 instructions.  Exponents are
+// limited so that no residual leaves the normal range; zeros keep their sign (q0); anything else sets
+// `bad` and is divided by div_ieee.
 struct Divisor {
   F64 b, y;
   bool ok;
@@ -785,12 +786,12 @@ __device__ void flux_rusanov(double g, const double* L, const double* R, double 
   F[4] = 0.5 * ((a * L[4] + b * R[4]) + pp * nz);
 }
 
-// Roe flux-difference splitting with Harten's entropy fix (new: Typhon has no Roe flux)
 // Harten's fix of a wave speed below delta: a call, taken by few faces
 __device__ __noinline__ double harten(double l, double delta) { return (l * l + delta * delta) / (2.0 * delta); }
 
-// Operations of calc_flux_roe.f90 in its order, as F64; the three divisions by a^2 share its reciprocal,
-// comparisons are of bit patterns.  Limited states and flux of 175,760 faces: 111 -> 92 us.
+// Roe flux-difference splitting with Harten's entropy fix (new: Typhon has no Roe flux).  The oracle's
+// operations in its order, as F64; the three divisions by a^2 share its reciprocal, comparisons are of
+// bit patterns.  Limited states and flux of 175,760 faces: 111 -> 92 us.
 __device__ void flux_roe(const SpatOpts& o, const double* Ls, const double* Rs, double nxs, double nys, double nzs,
                          double* F) {
   F64 L[5], R[5];
