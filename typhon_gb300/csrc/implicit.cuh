@@ -1051,12 +1051,15 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* b, unsigned parity
 // compute up to J = 16, so that with the producer every SM quarter has four (a row's sum of nv
 // dependent multiply-adds leaves two warps a quarter short of the pipe; 16 + 1 warps leave 96 registers
 // a thread, too few at J = 14 and 16); 8 beyond, whose rows take more shared memory.
-// One block per SM also because a block's reduction costs (nv + 1) (T/32 + 5) additions
-// and the last block adds a partial per block: 15 us of a 66 us sweep when eight blocks per SM did.
-// The vectors are padded to 16 bytes (ldv a multiple of 2, src at least ldv long).  GB300, us, project
-// on 15 / extend from 14 vectors: loads to registers 21 / 27 at 200,000 rows, 56 / 81 at 1,250,000,
-// 159 / 263 at 5,000,000; 8 warps 16 / 21, 52 / 78, 174 / 278; 15 warps 17 / 20, 49 / 76, 152 / 261.  24 vectors
-// of 1,412,500 rows 121 / 317 (the compiler spread the loads out) -> 79 / 146.
+// One block per SM also because a block's reduction costs (nv + 1) (T/32 + 5) additions and the last
+// block adds a partial per block: 15 us of a 66 us sweep when eight blocks per SM did.  The vectors are
+// padded to 16 bytes (ldv a multiple of 2, src at least ldv long).  GB300, us, project on 15 / extend
+// from 14 vectors:
+//   rows                  200,000   1,250,000   5,000,000
+//   loads to registers    21 / 27    56 / 81    159 / 263
+//   8 computing warps     16 / 21    52 / 78    174 / 278
+//   15                    17 / 20    49 / 76    152 / 261
+// 24 vectors of 1,412,500 rows 121 / 317 (the compiler spread the loads out) -> 79 / 146.
 template <int J>
 constexpr int kSweepThreads = J <= 16 ? 480 : 256;
 template <int J>

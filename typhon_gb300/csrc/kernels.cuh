@@ -44,8 +44,8 @@ constexpr int kBlock = 256;
 // and its writes are visible (at once in a kernel launched normally).  Every kernel so launched
 // calls it before it touches anything that a kernel writes (mesh tables copied at creation may
 // be read earlier), so completion is transitive along the stream.  Their parameters carry no
-// __restrict__: a compiler may take such data as constant and read it ahead of the wait.  The gap between the short
-// kernels of a Runge-Kutta stage shrinks from 2.7 to 0.2 us.  No kernel calls
+// __restrict__: a compiler may take such data as constant and read it ahead of the wait.  The gap
+// between the short kernels of a Runge-Kutta stage shrinks from 2.7 to 0.2 us.  No kernel calls
 // launch_dependents: blocks of the next kernel then fill the SMs that have room first and stay
 // there, which doubled the 8,192-cell vortex's step (75 -> 150 us).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
