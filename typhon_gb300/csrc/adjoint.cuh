@@ -585,8 +585,13 @@ __device__ __forceinline__ void hllc_vjp_fast(const SpatOpts& o, const double* Q
   const F64 vnl = fma(L[2], n[0], fma(L[3], n[1], L[4] * n[2])), vnr = fma(R[2], n[0], fma(R[3], n[1], R[4] * n[2]));
   const F64 dvn = vnr - vnl, vm = fma(kr, dvn, vnl);
   const F64 al2 = g * TL, ar2 = g * TR, am2 = fma(g, fma(kl, TL, kr * TR), hg1 * (kk * dd));
+  // sound speeds 0 at zero pressure, where the reciprocal root has no value (the derivative then has none
+  // for the cell of that pressure; its neighbour's does not depend on it)
   const F64 yl = rsqrt_nr(al2), yr = rsqrt_nr(ar2), ym = rsqrt_nr(am2);
-  const F64 am = am2 * ym, l1 = fma(-al2, yl, vnl), l2 = vm - am, r1 = fma(ar2, yr, vnr), r2 = vm + am;
+  const F64 a0 = am2 * ym, l0 = fma(-al2, yl, vnl), r0 = fma(ar2, yr, vnr);
+  const F64 am = __double2hiint(am2.v) > 0 ? a0.v : 0.0;
+  const F64 l1 = __double2hiint(al2.v) > 0 ? l0 : vnl, r1 = __double2hiint(ar2.v) > 0 ? r0 : vnr;
+  const F64 l2 = vm - am, r2 = vm + am;
   const bool slm = order_key(l2.v) < order_key(l1.v), srm = order_key(r1.v) < order_key(r2.v);
   const F64 sl = slm ? l2 : l1, sr = srm ? r2 : r1;
   const F64 dl = sl - vnl, dr = sr - vnr, rql = L[0] * dl, rqr = R[0] * dr;
